@@ -1,0 +1,172 @@
+// Double-precision arithmetic on the integer and FP32 pipes, rounded as IEEE 754 rounds it (to nearest, ties to
+// even), for kernels that are bound by the FP64 pipe.
+//
+// This GPU issues one FP64 warp instruction per SM every 16 clocks (2 lanes a clock), against 0.25-0.5 clocks for
+// a 32-bit integer or FP32 one, and the two run side by side.  A division, which the compiler builds from about
+// ten FP64 instructions, therefore costs far more there than its integer form, and even a multiplication is worth
+// moving while the FP64 pipe is the one that is full.
+//
+// The functions take finite operands whose results stay in the normal range; each says which zeros it accepts.
+// Callers test the range of what they feed in (a few integer instructions for a whole stencil) and keep the plain
+// FP64 expression for everything else (subnormals, infinities, NaN).  Host and device compile the same code, and
+// tests compare it with the host's own arithmetic bit for bit.
+//
+// Methods: a quotient is found by long division in three digits (two from a 24-bit reciprocal in FP32, one from the
+// exact integer remainder), and the exact integer remainder decides the rounding, so the result does not depend on
+// the reciprocal's last bits; a third is floor((N + 1) / 3) of the scaled significand N, which is its nearest
+// integer because N mod 3 is never a half.
+#pragma once
+#include <cmath>
+
+#include "sf_convert.cuh"
+
+namespace sf {
+
+#if defined(__CUDA_ARCH__)
+SF_CONV_FN float f32_rcp(float x) {  // 1 ulp
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+SF_CONV_FN float f32_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+SF_CONV_FN float f32_mul(float a, float b) { return __fmul_rn(a, b); }
+SF_CONV_FN float f32_add(float a, float b) { return __fadd_rn(a, b); }
+SF_CONV_FN int f32_nearest_int(float a) { return __float2int_rn(a); }
+SF_CONV_FN double f64_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+SF_CONV_FN uint32_t mulhi_u32(uint32_t a, uint32_t b) { return __umulhi(a, b); }
+SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) { return __funnelshift_l(lo, hi, n); }
+SF_CONV_FN uint32_t shf_r(uint32_t lo, uint32_t hi, int n) { return __funnelshift_r(lo, hi, n); }
+#else
+#if defined(SF_F64_TEST_RCP)
+float SF_F64_TEST_RCP(float x);  // a test's own reciprocal, off by as much as the device's may be
+SF_CONV_FN float f32_rcp(float x) { return SF_F64_TEST_RCP(x); }
+#else
+SF_CONV_FN float f32_rcp(float x) { return 1.0f / x; }
+#endif
+SF_CONV_FN float f32_fma(float a, float b, float c) { return std::fmaf(a, b, c); }
+SF_CONV_FN float f32_mul(float a, float b) { return a * b; }
+SF_CONV_FN float f32_add(float a, float b) { return a + b; }
+SF_CONV_FN int f32_nearest_int(float a) { return (int)std::nearbyintf(a); }
+SF_CONV_FN double f64_fma(double a, double b, double c) { return std::fma(a, b, c); }
+SF_CONV_FN uint32_t mulhi_u32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+// the high / low word of (hi:lo) shifted left / right by n in [0, 31]
+SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) { return (uint32_t)(((((uint64_t)hi << 32) | lo) << n) >> 32); }
+SF_CONV_FN uint32_t shf_r(uint32_t lo, uint32_t hi, int n) { return (uint32_t)((((uint64_t)hi << 32) | lo) >> n); }
+#endif
+
+constexpr uint32_t kF64Exp = 0x7ff00000u, kF64Frac = 0xfffffu, kF64One = 0x100000u, kF64Sign = 0x80000000u;
+
+// |v| == 0
+SF_CONV_FN bool f64_is_zero(double v) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    return ((h << 1) | l) == 0u;
+}
+
+// True when v is zero or 2^lo <= |v| < 2^hi (-1022 <= lo < hi <= 1023): the operands the functions below accept.
+SF_CONV_FN bool f64_in_range(double v, int lo, int hi) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    return (h & kF64Exp) - ((uint32_t)(lo + 1023) << 20) < ((uint32_t)(hi - lo) << 20) || ((h << 1) | l) == 0u;
+}
+
+// x / 3; x zero or normal with a normal result.
+SF_CONV_FN double f64_third(double x) {
+    uint32_t h, l;
+    f64_words(x, h, l);
+    const uint32_t m = (h & kF64Frac) | kF64One;
+    // N = significand * 2^s in [2^53.58, 2^54.58): N / 3 has 53 bits
+    const int s = m >= 0x180000u ? 1 : 2;
+    const uint32_t nh = shf_l(l, m, s), nl = l << s;
+    // in digits of 30 bits, so that the second digit's dividend (r 2^30 + low digit + 1) fits a word
+    const uint32_t d1 = shf_l(nl, nh, 2), d0 = nl & 0x3fffffffu;
+    const uint32_t q1 = mulhi_u32(d1, 0x55555556u);  // d1 / 3, exact below 2^31
+    const uint32_t z = ((d1 - 3u * q1) << 30) + d0 + 1u;
+    const uint32_t q0 = mulhi_u32(z, 0xaaaaaaabu) >> 1;
+    const uint64_t q = ((uint64_t)q1 << 30) + q0;
+    // exponent: N = M 2^s, so x / 3 = q 2^(e - s); q carries the implicit bit
+    const uint32_t e = (h & (kF64Sign | kF64Exp)) - ((uint32_t)(s + 1) << 20);
+    const double r = f64_from_words((uint32_t)(q >> 32) + e, (uint32_t)q);
+    return ((h << 1) | l) == 0u ? x : r;
+}
+
+// The FP32 digits of a significand (hi word with the implicit bit, low word) in [1, 2): leading 24 bits exactly,
+// next 24 bits exactly; the last 5 are left to the remainder.
+struct F64Digits {
+    float hi, lo;
+};
+SF_CONV_FN F64Digits f64_digits(uint32_t h, uint32_t l) {
+    F64Digits d;
+    d.hi = f32_from_bits((shf_l(l, h, 3) & 0x7fffffu) | 0x3f800000u);
+    // bits 28..5 of the low word: the leading one of an FP32 at 2^-23 scale, then taken off again (exact)
+    d.lo = f32_add(f32_from_bits((((l << 3) >> 9) & 0x7fffffu) | 0x34000000u), -f32_from_bits(0x34000000u));
+    return d;
+}
+
+// a / b; b normal, a zero or normal, the quotient normal.
+SF_CONV_FN double f64_div(double a, double b) {
+    uint32_t ah, al, bh, bl;
+    f64_words(a, ah, al);
+    f64_words(b, bh, bl);
+    const uint32_t am = (ah & kF64Frac) | kF64One, bm = (bh & kF64Frac) | kF64One;
+    const bool less = am < bm || (am == bm && al < bl);
+    const F64Digits x = f64_digits(am, al), y = f64_digits(bm, bl);
+    // quotient of the significands to about 2^-44: first digit q0, second digit q1 from the remainder
+    float y0 = f32_rcp(y.hi);
+    y0 = f32_fma(f32_fma(-y.hi, y0, 1.0f), y0, y0);  // within 2^-24 whatever the approximation's last bits
+    const float q0 = f32_mul(x.hi, y0);
+    const float r = f32_add(f32_fma(-q0, y.hi, x.hi), f32_fma(-q0, y.lo, x.lo));
+    const float q1 = f32_mul(r, y0);  // |q1| < 2^-22: its integer below is less than 2^31
+    // Q = quotient * 2^s, s = 53 where a's significand is the smaller and 52 otherwise: 53 bits
+    const uint32_t qb = f32_bits(q0);
+    const int sh = (int)(qb >> 23) - (127 + 23 - 52) + (less ? 1 : 0);  // 28 .. 30: q0's significand to 2^s
+    const uint32_t qm = (qb & 0x7fffffu) | 0x800000u;
+    const int c1 = f32_nearest_int(f32_mul(q1, less ? 9007199254740992.0f : 4503599627370496.0f));
+    int64_t q = (int64_t)((uint64_t)qm << sh) + c1;
+    // exact remainder a 2^s - Q b (its size fits 64 bits, so the low 64 bits of the products suffice); s >= 52, so
+    // only a's low bits reach the upper word
+    const uint64_t B = ((uint64_t)bm << 32) | bl;
+    int64_t rem = (int64_t)(((uint64_t)(al << (less ? 21 : 20)) << 32) - (uint64_t)q * B);
+    // third digit: the remainder over b, |digit| < 2^11, by the usual add of 1.5 2^23
+    const float rf = f32_fma((float)(int32_t)(rem >> 32), f32_mul(y0, 9.5367431640625e-7f), 12582912.0f);
+    const int c2 = (int)(f32_bits(rf) - 0x4b400000u);
+    q += c2;
+    rem -= (int64_t)((uint64_t)(int64_t)c2 * B);
+    // |rem| is now barely above b / 2 at most: the nearest quotient (a tie cannot occur)
+    const int64_t twice = rem * 2;
+    q += (twice > (int64_t)B ? 1 : 0) - (twice < -(int64_t)B ? 1 : 0);
+    const uint32_t ex = (ah & kF64Exp) - (bh & kF64Exp) + ((1023u - 1u) << 20) - (less ? kF64One : 0u);
+    const uint32_t sign = (ah ^ bh) & kF64Sign;
+    const uint32_t rh = (uint32_t)((uint64_t)q >> 32) + ex;
+    return ((ah << 1) | al) == 0u ? f64_from_words(sign, 0u) : f64_from_words(rh | sign, (uint32_t)q);
+}
+
+// a * b; each zero or normal, the product zero or normal.
+SF_CONV_FN double f64_mul(double a, double b) {
+    uint32_t ah, al, bh, bl;
+    f64_words(a, ah, al);
+    f64_words(b, bh, bl);
+    // (A << 1) * (B << 11) = A B << 12: the upper 64 bits hold 53 or 54 bits of the product, the lower 64 the rest
+    const uint32_t am = (ah & kF64Frac) | kF64One, bm = (bh & kF64Frac) | kF64One;
+    const uint32_t x1 = shf_l(al, am, 1), x0 = al << 1;
+    const uint32_t y1 = shf_l(bl, bm, 11), y0 = bl << 11;
+    const uint64_t p00 = (uint64_t)x0 * y0;
+    const uint64_t p01 = (uint64_t)x0 * y1 + (p00 >> 32);
+    const uint64_t p10 = (uint64_t)x1 * y0 + (uint32_t)p01;
+    uint64_t hi = (uint64_t)x1 * y1 + (p01 >> 32) + (p10 >> 32);
+    uint32_t lh = (uint32_t)p10, ll = (uint32_t)p00;
+    // a 54-bit product loses one bit more (the lowest 12 bits of the lower half are zero: none is lost here)
+    const int c = (int)(hi >> 53);
+    const uint32_t h1 = (uint32_t)(hi >> 32) >> c, h0 = shf_r((uint32_t)hi, (uint32_t)(hi >> 32), c);
+    lh = shf_r(lh, (uint32_t)hi, c);
+    // round to nearest even: add just under a half, plus one where the kept part is odd or a lower bit is set
+    const uint32_t st = (h0 & 1u) | ll ? 1u : 0u;
+    const uint64_t t = (uint64_t)lh + 0x7fffffffu + st;
+    const uint32_t ex = (ah & kF64Exp) + (bh & kF64Exp) - ((1023u + 1u) << 20) + ((uint32_t)c << 20);
+    const uint64_t m = ((uint64_t)(h1 + ex) << 32 | h0) + (t >> 32);
+    const uint32_t sign = (ah ^ bh) & kF64Sign;
+    const bool zero = ((ah << 1) | al) == 0u || ((bh << 1) | bl) == 0u;
+    return zero ? f64_from_words(sign, 0u) : f64_from_words((uint32_t)(m >> 32) | sign, (uint32_t)m);
+}
+
+}  // namespace sf

@@ -1,0 +1,79 @@
+// Checks the integer-pipe double-precision functions (csrc/sf_f64_int.cuh) against the host's own arithmetic, bit
+// for bit, with a reciprocal that is off by up to four units in the last place either way (the device's is off by
+// one).  Significands at the ends of the binade, with few set bits and at random; exponents over the range the
+// callers accept.  Prints the number of mismatches and the number of values checked.
+#include <cinttypes>
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <random>
+
+#define SF_F64_TEST_RCP test_rcp
+namespace sf {
+float test_rcp(float x);
+}
+#include "sf_f64_int.cuh"
+
+static int g_off = 0;
+namespace sf {
+float test_rcp(float x) {
+    float y = 1.0f / x;
+    for (int i = 0; i < std::abs(g_off); i++) y = std::nextafterf(y, g_off > 0 ? 2.f : 0.f);
+    return y;
+}
+}  // namespace sf
+
+static uint64_t bits(double v) {
+    uint64_t u;
+    std::memcpy(&u, &v, 8);
+    return u;
+}
+
+int main() {
+    long long bad = 0, n = 0;
+    std::mt19937_64 rng(2025);
+    auto draw = [&]() {
+        uint64_t m = rng() & 0xfffffffffffffull;
+        switch (rng() % 7) {
+            case 0: m = 0; break;
+            case 1: m = 0xfffffffffffffull; break;
+            case 2: m = rng() & 15; break;
+            case 3: m = 0xfffffffffffffull - (rng() & 15); break;
+            case 4: m &= ~0xffffffffull; break;
+            default: break;
+        }
+        const uint64_t u = ((rng() & 1) << 63) | ((uint64_t)(1023 - 250 + (int)(rng() % 500)) << 52) | m;
+        double v;
+        std::memcpy(&v, &u, 8);
+        return rng() % 40 == 0 ? std::copysign(0.0, v) : v;
+    };
+    auto check = [&](const char *what, double got, double want, double a, double b) {
+        n++;
+        if (bits(got) != bits(want)) {
+            if (bad < 10) std::printf("%s(%a, %a) = %a, expected %a\n", what, a, b, got, want);
+            bad++;
+        }
+    };
+    for (int t = 0; t < 6000000; t++) {
+        g_off = (int)(rng() % 9) - 4;
+        const double a = draw(), b = draw();
+        if (b != 0) {
+            check("div", sf::f64_div(a, b), a / b, a, b);
+            // a quotient next to a representable value and next to a midpoint
+            const double q = a / b, c = q * b;
+            if (c != 0) check("div", sf::f64_div(c, b), c / b, c, b);
+        }
+        check("mul", sf::f64_mul(a, b), a * b, a, b);
+        check("third", sf::f64_third(a), a / 3, a, 0);
+        const bool in = a == 0 || (std::fabs(a) >= 0x1p-100 && std::fabs(a) < 0x1p60);
+        n++;
+        bad += sf::f64_in_range(a, -100, 60) != in;
+    }
+    const double outside[] = {0x1p-1074, -0x1p-1030, 0x1p-101, 0x1p60, -0x1p60, 1e300, INFINITY, -INFINITY, NAN};
+    for (double v : outside) {
+        n++;
+        bad += sf::f64_in_range(v, -100, 60);
+    }
+    std::printf("%lld %lld\n", bad, n);
+    return bad != 0;
+}
