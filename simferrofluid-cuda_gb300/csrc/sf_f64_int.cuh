@@ -13,7 +13,7 @@
 //
 // Methods: a quotient is found by long division in three digits (two from a 24-bit reciprocal in FP32, one from the
 // exact integer remainder), and the exact integer remainder decides the rounding, so the result does not depend on
-// the reciprocal's last bits; a third is floor((N + 1) / 3) of the scaled significand N, which is its nearest
+// the reciprocal's last bits; a square root goes the same way; a third is floor((N + 1) / 3) of the scaled significand N, which is its nearest
 // integer because N mod 3 is never a half.
 #pragma once
 #include <cmath>
@@ -28,6 +28,11 @@ SF_CONV_FN float f32_rcp(float x) {  // 1 ulp
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+SF_CONV_FN float f32_rsqrt(float x) {  // within 2^-22
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 SF_CONV_FN float f32_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 SF_CONV_FN float f32_mul(float a, float b) { return __fmul_rn(a, b); }
 SF_CONV_FN float f32_add(float a, float b) { return __fadd_rn(a, b); }
@@ -38,10 +43,13 @@ SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) { return __funnelshif
 SF_CONV_FN uint32_t shf_r(uint32_t lo, uint32_t hi, int n) { return __funnelshift_r(lo, hi, n); }
 #else
 #if defined(SF_F64_TEST_RCP)
-float SF_F64_TEST_RCP(float x);  // a test's own reciprocal, off by as much as the device's may be
-SF_CONV_FN float f32_rcp(float x) { return SF_F64_TEST_RCP(x); }
+// a test's own approximations, off by as much as the device's may be
+float SF_F64_TEST_RCP(float y);
+SF_CONV_FN float f32_rcp(float x) { return SF_F64_TEST_RCP(1.0f / x); }
+SF_CONV_FN float f32_rsqrt(float x) { return SF_F64_TEST_RCP((float)(1.0 / std::sqrt((double)x))); }
 #else
 SF_CONV_FN float f32_rcp(float x) { return 1.0f / x; }
+SF_CONV_FN float f32_rsqrt(float x) { return (float)(1.0 / std::sqrt((double)x)); }
 #endif
 SF_CONV_FN float f32_fma(float a, float b, float c) { return std::fmaf(a, b, c); }
 SF_CONV_FN float f32_mul(float a, float b) { return a * b; }
@@ -70,12 +78,9 @@ SF_CONV_FN bool f64_in_range(double v, int lo, int hi) {
     return (h & kF64Exp) - ((uint32_t)(lo + 1023) << 20) < ((uint32_t)(hi - lo) << 20) || ((h << 1) | l) == 0u;
 }
 
-// x / 3; x zero or normal with a normal result.
-SF_CONV_FN double f64_third(double x) {
-    uint32_t h, l;
-    f64_words(x, h, l);
-    const uint32_t m = (h & kF64Frac) | kF64One;
-    // N = significand * 2^s in [2^53.58, 2^54.58): N / 3 has 53 bits
+// (M 2^s0 / 3) for a significand M in [2^52, 2^53] with sign and exponent bits `se` above it, packed.
+SF_CONV_FN double f64_third_sig(uint32_t m, uint32_t l, uint32_t se) {
+    // N = M 2^s in [2^53.58, 2^54.58): N / 3 has 53 bits
     const int s = m >= 0x180000u ? 1 : 2;
     const uint32_t nh = shf_l(l, m, s), nl = l << s;
     // in digits of 30 bits, so that the second digit's dividend (r 2^30 + low digit + 1) fits a word
@@ -84,9 +89,33 @@ SF_CONV_FN double f64_third(double x) {
     const uint32_t z = ((d1 - 3u * q1) << 30) + d0 + 1u;
     const uint32_t q0 = mulhi_u32(z, 0xaaaaaaabu) >> 1;
     const uint64_t q = ((uint64_t)q1 << 30) + q0;
-    // exponent: N = M 2^s, so x / 3 = q 2^(e - s); q carries the implicit bit
-    const uint32_t e = (h & (kF64Sign | kF64Exp)) - ((uint32_t)(s + 1) << 20);
-    const double r = f64_from_words((uint32_t)(q >> 32) + e, (uint32_t)q);
+    // x / 3 = q 2^(e - s); q carries the implicit bit
+    return f64_from_words((uint32_t)(q >> 32) + se - ((uint32_t)(s + 1) << 20), (uint32_t)q);
+}
+
+// x / 3; x zero or normal with a normal result.
+SF_CONV_FN double f64_third(double x) {
+    uint32_t h, l;
+    f64_words(x, h, l);
+    const double r = f64_third_sig((h & kF64Frac) | kF64One, l, h & (kF64Sign | kF64Exp));
+    return ((h << 1) | l) == 0u ? x : r;
+}
+
+// (K x) / 3 with K x rounded first, 2 <= K <= 15; x zero or normal with normal results.
+template <int K>
+SF_CONV_FN double f64_times_third(double x) {
+    uint32_t h, l;
+    f64_words(x, h, l);
+    const uint32_t m = (h & kF64Frac) | kF64One;
+    const uint64_t lo = (uint64_t)l * (uint32_t)K;
+    const uint64_t p = lo + ((uint64_t)(m * (uint32_t)K) << 32);
+    constexpr int s0 = K >= 8 ? 3 : (K >= 4 ? 2 : 1);
+    const int s = s0 + (int)(p >> (53 + s0));
+    // round to nearest even at bit s; the sum may reach 2^53, which the third takes
+    const uint32_t odd = ((uint32_t)p >> s) & 1u;
+    const uint64_t q = p + ((1u << (s - 1)) - 1u + odd);
+    const uint32_t ql = shf_r((uint32_t)q, (uint32_t)(q >> 32), s), qh = (uint32_t)(q >> 32) >> s;
+    const double r = f64_third_sig(qh, ql, (h & (kF64Sign | kF64Exp)) + ((uint32_t)s << 20));
     return ((h << 1) | l) == 0u ? x : r;
 }
 
@@ -141,32 +170,81 @@ SF_CONV_FN double f64_div(double a, double b) {
     return ((ah << 1) | al) == 0u ? f64_from_words(sign, 0u) : f64_from_words(rh | sign, (uint32_t)q);
 }
 
-// a * b; each zero or normal, the product zero or normal.
+// A product of two significands, each taken times 2^6 (so that the middle sums stay below 2^64): hi:lh:ll is
+// A B 2^12, whose upper word pair holds 53 or 54 bits.  Rounded to nearest even and packed with the exponent bits
+// `ex` of the 54-bit case less one (the implicit bit adds one) and the sign.
+SF_CONV_FN double f64_round_product(uint64_t hi, uint32_t lh, uint32_t ll, uint32_t ex, uint32_t sign) {
+    // a 54-bit product drops one bit more (the lowest 12 bits of ll are zero: none is lost below lh)
+    const int c = (int)(hi >> 53);
+    const uint32_t h1 = (uint32_t)(hi >> 32) >> c, h0 = shf_r((uint32_t)hi, (uint32_t)(hi >> 32), c);
+    lh = shf_r(lh, (uint32_t)hi, c);
+    // add just under a half, plus one where the kept part is odd or a lower bit is set
+    const uint32_t st = ((h0 & 1u) | ll) ? 1u : 0u;
+    const uint64_t t = (uint64_t)lh + 0x7fffffffu + st;
+    const uint64_t m = (((uint64_t)(h1 + ex + ((uint32_t)c << 20)) << 32) | h0) + (t >> 32);
+    return f64_from_words((uint32_t)(m >> 32) | sign, (uint32_t)m);
+}
+
+// a * b; each zero or normal, the product zero or normal.  NONZERO: neither operand is zero.
+template <bool NONZERO = false>
 SF_CONV_FN double f64_mul(double a, double b) {
     uint32_t ah, al, bh, bl;
     f64_words(a, ah, al);
     f64_words(b, bh, bl);
-    // (A << 1) * (B << 11) = A B << 12: the upper 64 bits hold 53 or 54 bits of the product, the lower 64 the rest
-    const uint32_t am = (ah & kF64Frac) | kF64One, bm = (bh & kF64Frac) | kF64One;
-    const uint32_t x1 = shf_l(al, am, 1), x0 = al << 1;
-    const uint32_t y1 = shf_l(bl, bm, 11), y0 = bl << 11;
+    const uint32_t x1 = shf_l(al, (ah & kF64Frac) | kF64One, 6), x0 = al << 6;
+    const uint32_t y1 = shf_l(bl, (bh & kF64Frac) | kF64One, 6), y0 = bl << 6;
     const uint64_t p00 = (uint64_t)x0 * y0;
-    const uint64_t p01 = (uint64_t)x0 * y1 + (p00 >> 32);
-    const uint64_t p10 = (uint64_t)x1 * y0 + (uint32_t)p01;
-    uint64_t hi = (uint64_t)x1 * y1 + (p01 >> 32) + (p10 >> 32);
-    uint32_t lh = (uint32_t)p10, ll = (uint32_t)p00;
-    // a 54-bit product loses one bit more (the lowest 12 bits of the lower half are zero: none is lost here)
-    const int c = (int)(hi >> 53);
-    const uint32_t h1 = (uint32_t)(hi >> 32) >> c, h0 = shf_r((uint32_t)hi, (uint32_t)(hi >> 32), c);
-    lh = shf_r(lh, (uint32_t)hi, c);
-    // round to nearest even: add just under a half, plus one where the kept part is odd or a lower bit is set
-    const uint32_t st = (h0 & 1u) | ll ? 1u : 0u;
-    const uint64_t t = (uint64_t)lh + 0x7fffffffu + st;
-    const uint32_t ex = (ah & kF64Exp) + (bh & kF64Exp) - ((1023u + 1u) << 20) + ((uint32_t)c << 20);
-    const uint64_t m = ((uint64_t)(h1 + ex) << 32 | h0) + (t >> 32);
+    const uint64_t mid = (uint64_t)x1 * y0 + ((uint64_t)x0 * y1 + (p00 >> 32));
+    const uint64_t hi = (uint64_t)x1 * y1 + (mid >> 32);
     const uint32_t sign = (ah ^ bh) & kF64Sign;
+    const double r = f64_round_product(hi, (uint32_t)mid, (uint32_t)p00,
+                                       (ah & kF64Exp) + (bh & kF64Exp) - (1024u << 20), sign);
+    if (NONZERO) return r;
     const bool zero = ((ah << 1) | al) == 0u || ((bh << 1) | bl) == 0u;
-    return zero ? f64_from_words(sign, 0u) : f64_from_words((uint32_t)(m >> 32) | sign, (uint32_t)m);
+    return zero ? f64_from_words(sign, 0u) : r;
+}
+
+// a * a; a zero or normal with a normal square.
+template <bool NONZERO = false>
+SF_CONV_FN double f64_sqr(double a) {
+    uint32_t ah, al;
+    f64_words(a, ah, al);
+    const uint32_t x1 = shf_l(al, (ah & kF64Frac) | kF64One, 6), x0 = al << 6;
+    const uint64_t p00 = (uint64_t)x0 * x0;
+    const uint64_t mid = (uint64_t)x1 * (2u * x0) + (((uint64_t)x1 * (x0 >> 31)) << 32) + (p00 >> 32);
+    const uint64_t hi = (uint64_t)x1 * x1 + (mid >> 32);
+    const double r = f64_round_product(hi, (uint32_t)mid, (uint32_t)p00, 2u * (ah & kF64Exp) - (1024u << 20), 0u);
+    return !NONZERO && ((ah << 1) | al) == 0u ? 0.0 : r;
+}
+
+// sqrt(a); a positive and normal.
+SF_CONV_FN double f64_sqrt(double a) {
+    uint32_t ah, al;
+    f64_words(a, ah, al);
+    const uint32_t am = (ah & kF64Frac) | kF64One;
+    const uint32_t odd = ((ah >> 20) & 1u) ^ 1u;  // exponent 2 k + odd
+    // the radicand in [1, 4) as FP32 digits, root to about 2^-45: s0, then s1 from the remainder
+    const F64Digits x = f64_digits(am, al);
+    const float xh = f32_from_bits(f32_bits(x.hi) + (odd << 23)), xl = odd ? f32_add(x.lo, x.lo) : x.lo;
+    float y = f32_rsqrt(xh);
+    y = f32_fma(f32_mul(0.5f, y), f32_fma(f32_mul(-xh, y), y, 1.0f), y);
+    const float s0 = f32_mul(xh, y);
+    const float r = f32_add(f32_fma(-s0, s0, xh), xl);
+    const float s1 = f32_mul(r, f32_mul(0.5f, y));
+    // S = root * 2^52 in [2^52, 2^53); remainder a 2^(52 + odd) - S^2 in the low 64 bits
+    const uint32_t sb = f32_bits(s0);
+    uint64_t s = (uint64_t)((sb & 0x7fffffu) | 0x800000u) << ((int)(sb >> 23) - 98);
+    s += (int64_t)f32_nearest_int(f32_mul(s1, 4503599627370496.0f));
+    int64_t rem = (int64_t)(((uint64_t)(al << (20 + odd)) << 32) - s * s);
+    // third digit: remainder / (2 S)
+    const float rf = f32_fma((float)(int32_t)(rem >> 32), f32_mul(y, 4.76837158203125e-7f), 12582912.0f);
+    const int64_t c = (int64_t)(int)(f32_bits(rf) - 0x4b400000u);
+    rem -= (int64_t)((uint64_t)c * (2 * s + (uint64_t)c));
+    s += (uint64_t)c;
+    // (S + 1/2)^2 = S^2 + S + 1/4: up where the remainder exceeds S, down where it is -S or less
+    s += (rem > (int64_t)s ? 1 : 0) - (rem <= -(int64_t)s ? 1 : 0);
+    const uint32_t ex = (((ah >> 20) + 1021u - odd) >> 1) << 20;
+    return f64_from_words((uint32_t)(s >> 32) + ex, (uint32_t)s);
 }
 
 }  // namespace sf

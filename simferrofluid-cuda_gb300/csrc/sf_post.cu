@@ -206,6 +206,12 @@ __global__ void __launch_bounds__(256) k_advect_velocity(Dims d, int a, Origin o
     out[fidx(f, i, j, k)] = trilerp_face(d, ua, a, og.o, h, invh, q);
 }
 
+// v < 0 on the bits (false for NaN and -0)
+__device__ __forceinline__ bool below0(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return b > 0x8000000000000000ULL && b <= 0xfff0000000000000ULL;
+}
+
 __device__ __forceinline__ double dmax0(double a, double b) { return (a < b) ? b : a; }  // std::max(a, b)
 
 // GetDrv (core/Reinitialization.cpp:4-27): the WENO5 one-sided derivative from five differences, the upwind side's
@@ -248,39 +254,33 @@ __device__ __noinline__ double weno_plain(double d0, double d1, double d2, doubl
 //   * 2 d and 4 d are exact, so d0 - 2 d1 is one fused multiply-add;
 //   * the largest square is the square of the largest magnitude (rounding is monotone), found by integer compares;
 //     its millionth is at least 2^-221, so adding 1e-99 leaves it unchanged.
-// Measured per warp and SM: an FP64 instruction takes 19 clocks, the compiler's division 137 and its x / 3 140; here
-// a division takes 27 and a third 9, beside the FP64 pipe.
+//   * products go to the integer pipe too, so that the FP64 pipe is left with the sums.
+// Measured per warp and SM: an FP64 instruction takes 19 clocks, the compiler's division 137, its x / 3 140 and its
+// square root 143; on the integer pipe, beside it, a product takes 12-14, a division 27, a third 9, a root 24.
 __device__ __forceinline__ double weno_fast(const double dev[5], double invdx) {
     long long big = 0;
 #pragma unroll
     for (int j = 0; j < 5; j++) big = max(big, __double_as_longlong(dev[j]) & 0x7fffffffffffffffLL);
     const double top = __longlong_as_double(big);
-    const double eps = top * top * 1e-6;
+    const double eps = f64_mul<true>(f64_sqr<true>(top), 1e-6);
     const double third1 = f64_third(dev[1]), third2 = f64_third(dev[2]), third3 = f64_third(dev[3]);
-    const double phix1 = __fma_rn(.5, f64_third(dev[2] * 11), __fma_rn(-.5, f64_third(dev[1] * 7), f64_third(dev[0])));
-    const double phix2 = __fma_rn(.5, f64_third(dev[2] * 5) - third1, third3);
-    const double phix3 = __fma_rn(-.5, f64_third(dev[4]), __fma_rn(.5, f64_third(dev[3] * 5), third2));
+    const double phix1 = __fma_rn(.5, f64_times_third<11>(dev[2]),
+                                  __fma_rn(-.5, f64_times_third<7>(dev[1]), f64_third(dev[0])));
+    const double phix2 = __fma_rn(.5, f64_times_third<5>(dev[2]) - third1, third3);
+    const double phix3 = __fma_rn(-.5, f64_third(dev[4]), __fma_rn(.5, f64_times_third<5>(dev[3]), third2));
     const double three2 = 3 * dev[2];
-    double t = __fma_rn(-2., dev[1], dev[0]) + dev[2];
-    double s1 = f64_third(t * t * 13);
-    t = __fma_rn(-4., dev[1], dev[0]) + three2;
-    s1 = s1 + t * t;  // four times the reference's value
-    t = __fma_rn(-2., dev[2], dev[1]) + dev[3];
-    double s2 = f64_third(t * t * 13);
-    t = dev[1] - dev[3];
-    s2 = s2 + t * t;
-    t = __fma_rn(-2., dev[3], dev[2]) + dev[4];
-    double s3 = f64_third(t * t * 13);
-    t = __fma_rn(-4., dev[3], three2) + dev[4];
-    s3 = s3 + t * t;
-    t = __fma_rn(.25, s1, eps);
-    const double alpha1 = f64_div(.1, t * t);
-    t = __fma_rn(.25, s2, eps);
-    const double alpha2 = f64_div(.6, t * t);
-    t = __fma_rn(.25, s3, eps);
-    const double alpha3 = f64_div(.3, t * t);
+    // s1, s2, s3: four times the reference's values
+    const double s1 = f64_times_third<13>(f64_sqr(__fma_rn(-2., dev[1], dev[0]) + dev[2])) +
+                      f64_sqr(__fma_rn(-4., dev[1], dev[0]) + three2);
+    const double s2 = f64_times_third<13>(f64_sqr(__fma_rn(-2., dev[2], dev[1]) + dev[3])) +
+                      f64_sqr(dev[1] - dev[3]);
+    const double s3 = f64_times_third<13>(f64_sqr(__fma_rn(-2., dev[3], dev[2]) + dev[4])) +
+                      f64_sqr(__fma_rn(-4., dev[3], three2) + dev[4]);
+    const double alpha1 = f64_div(.1, f64_sqr<true>(__fma_rn(.25, s1, eps)));
+    const double alpha2 = f64_div(.6, f64_sqr<true>(__fma_rn(.25, s2, eps)));
+    const double alpha3 = f64_div(.3, f64_sqr<true>(__fma_rn(.25, s3, eps)));
     const double sum = alpha1 + alpha2 + alpha3;
-    return f64_div(alpha1 * phix1 + alpha2 * phix2 + alpha3 * phix3, sum) * invdx;
+    return f64_mul(f64_div(f64_mul(alpha1, phix1) + f64_mul(alpha2, phix2) + f64_mul(alpha3, phix3), sum), invdx);
 }
 
 // An FP32 value within 2^-23 of v (truncated), v zero or in [2^-100, 2^60).
@@ -312,8 +312,9 @@ __device__ __forceinline__ int weno_sign(float d0, float d1, float d2, float d3,
 // one, it adds +0 to a sum that is never negative, and is left out.  On a smooth field that is one of the two sides
 // of each axis.  `plain` (h outside [2^-60, 2^60]) sends every derivative to the plain form.
 //
-// Bound by the FP64 pipe (at 128^3 a stage went from 4.39 ms, 1043 FP64 operations a cell and half of them inside
-// divisions, to 1.11 ms, about 200); DRAM carries 16-24 bytes a cell, 1% of its rate.
+// Bound by the FP64 pipe (83% busy, the integer pipes 50%): at 128^3 a stage went from 4.39 ms, 1043 FP64 operations a
+// cell and half of them inside divisions, to 1.11 ms with quotients off the pipe and 0.69 ms with products off it too
+// (168); DRAM carries 16-24 bytes a cell, 1% of its rate.
 template <int STAGE>
 __global__ void __launch_bounds__(256) k_reinit_advance(Dims d, double h, double invdx, double dt, int plain,
                                                         const double *__restrict__ f, const double *phi, double *out) {
@@ -356,17 +357,19 @@ __global__ void __launch_bounds__(256) k_reinit_advance(Dims d, double h, double
             const double dev[5] = {left ? dv[0] : dv[5], left ? dv[1] : dv[4], left ? dv[2] : dv[3],
                                    left ? dv[3] : dv[2], left ? dv[4] : dv[1]};
             const double w = fast ? weno_fast(dev, invdx) : weno_plain(dev[0], dev[1], dev[2], dev[3], dev[4], invdx);
-            const double t = left == neg ? (w < 0. ? w : 0.) : dmax0(w, 0.);
-            sum += t * t;
+            // min(w, 0) or std::max(w, 0) by the side and the sign of phi; the tests on the bits, off the FP64 pipe
+            const double t = below0(w) == (left == neg) ? w : 0.;
+            sum += fast ? f64_sqr(t) : t * t;
             if (left)
                 left = false;
             else
                 right = false;
         }
     }
-    sum = sqrt(sum);
+    sum = f64_in_range(sum, -600, 600) && !f64_is_zero(sum) ? f64_sqrt(sum) : sqrt(sum);
     const double sp = h * sum;
-    const double len = sqrt(fc * fc + sp * sp);
+    const double len2 = fc * fc + sp * sp;
+    const double len = f64_in_range(len2, -600, 600) && !f64_is_zero(len2) ? f64_sqrt(len2) : sqrt(len2);
     const double sgn = f64_in_range(fc, -300, 300) && f64_in_range(len, -300, 300) && !f64_is_zero(len)
                            ? f64_div(fc, len)
                            : fc / len;

@@ -10,14 +10,13 @@
 
 #define SF_F64_TEST_RCP test_rcp
 namespace sf {
-float test_rcp(float x);
+float test_rcp(float y);
 }
 #include "sf_f64_int.cuh"
 
 static int g_off = 0;
 namespace sf {
-float test_rcp(float x) {
-    float y = 1.0f / x;
+float test_rcp(float y) {
     for (int i = 0; i < std::abs(g_off); i++) y = std::nextafterf(y, g_off > 0 ? 2.f : 0.f);
     return y;
 }
@@ -65,6 +64,20 @@ int main() {
         }
         check("mul", sf::f64_mul(a, b), a * b, a, b);
         check("third", sf::f64_third(a), a / 3, a, 0);
+        check("times_third<5>", sf::f64_times_third<5>(a), a * 5 / 3, a, 0);
+        check("times_third<7>", sf::f64_times_third<7>(a), a * 7 / 3, a, 0);
+        check("times_third<11>", sf::f64_times_third<11>(a), a * 11 / 3, a, 0);
+        check("times_third<13>", sf::f64_times_third<13>(a), a * 13 / 3, a, 0);
+        check("sqr", sf::f64_sqr(a), a * a, a, a);
+        if (a != 0 && b != 0) check("mul nonzero", sf::f64_mul<true>(a, b), a * b, a, b);
+        if (a != 0) {
+            const double r = std::fabs(a);
+            check("sqrt", sf::f64_sqrt(r), std::sqrt(r), r, 0);
+            // a radicand next to a square and next to the square of a midpoint
+            const double w = std::sqrt(r), near = w * w, next = std::nextafter(w, 1e300) * w;
+            check("sqrt", sf::f64_sqrt(near), std::sqrt(near), near, 0);
+            check("sqrt", sf::f64_sqrt(next), std::sqrt(next), next, 0);
+        }
         const bool in = a == 0 || (std::fabs(a) >= 0x1p-100 && std::fabs(a) < 0x1p60);
         n++;
         bad += sf::f64_in_range(a, -100, 60) != in;
