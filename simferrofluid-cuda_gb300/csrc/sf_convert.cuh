@@ -21,8 +21,8 @@ namespace sf {
 
 SF_CONV_FN void f64_words(double v, uint32_t &hi, uint32_t &lo) {
 #if defined(__CUDA_ARCH__)
-    hi = (uint32_t)__double2hiint(v);
-    lo = (uint32_t)__double2loint(v);
+    // opaque to the compiler, which would turn a zero test on the words back into an FP64 comparison
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
 #else
     uint64_t b;
     std::memcpy(&b, &v, 8);

@@ -208,7 +208,9 @@ __global__ void __launch_bounds__(256) k_advect_velocity(Dims d, int a, Origin o
 
 // v < 0 on the bits (false for NaN and -0)
 __device__ __forceinline__ bool below0(double v) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    uint32_t h, l;
+    f64_words(v, h, l);
+    const uint64_t b = ((uint64_t)h << 32) | l;
     return b > 0x8000000000000000ULL && b <= 0xfff0000000000000ULL;
 }
 
@@ -258,10 +260,16 @@ __device__ __noinline__ double weno_plain(double d0, double d1, double d2, doubl
 // Measured per warp and SM: an FP64 instruction takes 19 clocks, the compiler's division 137, its x / 3 140 and its
 // square root 143; on the integer pipe, beside it, a product takes 12-14, a division 27, a third 9, a root 24.
 __device__ __forceinline__ double weno_fast(const double dev[5], double invdx) {
-    long long big = 0;
+    // the magnitudes as integers (an absolute value of doubles would take the FP64 pipe)
+    uint64_t big = 0;
 #pragma unroll
-    for (int j = 0; j < 5; j++) big = max(big, __double_as_longlong(dev[j]) & 0x7fffffffffffffffLL);
-    const double top = __longlong_as_double(big);
+    for (int j = 0; j < 5; j++) {
+        uint32_t h, l;
+        f64_words(dev[j], h, l);
+        const uint64_t v = ((uint64_t)(h & 0x7fffffffu) << 32) | l;
+        big = v > big ? v : big;
+    }
+    const double top = f64_from_words((uint32_t)(big >> 32), (uint32_t)big);
     const double eps = f64_mul<true>(f64_sqr<true>(top), 1e-6);
     const double third1 = f64_third(dev[1]), third2 = f64_third(dev[2]), third3 = f64_third(dev[3]);
     const double phix1 = __fma_rn(.5, f64_times_third<11>(dev[2]),
@@ -285,14 +293,21 @@ __device__ __forceinline__ double weno_fast(const double dev[5], double invdx) {
 
 // An FP32 value within 2^-23 of v (truncated), v zero or in [2^-100, 2^60).
 __device__ __forceinline__ float f32_near(double v) {
-    const uint32_t h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
+    uint32_t h, l;
+    f64_words(v, h, l);
     const uint32_t m = (h & 0x7fffffffu) - (896u << 20);  // exponent rebased
     return (h << 1) == 0u ? 0.f : __uint_as_float(((m << 3) | (l >> 29)) | (h & 0x80000000u));
 }
 
-// Sign of the WENO derivative when FP32 arithmetic can tell: +1 / -1 when its three candidate derivatives clearly
-// share it (each exceeds 2^-19 of the sum of its terms' magnitudes; the truncations and roundings here stay
-// below 2^-21 of it, so the FP64 values share the sign too, and so does their convex combination); 0 otherwise.
+// Sign of the WENO derivative of differences d0..d4 (FP32, truncated) when FP32 arithmetic can tell: +1 / -1, else 0.
+//   * Its three candidate derivatives clearly share a sign (each exceeds 2^-19 of the sum of its terms' magnitudes;
+//     truncations and roundings stay below 2^-21 of it): then so does their convex combination.
+//   * Otherwise the weights are formed in FP32 from the differences scaled to a largest magnitude in [1, 2).  The
+//     scaled differences are off by at most 2^-22, a smoothness measure's terms by 2^-18, and since the measure has
+//     1e-6 of the largest square added, the sum is off by at most 0.4% and a weight (its inverse square) by 1%; a
+//     candidate is off by 2^-19.  A combination above 5% of its terms' magnitudes and 2^-17 of the weights keeps its
+//     sign in FP64.
+// The second test takes 5% of the FP64 instructions off a rippled 128^3 field (168 to 160 a warp and stage).
 __device__ __forceinline__ int weno_sign(float d0, float d1, float d2, float d3, float d4) {
     const float tol = 1.9073486e-6f;
     const float a = d0 * (1.f / 3.f), b = d1 * (-7.f / 6.f), c = d2 * (11.f / 6.f);
@@ -301,8 +316,32 @@ __device__ __forceinline__ int weno_sign(float d0, float d1, float d2, float d3,
     const float p2 = f + g + h, e2 = (fabsf(f) + fabsf(g) + fabsf(h)) * tol;
     const float l = d2 * (1.f / 3.f), m = d3 * (5.f / 6.f), n = d4 * (-1.f / 6.f);
     const float p3 = l + m + n, e3 = (fabsf(l) + fabsf(m) + fabsf(n)) * tol;
-    return (p1 > e1 && p2 > e2 && p3 > e3) ? 1 : ((p1 < -e1 && p2 < -e2 && p3 < -e3) ? -1 : 0);
+    if (p1 > e1 && p2 > e2 && p3 > e3) return 1;
+    if (p1 < -e1 && p2 < -e2 && p3 < -e3) return -1;
+    const float top = fmaxf(fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3))), fabsf(d4));
+    const float sc = __uint_as_float((254u << 23) - (__float_as_uint(top) & 0x7f800000u));  // 2^-exponent
+    const float x0 = d0 * sc, x1 = d1 * sc, x2 = d2 * sc, x3 = d3 * sc, x4 = d4 * sc;
+    const float eps = 1e-6f * (top * sc) * (top * sc);
+    const float t1 = x0 - 2.f * x1 + x2, q1 = x0 - 4.f * x1 + 3.f * x2;
+    const float t2 = x1 - 2.f * x2 + x3, q2 = x1 - x3;
+    const float t3 = x2 - 2.f * x3 + x4, q3 = 3.f * x2 - 4.f * x3 + x4;
+    const float s1 = t1 * t1 * (13.f / 12.f) + q1 * q1 * .25f + eps;
+    const float s2 = t2 * t2 * (13.f / 12.f) + q2 * q2 * .25f + eps;
+    const float s3 = t3 * t3 * (13.f / 12.f) + q3 * q3 * .25f + eps;
+    const float a1 = __fdividef(.1f, s1 * s1), a2 = __fdividef(.6f, s2 * s2), a3 = __fdividef(.3f, s3 * s3);
+    const float n1 = a1 * (p1 * sc), n2 = a2 * (p2 * sc), n3 = a3 * (p3 * sc);
+    const float num = n1 + n2 + n3;
+    const float err = .05f * (fabsf(n1) + fabsf(n2) + fabsf(n3)) + 7.6293945e-6f * (a1 + a2 + a3);
+    return num > err ? 1 : (num < -err ? -1 : 0);
 }
+
+// Tile of the step kernel: 16 (z) x 4 (y) x 4 (x) cells, one thread each.  The differences along the three axes that
+// its stencils read are formed once, into shared memory: 9 x 4 x 16 along x, 4 x 9 x 16 along y, 4 x 4 x 21 along z,
+// 5.8 a cell instead of 18.
+constexpr int kRx = 4, kRy = 4, kRz = 16;
+constexpr int kRdx = (kRx + 5) * kRy * kRz, kRdy = kRx * (kRy + 5) * kRz, kRdz = kRx * kRy * (kRz + 5);
+
+__device__ __forceinline__ int clamp_to(int v, int last) { return v < 0 ? 0 : (v > last ? last : v); }
 
 // Reinitialization::Advance (core/Reinitialization.cpp:48-74): one explicit step of the reinitialisation equation
 // with Godunov upwinding of the WENO5 derivatives (clamped stencils at the grid ends), and the TVD-RK3 combination
@@ -310,62 +349,108 @@ __device__ __forceinline__ int weno_sign(float d0, float d1, float d2, float d3,
 //
 // A derivative enters only with one sign (Godunov): where its sign is known without evaluating it and is the other
 // one, it adds +0 to a sum that is never negative, and is left out.  On a smooth field that is one of the two sides
-// of each axis.  `plain` (h outside [2^-60, 2^60]) sends every derivative to the plain form.
+// of each axis; the few cells that need both (2% an axis next to kinks, but half of the warps hold one) leave the
+// second to a queue that the block's threads then share.  `plain` (h outside [2^-60, 2^60]) sends every derivative
+// to the plain form.
 //
-// Bound by the FP64 pipe (83% busy, the integer pipes 50%): at 128^3 a stage went from 4.39 ms, 1043 FP64 operations a
-// cell and half of them inside divisions, to 1.11 ms with quotients off the pipe and 0.69 ms with products off it too
-// (168); DRAM carries 16-24 bytes a cell, 1% of its rate.
+// Bound by the FP64 pipe, then by the integer pipes; DRAM carries 16-24 bytes a cell, 1% of its rate.  A stage at
+// 128^3: 4.39 ms with every operation on the FP64 pipe (1043 a cell, half of them inside divisions), 1.11 ms with
+// quotients off it, 0.69 ms with products off it too (168 instructions a warp), 0.48 ms with the differences shared, the
+// second sides queued and magnitudes taken on the words (108; the pipe 77% busy).  64 registers: four blocks an SM
+// instead of three are worth 2.5%.
 template <int STAGE>
-__global__ void __launch_bounds__(256) k_reinit_advance(Dims d, double h, double invdx, double dt, int plain,
+__global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, double invdx, double dt, int plain,
                                                         const double *__restrict__ f, const double *phi, double *out) {
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= d.nz || j >= d.ny) return;
+    __shared__ double diff[kRdx + kRdy + kRdz];
+    __shared__ double part[6][256];  // squares of the derivatives taken, minus (or only) and plus side of each axis
+    __shared__ uint16_t queue[3 * 256];
+    __shared__ int queued;
+    const int tid = threadIdx.x, lz = tid & 15, ly = (tid >> 4) & 3, lx = tid >> 6;
+    const int k0 = blockIdx.x * kRz, j0 = blockIdx.y * kRy, i0 = blockIdx.z * kRx;
+    const int lastx = d.nx - 1, lasty = d.ny - 1, lastz = d.nz - 1;
+    if (tid == 0) queued = 0;
+    for (int e = tid; e < kRdx; e += 256) {  // [m][y][z], m the lower x plane + 3
+        const int m = i0 + (e >> 6) - 3;
+        const long long r = cid(d, 0, clamp_to(j0 + ((e >> 4) & 3), lasty), clamp_to(k0 + (e & 15), lastz));
+        const long long sx = (long long)d.ny * d.nz;
+        diff[e] = f[r + clamp_to(m + 1, lastx) * sx] - f[r + clamp_to(m, lastx) * sx];
+    }
+    for (int e = tid; e < kRdy; e += 256) {  // [x][m][z]
+        const int r = e >> 4, x = r / (kRy + 5), m = j0 + r - x * (kRy + 5) - 3;
+        const long long c = cid(d, clamp_to(i0 + x, lastx), 0, clamp_to(k0 + (e & 15), lastz));
+        diff[kRdx + e] = f[c + (long long)clamp_to(m + 1, lasty) * d.nz] - f[c + (long long)clamp_to(m, lasty) * d.nz];
+    }
+    for (int e = tid; e < kRdz; e += 256) {  // [x][y][m]
+        const int r = e / (kRz + 5), m = k0 + e - r * (kRz + 5) - 3;
+        const long long c = cid(d, clamp_to(i0 + (r >> 2), lastx), clamp_to(j0 + (r & 3), lasty), 0);
+        diff[kRdx + kRdy + e] = f[c + clamp_to(m + 1, lastz)] - f[c + clamp_to(m, lastz)];
+    }
+    __syncthreads();
+    const int k = k0 + lz, j = j0 + ly, i = i0 + lx;
+    const bool cell = i <= lastx && j <= lasty && k <= lastz;
     const long long c = cid(d, i, j, k);
-    const double fc = f[c];
-    const bool neg = fc < 0;
-    double sum = 0;
+    const double fc = cell ? f[c] : 0.;
+    const bool neg = below0(fc);
+    if (cell) {
 #pragma unroll 1
-    for (int a = 0; a < 3; a++) {
-        const int at = a == 0 ? i : (a == 1 ? j : k), last = (a == 0 ? d.nx : (a == 1 ? d.ny : d.nz)) - 1;
-        const long long st = a == 0 ? (long long)d.ny * d.nz : (a == 1 ? d.nz : 1);
-        double v[7], dv[6];
-#pragma unroll
-        for (int q = 0; q < 7; q++) {
-            const int m = at + q - 3;
-            v[q] = f[c + ((m < 0 ? 0 : (m > last ? last : m)) - at) * st];
-        }
-        bool fast = !plain;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            dv[q] = v[q + 1] - v[q];
-            fast = fast && f64_in_range(dv[q], -100, 60);
-        }
-        bool left = true, right = true;
-        if (fast) {
+        for (int a = 0; a < 3; a++) {
+            const double *dd = diff + (a == 0 ? tid : (a == 1 ? kRdx + (lx * (kRy + 5) + ly) * kRz + lz
+                                                              : kRdx + kRdy + (lx * kRy + ly) * (kRz + 5) + lz));
+            const int st = a == 0 ? kRy * kRz : (a == 1 ? kRz : 1);
+            double dv[6];
             float w[6];
+            bool fast = !plain;
 #pragma unroll
-            for (int q = 0; q < 6; q++) w[q] = f32_near(dv[q]);
-            const int out_side = neg ? 1 : -1;  // the sign with which the minus derivative drops out
-            left = weno_sign(w[0], w[1], w[2], w[3], w[4]) != out_side &&
-                   !(w[0] == 0.f && w[1] == 0.f && w[2] == 0.f && w[3] == 0.f && w[4] == 0.f);
-            right = weno_sign(w[5], w[4], w[3], w[2], w[1]) != -out_side &&
-                    !(w[5] == 0.f && w[4] == 0.f && w[3] == 0.f && w[2] == 0.f && w[1] == 0.f);
-        }
-        // the minus side first, as the reference adds them; a thread that needs one side takes one turn
-#pragma unroll 1
-        while (left || right) {
-            const double dev[5] = {left ? dv[0] : dv[5], left ? dv[1] : dv[4], left ? dv[2] : dv[3],
-                                   left ? dv[3] : dv[2], left ? dv[4] : dv[1]};
-            const double w = fast ? weno_fast(dev, invdx) : weno_plain(dev[0], dev[1], dev[2], dev[3], dev[4], invdx);
-            // min(w, 0) or std::max(w, 0) by the side and the sign of phi; the tests on the bits, off the FP64 pipe
-            const double t = below0(w) == (left == neg) ? w : 0.;
-            sum += fast ? f64_sqr(t) : t * t;
-            if (left)
-                left = false;
-            else
-                right = false;
+            for (int q = 0; q < 6; q++) {
+                dv[q] = dd[q * st];
+                fast = fast && f64_in_range(dv[q], -100, 60);
+                w[q] = f32_near(dv[q]);
+            }
+            double p0 = 0., p1 = 0.;
+            if (fast) {
+                const int drops = neg ? 1 : -1;  // the sign with which the minus derivative drops out
+                const bool left = weno_sign(w[0], w[1], w[2], w[3], w[4]) != drops &&
+                                  !(w[0] == 0.f && w[1] == 0.f && w[2] == 0.f && w[3] == 0.f && w[4] == 0.f);
+                const bool right = weno_sign(w[5], w[4], w[3], w[2], w[1]) != -drops &&
+                                   !(w[5] == 0.f && w[4] == 0.f && w[3] == 0.f && w[2] == 0.f && w[1] == 0.f);
+                if (left || right) {
+                    // read again rather than selected: a select of doubles takes the FP64 pipe
+                    const double *s0 = left ? dd : dd + 5 * st;
+                    const int sst = left ? st : -st;
+                    const double dev[5] = {s0[0], s0[sst], s0[2 * sst], s0[3 * sst], s0[4 * sst]};
+                    const double v = weno_fast(dev, invdx);
+                    // min(v, 0) or std::max(v, 0) by the side and the sign of phi; tested on the bits
+                    if (below0(v) == (left == neg)) p0 = f64_sqr(v);
+                }
+                if (left && right) queue[atomicAdd(&queued, 1)] = (uint16_t)(a * 256 + tid);
+            } else {
+                double v = weno_plain(dv[0], dv[1], dv[2], dv[3], dv[4], invdx);
+                if (below0(v) == neg) p0 = v * v;
+                v = weno_plain(dv[5], dv[4], dv[3], dv[2], dv[1], invdx);
+                if (below0(v) != neg) p1 = v * v;
+            }
+            part[2 * a][tid] = p0;
+            part[2 * a + 1][tid] = p1;
         }
     }
+    __syncthreads();
+    for (int e = tid; e < queued; e += 256) {
+        const int a = queue[e] >> 8, t = queue[e] & 255;
+        const int tz = t & 15, ty = (t >> 4) & 3, tx = t >> 6;
+        const double *dd = diff + (a == 0 ? t : (a == 1 ? kRdx + (tx * (kRy + 5) + ty) * kRz + tz
+                                                        : kRdx + kRdy + (tx * kRy + ty) * (kRz + 5) + tz));
+        const int st = a == 0 ? kRy * kRz : (a == 1 ? kRz : 1);
+        const double dev[5] = {dd[5 * st], dd[4 * st], dd[3 * st], dd[2 * st], dd[st]};
+        const double v = weno_fast(dev, invdx);
+        const double fo = f[cid(d, i0 + tx, j0 + ty, k0 + tz)];
+        if (below0(v) != below0(fo)) part[2 * a + 1][t] = f64_sqr(v);
+    }
+    __syncthreads();
+    if (!cell) return;
+    double sum = part[0][tid];  // minus side first, as the reference adds them; a zero would leave the sum as it is
+#pragma unroll
+    for (int q = 1; q < 6; q++)
+        if (!f64_is_zero(part[q][tid])) sum += part[q][tid];
     sum = f64_in_range(sum, -600, 600) && !f64_is_zero(sum) ? f64_sqrt(sum) : sqrt(sum);
     const double sp = h * sum;
     const double len2 = fc * fc + sp * sp;
@@ -382,6 +467,10 @@ __global__ void __launch_bounds__(256) k_reinit_advance(Dims d, double h, double
         const double s = phi[c] + step * 2;
         out[c] = f64_in_range(s, -1000, 1000) ? f64_third(s) : s / 3;
     }
+}
+
+inline dim3 reinit_grid(const Dims &d) {
+    return dim3((d.nz + kRz - 1) / kRz, (d.ny + kRy - 1) / kRy, (d.nx + kRx - 1) / kRx);
 }
 
 inline dim3 cell_grid(const Dims &d) { return dim3((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx); }
@@ -405,9 +494,9 @@ void launch_reinitialize(cudaStream_t st, const Dims &d, double h, double *phi, 
     const double dt = h * .5, invdx = 1 / h;
     const int plain = !(h >= 0x1p-60 && h <= 0x1p60);
     for (int it = 0; it < max_steps; it++) {
-        k_reinit_advance<0><<<cell_grid(d), blk2(), 0, st>>>(d, h, invdx, dt, plain, phi, nullptr, p1);
-        k_reinit_advance<1><<<cell_grid(d), blk2(), 0, st>>>(d, h, invdx, dt, plain, p1, phi, p2);
-        k_reinit_advance<2><<<cell_grid(d), blk2(), 0, st>>>(d, h, invdx, dt, plain, p2, phi, phi);
+        k_reinit_advance<0><<<reinit_grid(d), 256, 0, st>>>(d, h, invdx, dt, plain, phi, nullptr, p1);
+        k_reinit_advance<1><<<reinit_grid(d), 256, 0, st>>>(d, h, invdx, dt, plain, p1, phi, p2);
+        k_reinit_advance<2><<<reinit_grid(d), 256, 0, st>>>(d, h, invdx, dt, plain, p2, phi, phi);
     }
 }
 
