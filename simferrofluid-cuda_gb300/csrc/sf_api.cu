@@ -30,8 +30,9 @@ struct Ctx {
     Dims mag_dims{0, 0, 0, 0};
     // staging buffers for the host-pointer entry points
     DevBuf phi, frac[3], vel[3], us[3], jump[3], hext[3], H[3], cells;
-    // velocity pipeline after the projection: extrapolation masks, enforce's copy of the old velocity, normals
-    DevBuf mask[6], old[3], normal[3];
+    // velocity pipeline after the projection: extrapolation validity bits, enforce's lists of
+    // faces (their new values in old) and its counters, normals; old also holds advection's copy of the velocity
+    DevBuf mask[6], old[3], enf[4], normal[3];
     // interface coupling: mesh vertices, vertex values and edge marks
     DevBuf vpos, vnrm, vval, kappa, edge[3];
     // level-set operations: two scratch cell fields
@@ -492,13 +493,13 @@ sf_status extrapolate_impl(Ctx *c, const sf_grid *g, double *const vel[3], const
     Faces ff{};
     if ((s = stage_vel(c, g, vel, dev, dvel, h2d)) != SF_OK) return s;
     if ((s = stage_in(c, c->phi, phi, d.n, dev, &dphi, h2d)) != SF_OK) return s;
-    uint8_t *m0[3], *m1[3];
+    uint32_t *m0[3], *m1[3];
     for (int a = 0; a < 3; a++) {
         if ((s = stage_in(c, c->frac[a], frac[a], face_count(g, a), dev, &ff.p[a], h2d)) != SF_OK) return s;
-        CK(c->mask[a].ensure((size_t)face_count(g, a)));
-        CK(c->mask[3 + a].ensure((size_t)face_count(g, a)));
-        m0[a] = (uint8_t *)c->mask[a].get();
-        m1[a] = (uint8_t *)c->mask[3 + a].get();
+        CK(c->mask[a].ensure(extrapolate_bits_bytes(d, a)));
+        CK(c->mask[3 + a].ensure(extrapolate_bits_bytes(d, a)));
+        m0[a] = (uint32_t *)c->mask[a].get();
+        m1[a] = (uint32_t *)c->mask[3 + a].get();
     }
     launch_extrapolate(c->st, d, dphi, ff, dvel, m0, m1, clear_val, max_steps);
     CK(cudaGetLastError());
@@ -670,19 +671,23 @@ sf_status enforce_impl(Ctx *c, const sf_grid *g, double *const vel[3], const dou
     const Dims d = make_dims(g->nx, g->ny, g->nz);
     long long h2d = 0;
     double *dvel[3];
-    Faces ff{}, fn{}, fus{}, fold{};
+    Faces ff{}, fn{}, fus{};
+    uint32_t *face[3];
+    double *value[3];
     if ((s = stage_vel(c, g, vel, dev, dvel, h2d)) != SF_OK) return s;
     for (int a = 0; a < 3; a++) {
         const long long nf = face_count(g, a);
         if ((s = stage_in(c, c->frac[a], frac[a], nf, dev, &ff.p[a], h2d)) != SF_OK) return s;
         if ((s = stage_in(c, c->normal[a], normal[a], nf, dev, &fn.p[a], h2d)) != SF_OK) return s;
         if ((s = stage_in(c, c->us[a], us ? us[a] : nullptr, nf, dev, &fus.p[a], h2d)) != SF_OK) return s;
-        // Collider::Enforce interpolates the velocity as it was before the call
+        // Collider::Enforce interpolates the velocity as it was before the call: new values wait in a list
         CK(c->old[a].ensure(8 * (size_t)nf));
-        launch_copy(c->st, nf, dvel[a], (double *)c->old[a].get());
-        fold.p[a] = (const double *)c->old[a].get();
+        CK(c->enf[a].ensure(4 * (size_t)nf));
+        value[a] = (double *)c->old[a].get();
+        face[a] = (uint32_t *)c->enf[a].get();
     }
-    launch_enforce(c->st, d, g->origin, g->h, fold, fus, fn, ff, dvel);
+    CK(c->enf[3].ensure(3 * sizeof(unsigned)));
+    launch_enforce(c->st, d, g->origin, g->h, fus, fn, ff, dvel, face, value, (unsigned *)c->enf[3].get());
     CK(cudaGetLastError());
     return unstage_vel(c, g, vel, dev, dvel);
 }

@@ -13,8 +13,8 @@
 //
 // Methods: a quotient is found by long division in three digits (two from a 24-bit reciprocal in FP32, one from the
 // exact integer remainder), and the exact integer remainder decides the rounding, so the result does not depend on
-// the reciprocal's last bits; a square root goes the same way; a third is floor((N + 1) / 3) of the scaled significand N, which is its nearest
-// integer because N mod 3 is never a half.
+// the reciprocal's last bits; a square root goes the same way; a third is floor((N + 1) / 3) of the scaled significand
+// N, which is its nearest integer because N mod 3 is never a half.
 #pragma once
 #include <cmath>
 
@@ -58,7 +58,9 @@ SF_CONV_FN int f32_nearest_int(float a) { return (int)std::nearbyintf(a); }
 SF_CONV_FN double f64_fma(double a, double b, double c) { return std::fma(a, b, c); }
 SF_CONV_FN uint32_t mulhi_u32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 // the high / low word of (hi:lo) shifted left / right by n in [0, 31]
-SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) { return (uint32_t)(((((uint64_t)hi << 32) | lo) << n) >> 32); }
+SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) {
+    return (uint32_t)(((((uint64_t)hi << 32) | lo) << n) >> 32);
+}
 SF_CONV_FN uint32_t shf_r(uint32_t lo, uint32_t hi, int n) { return (uint32_t)((((uint64_t)hi << 32) | lo) >> n); }
 #endif
 
@@ -246,5 +248,78 @@ SF_CONV_FN double f64_sqrt(double a) {
     const uint32_t ex = (((ah >> 20) + 1021u - odd) >> 1) << 20;
     return f64_from_words((uint32_t)(s >> 32) + ex, (uint32_t)s);
 }
+
+// floor(x) as an integer and as a double, as (int)floor(x) gives it; |x| < 2^31, else (and for NaN) the conversion's own
+// result.  The conversions and the rounding all issue on the FP64 pipe.
+SF_CONV_FN int f64_floor(double x, double &fl) {
+    uint32_t h, l;
+    f64_words(x, h, l);
+    const int e = (int)((h >> 20) & 0x7ffu) - 1023;
+    if (e > 30) {  // infinities and NaN among them
+        const int v = (int)std::floor(x);
+        fl = (double)v;
+        return v;
+    }
+    if ((int)h >= 0) {
+        if (e < 0) {
+            fl = 0.0;
+            return 0;
+        }
+        const uint32_t m = (h & kF64Frac) | kF64One;
+        if (e <= 20) {
+            fl = f64_from_words(h & ~(kF64Frac >> e), 0u);
+            return (int)(m >> (20 - e));
+        }
+        fl = f64_from_words(h, l & ~(0xffffffffu >> (e - 20)));
+        return (int)shf_l(l, m, e - 20);
+    }
+    if (((h << 1) | l) == 0u) {
+        fl = 0.0;
+        return 0;
+    }
+    const uint32_t m = (h & kF64Frac) | kF64One;
+    uint32_t t = 0, rest = 1;
+    if (e >= 0) {
+        t = e <= 20 ? m >> (20 - e) : shf_l(l, m, e - 20);
+        rest = e < 20 ? (m << (12 + e)) | l : (e == 20 ? l : l << (e - 20));
+    }
+    const int v = -(int)t - (rest ? 1 : 0);
+    // 2^52 + 2^31 + v exactly, less the constant
+    fl = f64_from_words(0x43300000u, (uint32_t)v ^ 0x80000000u) - 4503601774854144.0;
+    return v;
+}
+
+// v <= 0, v < 0 and v < 1 on the bits, false for NaN as the comparisons are
+SF_CONV_FN bool f64_le0(double v) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    const uint64_t b = ((uint64_t)h << 32) | l;
+    return b == 0 || (b >= 0x8000000000000000ull && b <= 0xfff0000000000000ull);
+}
+SF_CONV_FN bool f64_lt0(double v) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    const uint64_t b = ((uint64_t)h << 32) | l;
+    return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
+}
+SF_CONV_FN bool f64_lt1(double v) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    return (int)h < 0 ? (h < 0xfff00000u || (h == 0xfff00000u && l == 0u)) : h < 0x3ff00000u;
+}
+SF_CONV_FN bool f64_is_one(double v) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    return h == 0x3ff00000u && l == 0u;
+}
+
+// a / b, sqrt(a) and a / 3 for any operands: the integer form where the operands allow it, else the plain one.
+SF_CONV_FN double f64_div_any(double a, double b) {
+    return f64_in_range(a, -400, 400) && f64_in_range(b, -400, 400) && !f64_is_zero(b) ? f64_div(a, b) : a / b;
+}
+SF_CONV_FN double f64_sqrt_any(double a) {
+    return !f64_lt0(a) && f64_in_range(a, -1000, 1000) && !f64_is_zero(a) ? f64_sqrt(a) : std::sqrt(a);
+}
+SF_CONV_FN double f64_third_any(double a) { return f64_in_range(a, -1000, 1000) ? f64_third(a) : a / 3; }
 
 }  // namespace sf

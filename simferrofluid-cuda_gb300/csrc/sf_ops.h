@@ -28,10 +28,14 @@ cudaError_t launch_magnetic_residual_noalloc(cudaStream_t st, const Dims &d, con
                                              double bw, const Faces &hext, double h, const double *psi,
                                              double *result);
 // Velocity pipeline after the projection (sf_post.cu).
+// bits, bits1: two sets of validity bits, extrapolate_bits_bytes(d, a) bytes for axis a.
+size_t extrapolate_bits_bytes(const Dims &d, int a);
 void launch_extrapolate(cudaStream_t st, const Dims &d, const double *phi, const Faces &frac, double *const u[3],
-                        uint8_t *const valid[3], uint8_t *const valid1[3], double clear_val, int max_steps);
-void launch_enforce(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &old,
-                    const Faces &us, const Faces &normal, const Faces &frac, double *const u[3]);
+                        uint32_t *const bits[3], uint32_t *const bits1[3], double clear_val, int max_steps);
+// face, value: room for every face of each axis; count: three counters.
+void launch_enforce(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &us,
+                    const Faces &normal, const Faces &frac, double *const u[3], uint32_t *const face[3],
+                    double *const value[3], unsigned *count);
 void launch_vertex_pressures(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &H,
                              double chi, const double *pos, const double *nrm, long long nv, double *out);
 void launch_pressure_jump(cudaStream_t st, const Dims &d, const int32_t *const edge_mark[3], const double *kappa,

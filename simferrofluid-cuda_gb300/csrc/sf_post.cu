@@ -4,7 +4,9 @@
 //
 // Compiled with -fmad=false: each expression rounds as the reference's C++ does, so the results are bit-identical
 // to the CPU restatement on the same inputs.
+#include <algorithm>
 #include <cmath>
+#include <utility>
 
 #include "sf_f64_int.cuh"
 #include "sf_interp.cuh"
@@ -22,98 +24,223 @@ inline dim3 face_grid(const Dims &d, int a) {
 struct FDims {
     int fx, fy, fz;
 };
-__device__ __forceinline__ FDims fdims(const Dims &d, int a) { return FDims{d.nx + (a == 0), d.ny + (a == 1), d.nz + (a == 2)}; }
+__host__ __device__ __forceinline__ FDims fdims(const Dims &d, int a) {
+    return FDims{d.nx + (a == 0), d.ny + (a == 1), d.nz + (a == 2)};
+}
 __device__ __forceinline__ long long fidx(const FDims &f, int i, int j, int k) {
     return (long long)k + (long long)f.fz * ((long long)j + (long long)f.fy * i);
 }
 
-// Extrapolation validity (core/Simulation.cpp:237-240): fraction < 1 and an adjacent cell (face - e_a, face)
-// is liquid; a cell outside the grid is not liquid.
-__global__ void __launch_bounds__(256) k_extrap_init(Dims d, int a, const double *__restrict__ phi,
-                                                     const double *__restrict__ frac, uint8_t *__restrict__ valid) {
-    const FDims f = fdims(d, a);
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= f.fz || j >= f.fy) return;
-    const long long fi = fidx(f, i, j, k);
-    uint8_t v = 0;
-    if (frac[fi] < 1) {
-        int c0[3] = {i, j, k};
-        c0[a] -= 1;
-        const bool in0 = c0[0] >= 0 && c0[1] >= 0 && c0[2] >= 0;
-        const bool in1 = i < d.nx && j < d.ny && k < d.nz;
-        const bool l0 = in0 && phi[cid(d, c0[0], c0[1], c0[2])] <= 0;
-        const bool l1 = in1 && phi[cid(d, i, j, k)] <= 0;
-        v = (l0 || l1) ? 1 : 0;
-    }
-    valid[fi] = v;
-}
+// ------------------------------------------------------------------------------------------------ extrapolation
+// The validity of a face grid's faces is held as bits: row (i, j) of axis a has bit_words(fz) words, bit k & 31 of word
+// k >> 5 for face (i, j, k); bits past the row's end are zero.  At 256^3 the three axes' bits are 7 MB and stay in L2,
+// where a byte a face was 50 MB an axis and sweep.
+struct BitRows {
+    uint32_t *p[3];
+};
+__host__ __device__ __forceinline__ int bit_words(int fz) { return (fz + 31) >> 5; }
 
-// One sweep of Extrapolation::Solve (core/Extrapolation.cpp:7-28) on face grid a: invalid faces take the mean of
-// their valid 6-neighbours (order -x,+x,-y,+y,-z,+z) and become valid, or clear_val without any.  Valid faces are
-// never written in a sweep, so the in-place update reads only values of the previous sweep.
-__global__ void __launch_bounds__(256) k_extrap_step(Dims d, int a, double *__restrict__ u,
-                                                     const uint8_t *__restrict__ valid, uint8_t *__restrict__ valid1,
-                                                     double clear_val) {
-    const FDims f = fdims(d, a);
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= f.fz || j >= f.fy) return;
-    const long long fi = fidx(f, i, j, k);
-    if (valid[fi]) {
-        valid1[fi] = 1;
-        return;
-    }
-    int cnt = 0;
-    double sum = 0;
-    const int n3[3] = {f.fx, f.fy, f.fz};
+constexpr int kInitX = 2;  // x planes of a thread of k_extrap_init
+
+// Extrapolation validity (core/Simulation.cpp:237-240) of the three lower faces of cell (i, j, k): fraction < 1 and an
+// adjacent cell (face - e_a, face) is liquid; a cell outside the grid is not liquid.  A warp is one word of a row.
+// Invalid faces take clear_val here already (when there is a sweep at all): every sweep writes every invalid face,
+// and those it gives a value are written again below.  One pass over phi, the fractions and the written faces, all
+// comparisons on the bits; two x planes a thread keep enough loads in flight: 161 us at 256^3 (0.87 GB, 0.8 of the
+// measured bandwidth), 223 us with one plane, 316 us as a pass an axis.
+__global__ void __launch_bounds__(256) k_extrap_init(Dims d, const double *__restrict__ phi, Faces frac, Faces u,
+                                                     BitRows valid, double clear_val, int clear) {
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i0 = blockIdx.z * kInitX;
+    if (j > d.ny) return;  // whole warps: a warp is one row
+    const long long sx = (long long)d.ny * d.nz;
+    const bool col = j < d.ny && k < d.nz;
+    double p[kInitX + 1], py[kInitX], pz[kInitX], fr[3][kInitX];
 #pragma unroll
-    for (int o = 0; o < 6; o++) {
-        const int ax = o >> 1, s = (o & 1) ? 1 : -1;
-        int q[3] = {i, j, k};
-        q[ax] += s;
-        if (q[ax] < 0 || q[ax] >= n3[ax]) continue;
-        const long long nb = fidx(f, q[0], q[1], q[2]);
-        if (valid[nb]) {
-            sum += u[nb];
-            cnt++;
+    for (int q = 0; q <= kInitX; q++) {  // every load first: the pass is bound by their latency otherwise
+        const int i = i0 + q - 1;
+        p[q] = col && i >= 0 && i < d.nx ? phi[cid(d, i, j, k)] : 1.;
+    }
+#pragma unroll
+    for (int q = 0; q < kInitX; q++) {
+        const int i = i0 + q;
+        const bool in = i < d.nx;
+        py[q] = in && k < d.nz && j > 0 ? phi[cid(d, i, j - 1, k)] : 1.;
+        pz[q] = in && j < d.ny && k > 0 && k <= d.nz ? phi[cid(d, i, j, k - 1)] : 1.;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const FDims f = fdims(d, a);
+            fr[a][q] = i < f.fx && j < f.fy && k < f.fz ? frac.p[a][fidx(f, i, j, k)] : 1.;
         }
     }
-    if (cnt > 0) {
-        u[fi] = sum / cnt;
-        valid1[fi] = 1;
-    } else {
-        u[fi] = clear_val;
-        valid1[fi] = 0;
+#pragma unroll
+    for (int q = 0; q < kInitX; q++) {
+        const int i = i0 + q;
+        const bool liquid = f64_le0(p[q + 1]);
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const FDims f = fdims(d, a);
+            const bool row = i < f.fx && j < f.fy, face = row && k < f.fz;
+            const bool v = f64_lt1(fr[a][q]) && (liquid || f64_le0(a == 0 ? p[q] : (a == 1 ? py[q] : pz[q])));
+            if (face && !v && clear) const_cast<double *>(u.p[a])[fidx(f, i, j, k)] = clear_val;
+            const uint32_t bits = __ballot_sync(0xffffffffu, v);
+            if (row && threadIdx.x == 0 && (int)blockIdx.x < bit_words(f.fz))
+                valid.p[a][(long long)(i * f.fy + j) * bit_words(f.fz) + blockIdx.x] = bits;
+        }
     }
 }
 
-// Collider::Enforce (core/Collider.cpp:75-86) on the faces of axis a with fraction == 1: the interpolated old
-// velocity minus its normal component relative to the solid velocity (us.p[0] == nullptr: zero).
-__global__ void __launch_bounds__(256) k_enforce(Dims d, int a, Origin og, double h, double invh, Faces old,
-                                                 Faces us, Faces normal, const double *__restrict__ frac,
-                                                 double *__restrict__ u) {
+// One sweep of Extrapolation::Solve (core/Extrapolation.cpp:7-28) on the three face grids (blockIdx.z): invalid faces
+// with valid 6-neighbours take their mean (order -x,+x,-y,+y,-z,+z) and become valid.  A thread finds the new faces of
+// one word by bit operations on the words around it; the block lists its new faces and takes a thread to each, since a
+// word often holds one or two (next to a wall) and an interface fills the words of one row.  Valid faces are never
+// written in a sweep, so the in-place update reads only values of the previous sweep.  A sweep touches the bits and
+// its layer's faces alone: 98 us an axis and sweep as a pass over all faces, 62 us for the three axes with a warp
+// taking its words in turn, 32 us with the list (256^3).
+__global__ void __launch_bounds__(256) k_extrap_sweep(Dims d, Faces u, BitRows valid, BitRows valid1) {
+    __shared__ uint32_t near[6][256];
+    __shared__ uint16_t list[256 * 32];
+    __shared__ int sums[8];
+    const int a = blockIdx.z, i = blockIdx.y, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const FDims f = fdims(d, a);
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= f.fz || j >= f.fy) return;
-    const long long fi = fidx(f, i, j, k);
-    if (frac[fi] != 1.) return;
-    const int c3[3] = {i, j, k};
-    double p[3];
+    const int nw = bit_words(f.fz), e0 = blockIdx.x * 256, e = e0 + t;  // word of plane i
+    if (i >= f.fx || e0 >= f.fy * nw) return;
+    uint32_t fresh = 0;
+    if (e < f.fy * nw) {
+        const int j = e / nw, w = e - j * nw;
+        const uint32_t *b = valid.p[a] + (long long)i * f.fy * nw + e;
+        const long long sx = (long long)f.fy * nw;
+        const uint32_t m = b[0], lo = w > 0 ? b[-1] : 0u, hi = w < nw - 1 ? b[1] : 0u;
+        const uint32_t n[6] = {i > 0 ? b[-sx] : 0u,        i < f.fx - 1 ? b[sx] : 0u, j > 0 ? b[-nw] : 0u,
+                               j < f.fy - 1 ? b[nw] : 0u, (m << 1) | (lo >> 31),     (m >> 1) | (hi << 31)};
+        const int left = f.fz - 32 * w;
+        fresh = (n[0] | n[1] | n[2] | n[3] | n[4] | n[5]) & ~m & (left >= 32 ? 0xffffffffu : (1u << left) - 1u);
+        valid1.p[a][(long long)i * f.fy * nw + e] = m | fresh;
 #pragma unroll
-    for (int b = 0; b < 3; b++) p[b] = (b == a ? og.o[b] : og.o[b] + h / 2) + (double)c3[b] * h;  // PositionOf
-    double vel[3], vel0[3], n[3];
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-        vel[b] = trilerp_face(d, old.p[b], b, og.o, h, invh, p);
-        vel0[b] = us.p[0] ? trilerp_face(d, us.p[b], b, og.o, h, invh, p) : 0.0;
-        n[b] = trilerp_face(d, normal.p[b], b, og.o, h, invh, p);
+        for (int o = 0; o < 6; o++) near[o][t] = n[o];
     }
-    const double nn = sqrt((n[0] * n[0] + n[1] * n[1]) + n[2] * n[2]);  // Vector3d::normalized
-    if (nn > 0)
+    if (!__syncthreads_or(fresh != 0)) return;
+    int upto = __popc(fresh);
 #pragma unroll
-        for (int b = 0; b < 3; b++) n[b] = n[b] / nn;
-    const double dv0 = vel[0] - vel0[0], dv1 = vel[1] - vel0[1], dv2 = vel[2] - vel0[2];
-    const double dn = (dv0 * n[0] + dv1 * n[1]) + dv2 * n[2];
-    u[fi] = vel[a] - dn * n[a];
+    for (int o = 1; o < 32; o <<= 1) {
+        const int s = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += s;
+    }
+    if (lane == 31) sums[warp] = upto;
+    __syncthreads();
+    int at = upto - __popc(fresh), total = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        at += q < warp ? sums[q] : 0;
+        total += sums[q];
+    }
+    for (; fresh; fresh &= fresh - 1) list[at++] = (uint16_t)(t * 32 + __ffs(fresh) - 1);
+    __syncthreads();
+    double *v = const_cast<double *>(u.p[a]);
+    for (int q = t; q < total; q += 256) {
+        const int word = list[q] >> 5, bit = list[q] & 31, j = (e0 + word) / nw, w = e0 + word - j * nw;
+        const long long fi = fidx(f, i, j, w * 32 + bit);
+        const long long st[6] = {-(long long)f.fy * f.fz, (long long)f.fy * f.fz, -f.fz, f.fz, -1, 1};
+        double nb[6];
+#pragma unroll
+        for (int o = 0; o < 6; o++) nb[o] = near[o][word] >> bit & 1u ? v[fi + st[o]] : 0.;
+        int cnt = 0;
+        double sum = 0;
+#pragma unroll
+        for (int o = 0; o < 6; o++)
+            if (near[o][word] >> bit & 1u) {
+                sum += nb[o];
+                cnt++;
+            }
+        v[fi] = sum / cnt;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ enforcement
+// Collider::Enforce (core/Collider.cpp:75-86) changes the faces with fraction == 1 alone, one in 130 in a walled box, and
+// on the z walls one of a row's ends, so a pass with a thread a face leaves 31 lanes of a warp idle there (2.3 ms of
+// the 2.7 ms at 256^3).  Three passes instead: list the faces (all three fractions read once), evaluate the list from
+// the velocity as it was, write the values: 74, 129 (bound by the FP64 pipe) and 6 us.
+struct EnforceLists {
+    uint32_t *face[3];    // face indices with fraction == 1
+    double *value[3];     // their new velocities
+    unsigned *count;      // entries of the three lists
+};
+
+// 4096 faces a block; the order of the list's blocks is that of their arrival, which no result depends on.
+__global__ void __launch_bounds__(256) k_enforce_list(Dims d, Faces frac, EnforceLists l) {
+    __shared__ unsigned sums[8], base;
+    const int a = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const FDims f = fdims(d, a);
+    const long long n = (long long)f.fx * f.fy * f.fz, first = blockIdx.x * 4096LL + threadIdx.x;
+    if (blockIdx.x * 4096LL >= n) return;
+    unsigned hit = 0;
+#pragma unroll
+    for (int q = 0; q < 16; q++)
+        if (first + q * 256 < n && f64_is_one(frac.p[a][first + q * 256])) hit |= 1u << q;
+    if (!__syncthreads_or(hit != 0)) return;
+    const unsigned mine = __popc(hit);
+    unsigned upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += t;
+    }
+    if (lane == 31) sums[warp] = upto;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned t = 0;
+        for (int w = 0; w < 8; w++) {
+            const unsigned s = sums[w];
+            sums[w] = t;
+            t += s;
+        }
+        base = atomicAdd(l.count + a, t);
+    }
+    __syncthreads();
+    unsigned at = base + sums[warp] + upto - mine;
+    for (int q = 0; q < 16; q++)
+        if (hit >> q & 1u) l.face[a][at++] = (uint32_t)(first + q * 256);
+}
+
+// The new velocity of the listed faces: the interpolated old velocity minus its normal component relative to the solid
+// velocity (us.p[0] == nullptr: zero).
+__global__ void __launch_bounds__(128) k_enforce_eval(Dims d, Origin og, double h, double invh, Faces old, Faces us,
+                                                      Faces normal, EnforceLists l) {
+    const unsigned n0 = l.count[0], n1 = l.count[1], n2 = l.count[2];
+    const long long total = (long long)n0 + n1 + n2;
+    for (long long e = blockIdx.x * 128LL + threadIdx.x; e < total; e += gridDim.x * 128LL) {
+        const int a = e < n0 ? 0 : (e < (long long)n0 + n1 ? 1 : 2);
+        const long long at = e - (a == 0 ? 0 : (a == 1 ? n0 : (long long)n0 + n1));
+        const FDims f = fdims(d, a);
+        const uint32_t fi = l.face[a][at], row = fi / (uint32_t)f.fz;
+        const int c3[3] = {(int)(row / (uint32_t)f.fy), (int)(row % (uint32_t)f.fy), (int)(fi - row * (uint32_t)f.fz)};
+        double p[3];
+#pragma unroll
+        for (int b = 0; b < 3; b++) p[b] = (b == a ? og.o[b] : og.o[b] + h / 2) + (double)c3[b] * h;  // PositionOf
+        const GridPoint q = grid_point(og.o, h, invh, p);
+        double vel[3], vel0[3], n[3];
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const Trilinear t = trilinear(d, b, q);
+            vel[b] = t.of(old.p[b]);
+            vel0[b] = us.p[0] ? t.of(us.p[b]) : 0.0;
+            n[b] = t.of(normal.p[b]);
+        }
+        const double nn = f64_sqrt_any((n[0] * n[0] + n[1] * n[1]) + n[2] * n[2]);  // Vector3d::normalized
+        if (nn > 0)
+#pragma unroll
+            for (int b = 0; b < 3; b++) n[b] = f64_div_any(n[b], nn);
+        const double dv0 = vel[0] - vel0[0], dv1 = vel[1] - vel0[1], dv2 = vel[2] - vel0[2];
+        const double dn = (dv0 * n[0] + dv1 * n[1]) + dv2 * n[2];
+        l.value[a][at] = a == 0 ? vel[0] - dn * n[0] : (a == 1 ? vel[1] - dn * n[1] : vel[2] - dn * n[2]);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_enforce_put(EnforceLists l, Faces u) {
+    const int a = blockIdx.y;
+    const unsigned n = l.count[a];
+    for (unsigned e = blockIdx.x * 256 + threadIdx.x; e < n; e += gridDim.x * 256)
+        const_cast<double *>(u.p[a])[l.face[a][e]] = l.value[a][e];
 }
 
 // MagneticField::CalculateVertexPressures (core/MagneticField.cpp:37-48) for vertex v: H trilinear at its position,
@@ -204,14 +331,6 @@ __global__ void __launch_bounds__(256) k_advect_velocity(Dims d, int a, Origin o
     for (int b = 0; b < 3; b++) p[b] = (b == a ? og.o[b] : og.o[b] + h / 2) + (double)c3[b] * h;
     trace_rk2(d, u, og.o, h, invh, p, -dt, q);
     out[fidx(f, i, j, k)] = trilerp_face(d, ua, a, og.o, h, invh, q);
-}
-
-// v < 0 on the bits (false for NaN and -0)
-__device__ __forceinline__ bool below0(double v) {
-    uint32_t h, l;
-    f64_words(v, h, l);
-    const uint64_t b = ((uint64_t)h << 32) | l;
-    return b > 0x8000000000000000ULL && b <= 0xfff0000000000000ULL;
 }
 
 __device__ __forceinline__ double dmax0(double a, double b) { return (a < b) ? b : a; }  // std::max(a, b)
@@ -390,7 +509,7 @@ __global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, dou
     const bool cell = i <= lastx && j <= lasty && k <= lastz;
     const long long c = cid(d, i, j, k);
     const double fc = cell ? f[c] : 0.;
-    const bool neg = below0(fc);
+    const bool neg = f64_lt0(fc);
     if (cell) {
 #pragma unroll 1
         for (int a = 0; a < 3; a++) {
@@ -420,14 +539,14 @@ __global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, dou
                     const double dev[5] = {s0[0], s0[sst], s0[2 * sst], s0[3 * sst], s0[4 * sst]};
                     const double v = weno_fast(dev, invdx);
                     // min(v, 0) or std::max(v, 0) by the side and the sign of phi; tested on the bits
-                    if (below0(v) == (left == neg)) p0 = f64_sqr(v);
+                    if (f64_lt0(v) == (left == neg)) p0 = f64_sqr(v);
                 }
                 if (left && right) queue[atomicAdd(&queued, 1)] = (uint16_t)(a * 256 + tid);
             } else {
                 double v = weno_plain(dv[0], dv[1], dv[2], dv[3], dv[4], invdx);
-                if (below0(v) == neg) p0 = v * v;
+                if (f64_lt0(v) == neg) p0 = v * v;
                 v = weno_plain(dv[5], dv[4], dv[3], dv[2], dv[1], invdx);
-                if (below0(v) != neg) p1 = v * v;
+                if (f64_lt0(v) != neg) p1 = v * v;
             }
             part[2 * a][tid] = p0;
             part[2 * a + 1][tid] = p1;
@@ -443,7 +562,7 @@ __global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, dou
         const double dev[5] = {dd[5 * st], dd[4 * st], dd[3 * st], dd[2 * st], dd[st]};
         const double v = weno_fast(dev, invdx);
         const double fo = f[cid(d, i0 + tx, j0 + ty, k0 + tz)];
-        if (below0(v) != below0(fo)) part[2 * a + 1][t] = f64_sqr(v);
+        if (f64_lt0(v) != f64_lt0(fo)) part[2 * a + 1][t] = f64_sqr(v);
     }
     __syncthreads();
     if (!cell) return;
@@ -451,21 +570,16 @@ __global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, dou
 #pragma unroll
     for (int q = 1; q < 6; q++)
         if (!f64_is_zero(part[q][tid])) sum += part[q][tid];
-    sum = f64_in_range(sum, -600, 600) && !f64_is_zero(sum) ? f64_sqrt(sum) : sqrt(sum);
+    sum = f64_sqrt_any(sum);
     const double sp = h * sum;
-    const double len2 = fc * fc + sp * sp;
-    const double len = f64_in_range(len2, -600, 600) && !f64_is_zero(len2) ? f64_sqrt(len2) : sqrt(len2);
-    const double sgn = f64_in_range(fc, -300, 300) && f64_in_range(len, -300, 300) && !f64_is_zero(len)
-                           ? f64_div(fc, len)
-                           : fc / len;
+    const double sgn = f64_div_any(fc, f64_sqrt_any(fc * fc + sp * sp));
     const double step = fc + dt * sgn * (1. - sum);
     if (STAGE == 0) {
         out[c] = step;
     } else if (STAGE == 1) {
         out[c] = (phi[c] * 3 + step) / 4;
     } else {
-        const double s = phi[c] + step * 2;
-        out[c] = f64_in_range(s, -1000, 1000) ? f64_third(s) : s / 3;
+        out[c] = f64_third_any(phi[c] + step * 2);
     }
 }
 
@@ -516,26 +630,37 @@ void launch_pressure_jump(cudaStream_t st, const Dims &d, const int32_t *const e
         k_pressure_jump<<<face_grid(d, a), blk2(), 0, st>>>(d, a, em, kappa, pm, sigma, rho, 1 / h, dt, jump[a]);
 }
 
+size_t extrapolate_bits_bytes(const Dims &d, int a) {
+    const FDims f = fdims(d, a);
+    return 4 * (size_t)f.fx * f.fy * bit_words(f.fz);
+}
+
 void launch_extrapolate(cudaStream_t st, const Dims &d, const double *phi, const Faces &frac, double *const u[3],
-                        uint8_t *const valid[3], uint8_t *const valid1[3], double clear_val, int max_steps) {
-    for (int a = 0; a < 3; a++) {
-        k_extrap_init<<<face_grid(d, a), blk2(), 0, st>>>(d, a, phi, frac.p[a], valid[a]);
-        uint8_t *v0 = valid[a], *v1 = valid1[a];
-        for (int it = 0; it < max_steps; it++) {
-            k_extrap_step<<<face_grid(d, a), blk2(), 0, st>>>(d, a, u[a], v0, v1, clear_val);
-            uint8_t *t = v0;
-            v0 = v1;
-            v1 = t;
-        }
+                        uint32_t *const bits[3], uint32_t *const bits1[3], double clear_val, int max_steps) {
+    const Faces fu{{u[0], u[1], u[2]}};
+    BitRows v0{{bits[0], bits[1], bits[2]}}, v1{{bits1[0], bits1[1], bits1[2]}};
+    const dim3 nodes((d.nz + 32) / 32, (d.ny + 8) / 8, (d.nx + kInitX) / kInitX);
+    k_extrap_init<<<nodes, blk2(), 0, st>>>(d, phi, frac, fu, v0, clear_val, max_steps > 0 ? 1 : 0);
+    // words of one x plane, the most of the three axes
+    const int words = std::max((d.ny + 1) * bit_words(d.nz), d.ny * bit_words(d.nz + 1));
+    for (int it = 0; it < max_steps; it++) {
+        k_extrap_sweep<<<dim3((words + 255) / 256, d.nx + 1, 3), 256, 0, st>>>(d, fu, v0, v1);
+        std::swap(v0, v1);
     }
 }
 
-void launch_enforce(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &old,
-                    const Faces &us, const Faces &normal, const Faces &frac, double *const u[3]) {
+void launch_enforce(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &us,
+                    const Faces &normal, const Faces &frac, double *const u[3], uint32_t *const face[3],
+                    double *const value[3], unsigned *count) {
     Origin og{{origin[0], origin[1], origin[2]}};
-    const double invh = 1 / h;  // Grid::m_InvSpacing
-    for (int a = 0; a < 3; a++)
-        k_enforce<<<face_grid(d, a), blk2(), 0, st>>>(d, a, og, h, invh, old, us, normal, frac.p[a], u[a]);
+    const Faces fu{{u[0], u[1], u[2]}};
+    EnforceLists l{{face[0], face[1], face[2]}, {value[0], value[1], value[2]}, count};
+    cudaMemsetAsync(count, 0, 3 * sizeof(unsigned), st);
+    const long long most = std::max({(long long)(d.nx + 1) * d.ny * d.nz, (long long)d.nx * (d.ny + 1) * d.nz,
+                                     (long long)d.nx * d.ny * (d.nz + 1)});
+    k_enforce_list<<<dim3((unsigned)((most + 4095) / 4096), 3), 256, 0, st>>>(d, frac, l);
+    k_enforce_eval<<<152 * 4, 128, 0, st>>>(d, og, h, 1 / h, fu, us, normal, l);  // 1 / h: Grid::m_InvSpacing
+    k_enforce_put<<<dim3(152, 3), 256, 0, st>>>(l, fu);
 }
 
 }  // namespace sf

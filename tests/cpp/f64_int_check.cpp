@@ -82,6 +82,33 @@ int main() {
         n++;
         bad += sf::f64_in_range(a, -100, 60) != in;
     }
+    auto check_floor = [&](double v) {
+        double fl;
+        const int i = sf::f64_floor(v, fl), w = (int)std::floor(v);
+        n++;
+        if (i != w || fl != (double)w) {
+            if (bad < 10) std::printf("floor(%a) = %d, %a, expected %d\n", v, i, fl, w);
+            bad++;
+        }
+    };
+    auto check_order = [&](double v) {
+        n++;
+        bad += sf::f64_le0(v) != (v <= 0) || sf::f64_lt0(v) != (v < 0) || sf::f64_lt1(v) != (v < 1) ||
+               sf::f64_is_one(v) != (v == 1);
+    };
+    for (int t = 0; t < 3000000; t++) {
+        const double v = std::ldexp((double)(int64_t)rng(), -33 - (int)(rng() % 60));  // |v| < 2^30
+        check_floor(v);
+        check_floor(std::rint(v));
+        check_floor(std::nextafter(std::rint(v), rng() & 1 ? 1e9 : -1e9));
+        check_order(v);
+    }
+    for (double v : {0.0, -0.0, 0x1p-1074, -0x1p-1074, 1.0, -1.0, 0x1p30, -0x1p30, 2147483647.0, -2147483648.0 + 0.5,
+                     2147483646.5, -2147483647.0, 0x1p20, 0x1p21, -0x1p20 - 0.5, 0x1.fffffffffffffp-1}) {
+        check_floor(v);
+        check_order(v);
+    }
+    for (double v : {(double)NAN, -(double)NAN, (double)INFINITY, -(double)INFINITY, 1 + 0x1p-52, -1e308, 1e308}) check_order(v);
     const double outside[] = {0x1p-1074, -0x1p-1030, 0x1p-101, 0x1p60, -0x1p60, 1e300, INFINITY, -INFINITY, NAN};
     for (double v : outside) {
         n++;
