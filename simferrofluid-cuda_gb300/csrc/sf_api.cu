@@ -35,8 +35,8 @@ struct Ctx {
     DevBuf mask[6], old[3], enf[4], normal[3];
     // interface coupling: mesh vertices, vertex values and edge marks
     DevBuf vpos, vnrm, vval, kappa, edge[3];
-    // level-set operations: two scratch cell fields
-    DevBuf ls1, ls2;
+    // level-set operations: two scratch cell fields; advection's table of its first trace points
+    DevBuf ls1, ls2, own;
     // learned form: attached network (not owned) and its buffers; every network created on this context is
     // registered so that destroying the context first leaves the network handles safe to destroy later
     UNet *net = nullptr;
@@ -611,7 +611,8 @@ sf_status advect_levelset_impl(Ctx *c, const sf_grid *g, double *phi, const doub
         if ((s = stage_in(c, c->vel[a], vel[a], face_count(g, a), dev, &fu.p[a], h2d)) != SF_OK) return s;
     CK(c->ls1.ensure(8 * (size_t)d.n));
     double *out = (double *)c->ls1.get();
-    launch_advect_levelset(c->st, d, g->origin, g->h, fu, dt, dphi, out);
+    CK(c->own.ensure(advect_table_bytes(d)));
+    launch_advect_levelset(c->st, d, g->origin, g->h, fu, dt, dphi, out, c->own.get());
     launch_copy(c->st, d.n, out, dphi);  // Advection::Solve replaces the field with the advected one
     CK(cudaGetLastError());
     if (!dev) CK(cudaMemcpyAsync(phi, dphi, 8 * (size_t)d.n, cudaMemcpyDeviceToHost, c->st));
@@ -636,7 +637,8 @@ sf_status advect_velocity_impl(Ctx *c, const sf_grid *g, double *const vel[3], d
         launch_copy(c->st, nf, dvel[a], (double *)c->old[a].get());
         fold.p[a] = (const double *)c->old[a].get();
     }
-    launch_advect_velocity(c->st, d, g->origin, g->h, fold, dt, dvel);
+    CK(c->own.ensure(advect_table_bytes(d)));
+    launch_advect_velocity(c->st, d, g->origin, g->h, fold, dt, dvel, c->own.get());
     CK(cudaGetLastError());
     return unstage_vel(c, g, vel, dev, dvel);
 }

@@ -187,8 +187,8 @@ SF_CONV_FN double f64_round_product(uint64_t hi, uint32_t lh, uint32_t ll, uint3
     return f64_from_words((uint32_t)(m >> 32) | sign, (uint32_t)m);
 }
 
-// a * b; each zero or normal, the product zero or normal.  NONZERO: neither operand is zero.
-template <bool NONZERO = false>
+// a * b; each zero (where A0, B0 allow it) or normal, the product zero or normal.
+template <bool A0 = true, bool B0 = true>
 SF_CONV_FN double f64_mul(double a, double b) {
     uint32_t ah, al, bh, bl;
     f64_words(a, ah, al);
@@ -201,8 +201,7 @@ SF_CONV_FN double f64_mul(double a, double b) {
     const uint32_t sign = (ah ^ bh) & kF64Sign;
     const double r = f64_round_product(hi, (uint32_t)mid, (uint32_t)p00,
                                        (ah & kF64Exp) + (bh & kF64Exp) - (1024u << 20), sign);
-    if (NONZERO) return r;
-    const bool zero = ((ah << 1) | al) == 0u || ((bh << 1) | bl) == 0u;
+    const bool zero = (A0 && ((ah << 1) | al) == 0u) || (B0 && ((bh << 1) | bl) == 0u);
     return zero ? f64_from_words(sign, 0u) : r;
 }
 
@@ -289,6 +288,14 @@ SF_CONV_FN int f64_floor(double x, double &fl) {
     return v;
 }
 
+// The distance of v's exponent above 2^lo, for a test against (hi - lo) << 20: below it exactly when 2^lo <= |v| < 2^hi.
+// Zeros are outside, so several values are tested by their largest distance.
+SF_CONV_FN uint32_t f64_above(double v, int lo) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    return (h & kF64Exp) - ((uint32_t)(lo + 1023) << 20);
+}
+
 // v <= 0, v < 0 and v < 1 on the bits, false for NaN as the comparisons are
 SF_CONV_FN bool f64_le0(double v) {
     uint32_t h, l;
@@ -311,6 +318,15 @@ SF_CONV_FN bool f64_is_one(double v) {
     uint32_t h, l;
     f64_words(v, h, l);
     return h == 0x3ff00000u && l == 0u;
+}
+
+// x / 2, or -x / 2 (NEG); x zero or normal with a normal half.
+template <bool NEG = false>
+SF_CONV_FN double f64_half(double x) {
+    uint32_t h, l;
+    f64_words(x, h, l);
+    const uint32_t r = ((h << 1) | l) == 0u ? h : h - kF64One;
+    return f64_from_words(NEG ? r ^ kF64Sign : r, l);
 }
 
 // a / b, sqrt(a) and a / 3 for any operands: the integer form where the operands allow it, else the plain one.

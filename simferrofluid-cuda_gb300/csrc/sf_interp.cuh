@@ -13,134 +13,212 @@ struct Origin {
     double o[3];  // staggered-grid corner (StaggeredGrid::GetOrigin)
 };
 
-// TriLerp::Interpolate of face grid b (size res + e_b, origin = corner + h/2 on the other axes) at p:
-// Grid::CalcLower<1> / CalcLowerFrac and clamped At().
-__device__ __forceinline__ double trilerp_face(const Dims &d, const double *__restrict__ v, int b, const double o[3],
-                                               double h, double invh, const double p[3]) {
-    const int s[3] = {d.nx + (b == 0), d.ny + (b == 1), d.nz + (b == 2)};
-    int lo[3];
-    double w[2][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const double co = a == b ? o[a] : o[a] + h / 2;  // face grid origin (core/StaggeredGrid.h:16-20)
-        lo[a] = (int)floor((p[a] - co) * invh - 0.0);
-        const double fr = (p[a] - co - (double)lo[a] * h) * invh;
-        w[0][a] = 1. - fr;
-        w[1][a] = fr;
-    }
-    double val = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const int dx = q & 1, dy = (q >> 1) & 1, dz = (q >> 2) & 1;
-        int ci[3] = {lo[0] + dx, lo[1] + dy, lo[2] + dz};
-#pragma unroll
-        for (int a = 0; a < 3; a++) ci[a] = ci[a] < 0 ? 0 : (ci[a] > s[a] - 1 ? s[a] - 1 : ci[a]);
-        const double wt = w[dx][0] * w[dy][1] * w[dz][2];
-        val += v[(long long)ci[2] + (long long)s[2] * ((long long)ci[1] + (long long)s[1] * ci[0])] * wt;
-    }
-    return val;
+// Where the FP64 pipe is the bound, the weights' products and the products with the field go to the integer pipe
+// (sf_f64_int.cuh, about 13 clocks a warp and SM against 19, side by side) and the FP64 pipe keeps the sums.
+
+// The lower cell and the weights of coordinate p on one axis of a grid with origin co -- Grid::CalcLower<1> /
+// CalcLowerFrac.
+struct AxisPoint {
+    int lo;
+    double w[2];  // lower, upper
+};
+__device__ __forceinline__ AxisPoint axis_point(double p, double co, double h, double invh) {
+    AxisPoint g;
+    const double t = p - co;
+    double fl;
+    g.lo = f64_floor(t * invh, fl);
+    const double fr = (t - fl * h) * invh;
+    g.w[0] = 1. - fr;
+    g.w[1] = fr;
+    return g;
 }
 
-// The cells and weights of a point on the staggered grids: per axis on the grid of the faces normal to it ([0], origin
-// at the corner) and on the grids of the other faces and of the cells ([1], half a cell further) -- Grid::CalcLower<1> /
-// CalcLowerFrac.  Six sets serve the three face grids.
+// A point on the staggered grids: per axis on the grid of the faces normal to it ([0], origin at the corner) and on the
+// grids of the other faces and of the cells ([1], half a cell further).  Six sets serve the three face grids.
 struct GridPoint {
-    int lo[2][3];
-    double w[2][2][3];  // [grid][lower, upper][axis]
+    AxisPoint on[2][3];
+    // every fraction is zero or in [2^-200, 2), so 1 - fraction is zero or at least 2^-53 in size: the integer products
+    // of three weights are exact to their range
+    bool plain;
+    __device__ __forceinline__ void check() {
+        plain = false;
+#pragma unroll
+        for (int s = 0; s < 2; s++)
+#pragma unroll
+            for (int a = 0; a < 3; a++) plain = plain || !f64_in_range(on[s][a].w[1], -200, 1);
+    }
 };
 __device__ __forceinline__ GridPoint grid_point(const double o[3], double h, double invh, const double p[3]) {
     GridPoint g;
 #pragma unroll
-    for (int s = 0; s < 2; s++)
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const double co = s == 0 ? o[a] : o[a] + h / 2;  // core/StaggeredGrid.h:16-20
-            const double t = p[a] - co;
-            double fl;
-            g.lo[s][a] = f64_floor(t * invh, fl);
-            const double fr = (t - fl * h) * invh;
-            g.w[s][0][a] = 1. - fr;
-            g.w[s][1][a] = fr;
-        }
+    for (int a = 0; a < 3; a++) {
+        g.on[0][a] = axis_point(p[a], o[a], h, invh);  // core/StaggeredGrid.h:16-20
+        g.on[1][a] = axis_point(p[a], o[a] + h / 2, h, invh);
+    }
+    g.check();
     return g;
 }
 
-// TriLerp::Interpolate of face grid b at a point: the eight clamped faces and their weights, shared by every field on
-// that grid.
-struct Trilinear {
-    int at[8];
-    double w[8];
-    __device__ __forceinline__ double of(const double *__restrict__ v) const {
-        double f[8];
-        uint32_t any = 0;  // magnitude bits of the eight values
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            f[q] = v[at[q]];
-            uint32_t h, l;
-            f64_words(f[q], h, l);
-            any |= (h << 1) | l;
-        }
-        // eight zeros (the air beyond the extrapolated layers, a normal's other components) sum to +0 as long as the
-        // weights are finite, which all are when the first, (1 - x)(1 - y)(1 - z), is
-        uint32_t wh, wl;
-        f64_words(w[0], wh, wl);
-        if (any == 0 && (wh & kF64Exp) != kF64Exp) return 0.;
-        // 0 + v w rounds as v w does, and takes -0 to +0 as the sum from zero does
-        double val = __fma_rn(f[0], w[0], 0.);
-#pragma unroll
-        for (int q = 1; q < 8; q++) val += f[q] * w[q];
-        return val;
-    }
-};
-__device__ __forceinline__ Trilinear trilinear(const Dims &d, int b, const GridPoint &g) {
-    const int s[3] = {d.nx + (b == 0), d.ny + (b == 1), d.nz + (b == 2)};
-    int c[2][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const int lo = g.lo[a == b ? 0 : 1][a];
-        c[0][a] = min(max(lo, 0), s[a] - 1);
-        c[1][a] = min(max(lo + 1, 0), s[a] - 1);
-    }
-    Trilinear t;
-#pragma unroll
+// TriLerp::Interpolate of a face grid of sx * sy * sz faces (fewer than 2^31) at a point: the eight clamped faces in the
+// reference's order, x fastest.  In plain FP64, for weights or values outside the integer form's range; its own function,
+// because beside the other form its instructions would be issued with their lanes off.
+__device__ __noinline__ double trilinear_plain(const double *v, int sx, int sy, int sz, AxisPoint x, AxisPoint y,
+                                               AxisPoint z) {
+    double val = 0;
+#pragma unroll 1
     for (int q = 0; q < 8; q++) {
-        const int dx = q & 1, dy = (q >> 1) & 1, dz = (q >> 2) & 1;
-        t.at[q] = c[dz][2] + s[2] * (c[dy][1] + s[1] * c[dx][0]);  // a face grid has fewer than 2^31 faces
-        t.w[q] = g.w[b == 0 ? 0 : 1][dx][0] * g.w[b == 1 ? 0 : 1][dy][1] * g.w[b == 2 ? 0 : 1][dz][2];
+        const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+        const int cx = min(max(x.lo + dx, 0), sx - 1), cy = min(max(y.lo + dy, 0), sy - 1);
+        const int cz = min(max(z.lo + dz, 0), sz - 1);
+        const double wt = (dx ? x.w[1] : x.w[0]) * (dy ? y.w[1] : y.w[0]) * (dz ? z.w[1] : z.w[0]);
+        val += v[cz + sz * (cy + sy * cx)] * wt;
     }
-    return t;
+    return val;
 }
 
-// TriCuInterp::Interpolate of the cell grid at p (core/TriCuInterp.h:12-37): CalcLower<3> = floor((p - o)/h - 1),
-// cubic Lagrange weights per axis, 64 points in (k, j, i) order, clamped At().
-__device__ __forceinline__ double tricubic_cell(const Dims &d, const double *__restrict__ f, const double o[3],
-                                                double h, double invh, const double p[3]) {
-    const int sz[3] = {d.nx, d.ny, d.nz};
-    int lo[3];
-    double w[4][3];
+// The same; `plain`: the weights are outside the integer form's range (GridPoint::plain).  A call rather than inlined: a
+// kernel that takes many samples then stays in the instruction cache (with every sample inlined, warps of the advection
+// kernels waited for instructions as often as they issued one).
+__device__ __noinline__ double trilinear(const double *v, int sx, int sy, int sz, AxisPoint x, AxisPoint y, AxisPoint z,
+                                         bool plain) {
+    const int cx[2] = {min(max(x.lo, 0), sx - 1), min(max(x.lo + 1, 0), sx - 1)};
+    const int cy[2] = {min(max(y.lo, 0), sy - 1), min(max(y.lo + 1, 0), sy - 1)};
+    const int cz[2] = {min(max(z.lo, 0), sz - 1), min(max(z.lo + 1, 0), sz - 1)};
+    double f[8];
+    uint32_t any = 0, most = 0;  // magnitude bits of the values; the largest exponent above 2^-300
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        f[q] = v[cz[q >> 2] + sz * (cy[(q >> 1) & 1] + sy * cx[q & 1])];
+        uint32_t h, l;
+        f64_words(f[q], h, l);
+        any |= (h << 1) | l;
+        most = max(most, f64_above(f[q], -300));
+    }
+    // eight zeros (the air beyond the extrapolated layers, a normal's other components) times finite weights sum to +0
+    if (any == 0 && !plain) return 0.;
+    if (plain || most >= (600u << 20)) return trilinear_plain(v, sx, sy, sz, x, y, z);
+    double val = 0.;
+#pragma unroll
+    for (int dz = 0; dz < 2; dz++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const double wt = f64_mul(f64_mul(x.w[q & 1], y.w[q >> 1]), z.w[dz]);
+            const double term = f64_mul<false>(f[4 * dz + q], wt);
+            val = 4 * dz + q == 0 ? term : val + term;
+        }
+    return f64_is_zero(val) ? 0. : val;  // the reference sums from +0, which leaves no -0
+}
+
+// Face grid b's field v at a point.
+__device__ __forceinline__ double trilinear_face(const Dims &d, int b, const GridPoint &g, const double *v) {
+    return trilinear(v, d.nx + (b == 0), d.ny + (b == 1), d.nz + (b == 2), g.on[b == 0 ? 0 : 1][0],
+                     g.on[b == 1 ? 0 : 1][1], g.on[b == 2 ? 0 : 1][2], g.plain);
+}
+
+// CalcLower<3> and the cubic Lagrange weights of one axis (core/TriCuInterp.h:12-37): lower = floor((p - o)/h - 1).
+struct CubicPoint {
+    int lo;
+    double w[4];
+};
+__device__ __forceinline__ CubicPoint cubic_point(double p, double co, double h, double invh) {
+    CubicPoint g;
+    const double t = p - co;
+    double fl;
+    g.lo = f64_floor(t * invh - 1.0, fl);
+    const double fr = (t - fl * h) * invh;
+    const double a1 = fr - 1, a2 = fr - 2, a3 = fr - 3;
+    if (f64_in_range(fr, -200, 3)) {  // and so the differences are zero or at least 2^-53 in size
+        const double f1 = f64_mul(fr, a1);
+        g.w[0] = f64_half<true>(f64_third(f64_mul(f64_mul(a1, a2), a3)));  // x / 6 is x / 3 halved, exactly
+        g.w[1] = f64_half(f64_mul(f64_mul(fr, a2), a3));
+        g.w[2] = f64_half<true>(f64_mul(f1, a3));
+        g.w[3] = f64_half(f64_third(f64_mul(f1, a2)));
+    } else {
+        g.w[0] = a1 * a2 * a3 / -6;
+        g.w[1] = fr * a2 * a3 / 2;
+        g.w[2] = fr * a1 * a3 / -2;
+        g.w[3] = fr * a1 * a2 / 6;
+    }
+    return g;
+}
+
+// TriCuInterp::Interpolate of the cell grid: 64 points in (k, j, i) order, clamped At().  In plain FP64, for weights or
+// values outside the integer form's range.
+__device__ __noinline__ double tricubic_plain(int nx, int ny, int nz, const double *f, CubicPoint x, CubicPoint y,
+                                              CubicPoint z) {
+    double val = 0;
+#pragma unroll 1
+    for (int q = 0; q < 64; q++) {
+        const int i = q & 3, j = (q >> 2) & 3, k = q >> 4;
+        const int cx = min(max(x.lo + i, 0), nx - 1), cy = min(max(y.lo + j, 0), ny - 1);
+        const int cz = min(max(z.lo + k, 0), nz - 1);
+        const double wx = i == 0 ? x.w[0] : (i == 1 ? x.w[1] : (i == 2 ? x.w[2] : x.w[3]));
+        const double wy = j == 0 ? y.w[0] : (j == 1 ? y.w[1] : (j == 2 ? y.w[2] : y.w[3]));
+        const double wz = k == 0 ? z.w[0] : (k == 1 ? z.w[1] : (k == 2 ? z.w[2] : z.w[3]));
+        val += f[cz + nz * (cy + ny * cx)] * (wx * wy * wz);
+    }
+    return val;
+}
+
+// The same.  An axis on which the point sits on a cell (weights exactly 0, 1, 0, 0: no motion along it) keeps its second
+// point alone: the others would add a signed zero to a sum that starts at +0, as long as their values are finite.
+// Otherwise the weights are normal and so is every product, as long as the values are in [2^-100, 2^300); one that is
+// not (a zero among them) leaves the sum to the plain form.
+// The sixteen products of the x and y weights wait in shared memory (`xy`, this thread's column of 256), so that the
+// loops over k and j stay loops: unrolled over j they took 2600 us at 192^3, the warps waiting for instructions.
+__device__ __forceinline__ double tricubic(const Dims &d, const double *__restrict__ f, const CubicPoint g[3],
+                                           double (*xy)[256]) {
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    int cx[4];
+    bool one[3];
+    uint32_t most = 0;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const double co = o[a] + h / 2;  // cell grid origin
-        lo[a] = (int)floor((p[a] - co) * invh - 1.0);
-        const double fr = (p[a] - co - (double)lo[a] * h) * invh;
-        w[0][a] = (fr - 1) * (fr - 2) * (fr - 3) / -6;
-        w[1][a] = fr * (fr - 2) * (fr - 3) / 2;
-        w[2][a] = fr * (fr - 1) * (fr - 3) / -2;
-        w[3][a] = fr * (fr - 1) * (fr - 2) / 6;
-    }
-    double val = 0;
+        one[a] = f64_is_zero(g[a].w[0]) && f64_is_one(g[a].w[1]) && f64_is_zero(g[a].w[2]) && f64_is_zero(g[a].w[3]);
 #pragma unroll
-    for (int k = 0; k < 4; k++)
+        for (int q = 0; q < 4; q++) most = one[a] ? most : max(most, f64_above(g[a].w[q], -300));
+    }
+    bool hard = most >= (330u << 20);
+    double val = 0;
+    if (!hard) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) cx[q] = min(max(g[0].lo + q, 0), d.nx - 1) * (d.ny * d.nz);  // fewer than 2^31 cells
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                int ci[3] = {lo[0] + i, lo[1] + j, lo[2] + k};
+            for (int i = 0; i < 4; i++) xy[4 * j + i][tid] = f64_mul(g[0].w[i], g[1].w[j]);
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) {
+            const double wk = k == 0 ? g[2].w[0] : (k == 1 ? g[2].w[1] : (k == 2 ? g[2].w[2] : g[2].w[3]));
+            const int ck = min(max(g[2].lo + k, 0), d.nz - 1);
+#pragma unroll 1
+            for (int j = 0; j < 4; j++) {
+                const int row = ck + min(max(g[1].lo + j, 0), d.ny - 1) * d.nz;
+                double v[4];
+                uint32_t far = 0, size = 0;
 #pragma unroll
-                for (int a = 0; a < 3; a++) ci[a] = ci[a] < 0 ? 0 : (ci[a] > sz[a] - 1 ? sz[a] - 1 : ci[a]);
-                val += f[cid(d, ci[0], ci[1], ci[2])] * (w[i][0] * w[j][1] * w[k][2]);
+                for (int i = 0; i < 4; i++) {
+                    v[i] = f[row + cx[i]];
+                    far = max(far, f64_above(v[i], -100));
+                    size = max(size, f64_above(v[i], -1023));  // the exponent field itself
+                }
+                if (size < kF64Exp && ((one[2] && k != 1) || (one[1] && j != 1))) continue;  // finite times zero
+                if (far >= (400u << 20)) {
+                    hard = true;
+                    continue;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (one[0] && i != 1) continue;
+                    const double w2 = xy[4 * j + i][tid];
+                    const double wt = one[2] ? w2 : f64_mul<false, false>(w2, wk);
+                    // three products in four on the integer pipe balance the two
+                    val += i < 3 ? f64_mul<false, false>(v[i], wt) : v[i] * wt;
+                }
             }
-    return val;
+        }
+    }
+    return hard ? tricubic_plain(d.nx, d.ny, d.nz, f, g[0], g[1], g[2]) : val;
 }
 
 }  // namespace sf

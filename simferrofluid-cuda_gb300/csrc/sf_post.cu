@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) k_extrap_sweep(Dims d, Faces u, BitRows v
 // Collider::Enforce (core/Collider.cpp:75-86) changes the faces with fraction == 1 alone, one in 130 in a walled box, and
 // on the z walls one of a row's ends, so a pass with a thread a face leaves 31 lanes of a warp idle there (2.3 ms of
 // the 2.7 ms at 256^3).  Three passes instead: list the faces (all three fractions read once), evaluate the list from
-// the velocity as it was, write the values: 74, 129 (bound by the FP64 pipe) and 6 us.
+// the velocity as it was, write the values: 74, 115 (bound by the FP64 and integer pipes) and 6 us.
 struct EnforceLists {
     uint32_t *face[3];    // face indices with fraction == 1
     double *value[3];     // their new velocities
@@ -221,10 +221,9 @@ __global__ void __launch_bounds__(128) k_enforce_eval(Dims d, Origin og, double 
         double vel[3], vel0[3], n[3];
 #pragma unroll
         for (int b = 0; b < 3; b++) {
-            const Trilinear t = trilinear(d, b, q);
-            vel[b] = t.of(old.p[b]);
-            vel0[b] = us.p[0] ? t.of(us.p[b]) : 0.0;
-            n[b] = t.of(normal.p[b]);
+            vel[b] = trilinear_face(d, b, q, old.p[b]);
+            vel0[b] = us.p[0] ? trilinear_face(d, b, q, us.p[b]) : 0.0;
+            n[b] = trilinear_face(d, b, q, normal.p[b]);
         }
         const double nn = f64_sqrt_any((n[0] * n[0] + n[1] * n[1]) + n[2] * n[2]);  // Vector3d::normalized
         if (nn > 0)
@@ -253,9 +252,10 @@ __global__ void k_vertex_pressures(Dims d, Origin og, double h, double invh, Fac
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x) {
         const double p[3] = {pos[3 * v], pos[3 * v + 1], pos[3 * v + 2]};
         const double n[3] = {nrm[3 * v], nrm[3 * v + 1], nrm[3 * v + 2]};
+        const GridPoint q = grid_point(og.o, h, invh, p);
         double hv[3];
 #pragma unroll
-        for (int b = 0; b < 3; b++) hv[b] = trilerp_face(d, H.p[b], b, og.o, h, invh, p);
+        for (int b = 0; b < 3; b++) hv[b] = trilinear_face(d, b, q, H.p[b]);
         double coeff = (hv[0] * hv[0] + hv[1] * hv[1]) + hv[2] * hv[2];
         const double hn = (hv[0] * n[0] + hv[1] * n[1]) + hv[2] * n[2];
         coeff += chi * chi / (4 * chi + 4) * hn * hn;
@@ -289,48 +289,131 @@ __global__ void __launch_bounds__(256) k_pressure_jump(Dims d, int a, EdgeMarks 
 }
 
 // ------------------------------------------------------------------------------------------------ level set
-// Advection::Trace<2> (core/Advection.h:15-18): TVD Runge-Kutta trace of second order from p over dt.
-__device__ __forceinline__ void trace_rk2(const Dims &d, const Faces &u, const double o[3], double h, double invh,
-                                          const double p[3], double dt, double out[3]) {
-    double v0[3], v1[3], q[3];
+// The first point of a trace is the cell's centre or the face's, whose cells and weights depend on its index along each
+// axis alone: a table for the three axes (entry 0 of axis a at OwnTable::first[a]) instead of 36 FP64 operations a
+// trace and 45 for the tricubic weights of a cell that does not move.  Positions: 0 on the faces normal to the axis, 1 on
+// the cells' centres; grids as in GridPoint.
+struct OwnTable {
+    int n, first[3];
+    int *lo;     // [position][grid][n], then cubic [n]
+    double *w;   // [position][grid][lower, upper][n], then cubic [4][n]
+    __device__ __forceinline__ AxisPoint point(int pos, int grid, int e) const {
+        const int k = pos * 2 + grid;
+        AxisPoint p;
+        p.lo = lo[k * n + e];
+        p.w[0] = w[(2 * k) * n + e];
+        p.w[1] = w[(2 * k + 1) * n + e];
+        return p;
+    }
+    __device__ __forceinline__ CubicPoint cubic(int e) const {
+        CubicPoint p;
+        p.lo = lo[4 * n + e];
 #pragma unroll
-    for (int b = 0; b < 3; b++) v0[b] = trilerp_face(d, u.p[b], b, o, h, invh, p);
+        for (int q = 0; q < 4; q++) p.w[q] = w[(8 + q) * n + e];
+        return p;
+    }
+};
+
+__global__ void k_own_table(OwnTable t, Origin og, double h, double invh) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x, pos = blockIdx.y;
+    if (e >= t.n) return;
+    const int a = e >= t.first[2] ? 2 : (e >= t.first[1] ? 1 : 0);
+    const double o = a == 0 ? og.o[0] : (a == 1 ? og.o[1] : og.o[2]);
+    const double p = (pos == 0 ? o : o + h / 2) + (double)(e - t.first[a]) * h;
 #pragma unroll
-    for (int b = 0; b < 3; b++) q[b] = p[b] + v0[b] * dt;
+    for (int grid = 0; grid < 2; grid++) {
+        const AxisPoint q = axis_point(p, grid == 0 ? o : o + h / 2, h, invh);
+        const int k = pos * 2 + grid;
+        t.lo[k * t.n + e] = q.lo;
+        t.w[(2 * k) * t.n + e] = q.w[0];
+        t.w[(2 * k + 1) * t.n + e] = q.w[1];
+    }
+    if (pos == 1) {
+        const CubicPoint c = cubic_point(p, o + h / 2, h, invh);
+        t.lo[4 * t.n + e] = c.lo;
+        for (int q = 0; q < 4; q++) t.w[(8 + q) * t.n + e] = c.w[q];
+    }
+}
+
+// Advection::Trace<2> (core/Advection.h:15-18): TVD Runge-Kutta trace of second order over dt from the face (i, j, k) of
+// axis FACE (-1: the cell).  False when the velocity there is exactly zero (the air beyond the extrapolated layers),
+// where p + 0 dt is p, the second sample is the first again and the departure point is p.
+template <int FACE>
+__device__ __forceinline__ bool trace_rk2(const Dims &d, const Faces &u, const OwnTable &own, const Origin &og,
+                                          double h, double invh, const int c3[3], double dt, double out[3]) {
+    GridPoint g;
 #pragma unroll
-    for (int b = 0; b < 3; b++) v1[b] = trilerp_face(d, u.p[b], b, o, h, invh, q);
+    for (int s = 0; s < 2; s++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) g.on[s][a] = own.point(a == FACE ? 0 : 1, s, own.first[a] + c3[a]);
+    g.check();
+    double v0[3], v1[3], p[3], q[3];
+#pragma unroll
+    for (int b = 0; b < 3; b++) v0[b] = trilinear_face(d, b, g, u.p[b]);
+    if (f64_is_zero(v0[0]) && f64_is_zero(v0[1]) && f64_is_zero(v0[2])) return false;
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        p[b] = (b == FACE ? og.o[b] : og.o[b] + h / 2) + (double)c3[b] * h;
+        q[b] = p[b] + v0[b] * dt;
+    }
+    g = grid_point(og.o, h, invh, q);
+#pragma unroll
+    for (int b = 0; b < 3; b++) v1[b] = trilinear_face(d, b, g, u.p[b]);
 #pragma unroll
     for (int b = 0; b < 3; b++) out[b] = p[b] + (v0[b] + v1[b]) * dt / 2;
+    return true;
 }
 
-// Advection::Solve<2>(levelSet, velocity, dt) (core/Advection.h:40-49): phi at each cell centre's RK2 departure
-// point (trace over -dt), by tricubic interpolation of the old phi.
-__global__ void __launch_bounds__(256) k_advect_levelset(Dims d, Origin og, double h, double invh, Faces u,
-                                                         double dt, const double *__restrict__ phi,
-                                                         double *__restrict__ out) {
+// Advection::Solve<2>(levelSet, velocity, dt) (core/Advection.h:40-49): phi at each cell centre's RK2 departure point
+// (trace over -dt), by tricubic interpolation of the old phi.
+//
+// 620 FP64 operations a cell bound it (8.3 ms at 192^3, a quarter of it liquid); with the weights and three in four of
+// the products on the integer pipe, the first point from a table and zero velocities cut short, the FP64 pipe (70%
+// busy) and the integer pipe (64%) take 2.4-2.5 ms.  64 registers: four blocks an SM against three are worth 7%.
+__global__ void __launch_bounds__(256, 4) k_advect_levelset(Dims d, Origin og, double h, double invh, Faces u,
+                                                            OwnTable own, double dt, const double *__restrict__ phi,
+                                                            double *__restrict__ out) {
+    __shared__ double xy[16][256];
     const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
     if (k >= d.nz || j >= d.ny) return;
-    const double p[3] = {og.o[0] + h / 2 + (double)i * h, og.o[1] + h / 2 + (double)j * h,
-                         og.o[2] + h / 2 + (double)k * h};
+    const int c3[3] = {i, j, k};
     double q[3];
-    trace_rk2(d, u, og.o, h, invh, p, -dt, q);
-    out[cid(d, i, j, k)] = tricubic_cell(d, phi, og.o, h, invh, q);
+    CubicPoint c[3];
+    if (trace_rk2<-1>(d, u, own, og, h, invh, c3, -dt, q)) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) c[a] = cubic_point(q[a], og.o[a] + h / 2, h, invh);
+    } else {
+#pragma unroll
+        for (int a = 0; a < 3; a++) c[a] = own.cubic(own.first[a] + c3[a]);
+    }
+    out[cid(d, i, j, k)] = tricubic(d, phi, c, xy);
 }
 
-// Advection::Solve<2>(velocity, velocity, dt) (core/Advection.h:51-59) for the faces of axis a: trilinear
-// interpolation of the old face grid a at each face's RK2 departure point.
-__global__ void __launch_bounds__(256) k_advect_velocity(Dims d, int a, Origin og, double h, double invh, Faces u,
-                                                         const double *__restrict__ ua, double dt,
-                                                         double *__restrict__ out) {
-    const FDims f = fdims(d, a);
+// Advection::Solve<2>(velocity, velocity, dt) (core/Advection.h:51-59) for the faces of axis A: trilinear
+// interpolation of the old face grid A at each face's RK2 departure point.  Bound as k_advect_levelset is: 9.0 ms at
+// 160^3 for the three axes with every operation on the FP64 pipe, 1.9 ms now (73% of the FP64 pipe).
+template <int A>
+__global__ void __launch_bounds__(256, 4) k_advect_velocity(Dims d, Origin og, double h, double invh, Faces u,
+                                                            OwnTable own, double dt, double *__restrict__ out) {
+    const FDims f = fdims(d, A);
     const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
     if (k >= f.fz || j >= f.fy) return;
     const int c3[3] = {i, j, k};
-    double p[3], q[3];
+    double q[3];
+    GridPoint g;
+    if (trace_rk2<A>(d, u, own, og, h, invh, c3, -dt, q)) {
 #pragma unroll
-    for (int b = 0; b < 3; b++) p[b] = (b == a ? og.o[b] : og.o[b] + h / 2) + (double)c3[b] * h;
-    trace_rk2(d, u, og.o, h, invh, p, -dt, q);
-    out[fidx(f, i, j, k)] = trilerp_face(d, ua, a, og.o, h, invh, q);
+        for (int b = 0; b < 3; b++)
+            g.on[0][b] = g.on[1][b] = axis_point(q[b], b == A ? og.o[b] : og.o[b] + h / 2, h, invh);
+    } else {
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int s = b == A ? 0 : 1;
+            g.on[0][b] = g.on[1][b] = own.point(s, s, own.first[b] + c3[b]);
+        }
+    }
+    g.check();
+    out[fidx(f, i, j, k)] = trilinear_face(d, A, g, u.p[A]);
 }
 
 __device__ __forceinline__ double dmax0(double a, double b) { return (a < b) ? b : a; }  // std::max(a, b)
@@ -389,7 +472,7 @@ __device__ __forceinline__ double weno_fast(const double dev[5], double invdx) {
         big = v > big ? v : big;
     }
     const double top = f64_from_words((uint32_t)(big >> 32), (uint32_t)big);
-    const double eps = f64_mul<true>(f64_sqr<true>(top), 1e-6);
+    const double eps = f64_mul<false, false>(f64_sqr<true>(top), 1e-6);
     const double third1 = f64_third(dev[1]), third2 = f64_third(dev[2]), third3 = f64_third(dev[3]);
     const double phix1 = __fma_rn(.5, f64_times_third<11>(dev[2]),
                                   __fma_rn(-.5, f64_times_third<7>(dev[1]), f64_third(dev[0])));
@@ -407,7 +490,8 @@ __device__ __forceinline__ double weno_fast(const double dev[5], double invdx) {
     const double alpha2 = f64_div(.6, f64_sqr<true>(__fma_rn(.25, s2, eps)));
     const double alpha3 = f64_div(.3, f64_sqr<true>(__fma_rn(.25, s3, eps)));
     const double sum = alpha1 + alpha2 + alpha3;
-    return f64_mul(f64_div(f64_mul(alpha1, phix1) + f64_mul(alpha2, phix2) + f64_mul(alpha3, phix3), sum), invdx);
+    return f64_mul<true, false>(f64_div(f64_mul<false>(alpha1, phix1) + f64_mul<false>(alpha2, phix2) +
+                                           f64_mul<false>(alpha3, phix3), sum), invdx);
 }
 
 // An FP32 value within 2^-23 of v (truncated), v zero or in [2^-100, 2^60).
@@ -590,17 +674,39 @@ inline dim3 reinit_grid(const Dims &d) {
 inline dim3 cell_grid(const Dims &d) { return dim3((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx); }
 }  // namespace
 
+namespace {
+// The table in `work` (advect_table_bytes), filled on the stream.
+OwnTable own_table(cudaStream_t st, const Dims &d, const Origin &og, double h, void *work) {
+    OwnTable t;
+    t.first[0] = 0;
+    t.first[1] = d.nx + 1;
+    t.first[2] = d.nx + d.ny + 2;
+    t.n = d.nx + d.ny + d.nz + 3;
+    t.w = (double *)work;
+    t.lo = (int *)(t.w + 12 * (size_t)t.n);
+    k_own_table<<<dim3((t.n + 127) / 128, 2), 128, 0, st>>>(t, og, h, 1 / h);
+    return t;
+}
+}  // namespace
+
+size_t advect_table_bytes(const Dims &d) {
+    return (12 * sizeof(double) + 5 * sizeof(int)) * ((size_t)d.nx + d.ny + d.nz + 3);
+}
+
 void launch_advect_levelset(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &u,
-                            double dt, const double *phi, double *out) {
+                            double dt, const double *phi, double *out, void *work) {
     Origin og{{origin[0], origin[1], origin[2]}};
-    k_advect_levelset<<<cell_grid(d), blk2(), 0, st>>>(d, og, h, 1 / h, u, dt, phi, out);
+    const OwnTable own = own_table(st, d, og, h, work);
+    k_advect_levelset<<<cell_grid(d), blk2(), 0, st>>>(d, og, h, 1 / h, u, own, dt, phi, out);
 }
 
 void launch_advect_velocity(cudaStream_t st, const Dims &d, const double origin[3], double h, const Faces &u,
-                            double dt, double *const out[3]) {
+                            double dt, double *const out[3], void *work) {
     Origin og{{origin[0], origin[1], origin[2]}};
-    for (int a = 0; a < 3; a++)
-        k_advect_velocity<<<face_grid(d, a), blk2(), 0, st>>>(d, a, og, h, 1 / h, u, u.p[a], dt, out[a]);
+    const OwnTable own = own_table(st, d, og, h, work);
+    k_advect_velocity<0><<<face_grid(d, 0), blk2(), 0, st>>>(d, og, h, 1 / h, u, own, dt, out[0]);
+    k_advect_velocity<1><<<face_grid(d, 1), blk2(), 0, st>>>(d, og, h, 1 / h, u, own, dt, out[1]);
+    k_advect_velocity<2><<<face_grid(d, 2), blk2(), 0, st>>>(d, og, h, 1 / h, u, own, dt, out[2]);
 }
 
 void launch_reinitialize(cudaStream_t st, const Dims &d, double h, double *phi, double *p1, double *p2,

@@ -69,7 +69,12 @@ int main() {
         check("times_third<11>", sf::f64_times_third<11>(a), a * 11 / 3, a, 0);
         check("times_third<13>", sf::f64_times_third<13>(a), a * 13 / 3, a, 0);
         check("sqr", sf::f64_sqr(a), a * a, a, a);
-        if (a != 0 && b != 0) check("mul nonzero", sf::f64_mul<true>(a, b), a * b, a, b);
+        check("half", sf::f64_half(a), a / 2, a, 0);
+        check("-half", sf::f64_half<true>(a), a / -2, a, 0);
+        check("div_any", sf::f64_div_any(a, b != 0 ? b : 1), a / (b != 0 ? b : 1), a, b);
+        check("sqrt_any", sf::f64_sqrt_any(std::fabs(a)), std::sqrt(std::fabs(a)), a, 0);
+        check("third_any", sf::f64_third_any(a), a / 3, a, 0);
+        if (a != 0 && b != 0) check("mul nonzero", sf::f64_mul<false, false>(a, b), a * b, a, b);
         if (a != 0) {
             const double r = std::fabs(a);
             check("sqrt", sf::f64_sqrt(r), std::sqrt(r), r, 0);
@@ -81,6 +86,8 @@ int main() {
         const bool in = a == 0 || (std::fabs(a) >= 0x1p-100 && std::fabs(a) < 0x1p60);
         n++;
         bad += sf::f64_in_range(a, -100, 60) != in;
+        n++;
+        bad += (sf::f64_above(a, -100) < (160u << 20)) != (in && a != 0);
     }
     auto check_floor = [&](double v) {
         double fl;
@@ -109,6 +116,14 @@ int main() {
         check_order(v);
     }
     for (double v : {(double)NAN, -(double)NAN, (double)INFINITY, -(double)INFINITY, 1 + 0x1p-52, -1e308, 1e308}) check_order(v);
+    for (double v : {0x1p-1074, -0x1p-1030, 1e308, -1e308, (double)INFINITY, -0.0, 0x1p-1022, 0x1p1023}) {
+        check("div_any", sf::f64_div_any(v, 3.0), v / 3.0, v, 3);
+        check("div_any", sf::f64_div_any(1.0, v), 1.0 / v, 1, v);
+        check("sqrt_any", sf::f64_sqrt_any(std::fabs(v)), std::sqrt(std::fabs(v)), v, 0);
+        check("third_any", sf::f64_third_any(v), v / 3, v, 0);
+    }
+    n++;
+    bad += !std::isnan(sf::f64_sqrt_any(-1.0)) || !std::isnan(sf::f64_div_any(NAN, 1.0));
     const double outside[] = {0x1p-1074, -0x1p-1030, 0x1p-101, 0x1p60, -0x1p60, 1e300, INFINITY, -INFINITY, NAN};
     for (double v : outside) {
         n++;
