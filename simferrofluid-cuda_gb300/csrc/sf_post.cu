@@ -243,12 +243,14 @@ __global__ void __launch_bounds__(256) k_enforce_put(EnforceLists l, Faces u) {
 }
 
 // MagneticField::CalculateVertexPressures (core/MagneticField.cpp:37-48) for vertex v: H trilinear at its position,
-// p = mu0/2 chi (|H|^2 + chi^2/(4chi+4) (H.n)^2), mu0 = 4e-7 pi (core/MagneticField.cpp:7-8).
-__global__ void k_vertex_pressures(Dims d, Origin og, double h, double invh, Faces H, double chi,
-                                   const double *__restrict__ pos, const double *__restrict__ nrm, long long nv,
-                                   double *__restrict__ out) {
-    const double pi = 3.141592653589793238462643383279502884;
-    const double mu0 = 4e-7 * pi;
+// p = mu0/2 chi (|H|^2 + chi^2/(4chi+4) (H.n)^2), mu0 = 4e-7 pi (core/MagneticField.cpp:7-8).  The two factors that
+// depend on chi alone come from the host (an FP64 division a vertex otherwise): 74 us for 196,608 vertices at the start,
+// 45 us with that and the samples' products on the integer pipe.
+__global__ void __launch_bounds__(128) k_vertex_pressures(Dims d, Origin og, double h, double invh, Faces H,
+                                                          double scale, double normal_part,
+                                                          const double *__restrict__ pos,
+                                                          const double *__restrict__ nrm, long long nv,
+                                                          double *__restrict__ out) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x) {
         const double p[3] = {pos[3 * v], pos[3 * v + 1], pos[3 * v + 2]};
         const double n[3] = {nrm[3 * v], nrm[3 * v + 1], nrm[3 * v + 2]};
@@ -258,8 +260,8 @@ __global__ void k_vertex_pressures(Dims d, Origin og, double h, double invh, Fac
         for (int b = 0; b < 3; b++) hv[b] = trilinear_face(d, b, q, H.p[b]);
         double coeff = (hv[0] * hv[0] + hv[1] * hv[1]) + hv[2] * hv[2];
         const double hn = (hv[0] * n[0] + hv[1] * n[1]) + hv[2] * n[2];
-        coeff += chi * chi / (4 * chi + 4) * hn * hn;
-        out[v] = mu0 * 0.5 * chi * coeff;
+        coeff += normal_part * hn * hn;
+        out[v] = scale * coeff;
     }
 }
 
@@ -267,25 +269,38 @@ struct EdgeMarks {
     const int32_t *p[3];
 };
 
-// The pressure-jump callback of core/Simulation.cpp:216-235 on the faces of axis a: the vertex of edge
+// The pressure-jump callback of core/Simulation.cpp:216-235 on the faces of the three axes (blockIdx.z): the vertex of edge
 // (a, face - e_a) (Contour::VertexIndexOf; edge grid of axis a = cell grid minus e_a, -1 = no vertex) gives
 // J = kappa sigma / rho / h dt - p_m / rho / h dt (terms present when their arrays are), 0 without a vertex.
-__global__ void __launch_bounds__(256) k_pressure_jump(Dims d, int a, EdgeMarks em, const double *__restrict__ kappa,
+// A warp takes a row, four faces a lane at a time: every mark is loaded before the first jump is stored.  Bound by HBM
+// (4 bytes in and 8 out a face): 100 us an axis with one face a thread, 116 us for the three now (256^3).
+__global__ void __launch_bounds__(256) k_pressure_jump(Dims d, EdgeMarks em, const double *__restrict__ kappa,
                                                        const double *__restrict__ pm, double sigma, double rho,
-                                                       double invh, double dt, double *__restrict__ jump) {
+                                                       double invh, double dt, Faces jump) {
+    const int a = blockIdx.z, i = blockIdx.y, j = blockIdx.x * 8 + threadIdx.y;
     const FDims f = fdims(d, a);
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= f.fz || j >= f.fy) return;
+    if (i >= f.fx || j >= f.fy) return;
     const int ex = d.nx - (a == 0), ey = d.ny - (a == 1), ez = d.nz - (a == 2);
-    int e[3] = {i, j, k};
-    e[a] -= 1;
-    int idx = -1;
-    if (e[0] >= 0 && e[1] >= 0 && e[2] >= 0 && e[0] < ex && e[1] < ey && e[2] < ez)
-        idx = em.p[a][(long long)e[2] + (long long)ez * ((long long)e[1] + (long long)ey * e[0])];
-    double pressure = 0;
-    if (kappa && idx >= 0) pressure += kappa[idx] * sigma / rho * invh * dt;
-    if (pm && idx >= 0) pressure -= pm[idx] / rho * invh * dt;
-    jump[fidx(f, i, j, k)] = pressure;
+    const int ei = i - (a == 0), ej = j - (a == 1);
+    const bool row = ei >= 0 && ej >= 0 && ei < ex && ej < ey;
+    const int32_t *marks = em.p[a] + ((long long)ei * ey + ej) * ez - (a == 2);  // mark of face k at marks[k]
+    double *out = const_cast<double *>(jump.p[a]) + fidx(f, i, j, 0);
+    for (int k0 = threadIdx.x; k0 < f.fz; k0 += 128) {
+        int idx[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = k0 + 32 * q, ek = k - (a == 2);
+            idx[q] = row && ek >= 0 && ek < ez ? marks[k] : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = k0 + 32 * q;
+            double pressure = 0;
+            if (kappa && idx[q] >= 0) pressure += f64_div_any(kappa[idx[q]] * sigma, rho) * invh * dt;
+            if (pm && idx[q] >= 0) pressure -= f64_div_any(pm[idx[q]], rho) * invh * dt;
+            if (k < f.fz) out[k] = pressure;
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ level set
@@ -724,16 +739,17 @@ void launch_vertex_pressures(cudaStream_t st, const Dims &d, const double origin
                              double chi, const double *pos, const double *nrm, long long nv, double *out) {
     if (nv <= 0) return;
     Origin og{{origin[0], origin[1], origin[2]}};
-    long long blocks = (nv + 255) / 256;
-    if (blocks > 152 * 16) blocks = 152 * 16;
-    k_vertex_pressures<<<(unsigned)blocks, 256, 0, st>>>(d, og, h, 1 / h, H, chi, pos, nrm, nv, out);
+    const double mu0 = 4e-7 * 3.141592653589793238462643383279502884;
+    const long long blocks = std::min((nv + 127) / 128, 152LL * 32);
+    k_vertex_pressures<<<(unsigned)blocks, 128, 0, st>>>(d, og, h, 1 / h, H, mu0 * 0.5 * chi, chi * chi / (4 * chi + 4),
+                                                         pos, nrm, nv, out);
 }
 
 void launch_pressure_jump(cudaStream_t st, const Dims &d, const int32_t *const edge_mark[3], const double *kappa,
                           const double *pm, double sigma, double rho, double h, double dt, double *const jump[3]) {
     EdgeMarks em{{edge_mark[0], edge_mark[1], edge_mark[2]}};
-    for (int a = 0; a < 3; a++)
-        k_pressure_jump<<<face_grid(d, a), blk2(), 0, st>>>(d, a, em, kappa, pm, sigma, rho, 1 / h, dt, jump[a]);
+    const Faces fj{{jump[0], jump[1], jump[2]}};
+    k_pressure_jump<<<dim3((d.ny + 8) / 8, d.nx + 1, 3), blk2(), 0, st>>>(d, em, kappa, pm, sigma, rho, 1 / h, dt, fj);
 }
 
 size_t extrapolate_bits_bytes(const Dims &d, int a) {
