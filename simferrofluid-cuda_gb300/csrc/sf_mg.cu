@@ -2435,7 +2435,7 @@ cudaError_t MGSolver::solve_mixed(bool x_is_zero, SolveResult &res) {
         }
         total_inner += it;
         if (split0_)
-            k_ir_update_s<<<row_grid((const void *)k_ir_update_s, (long long)d.nx * d.ny * (((d.nz >> 1) + 31) / 32)),
+            k_ir_update_s<<<row_grid((const void *)k_ir_update_s, (long long)d.nx * d.ny * (((d.nz >> 1) + 127) / 128)),
                             dim3(32, 8), 0, st_>>>(d, x_, d32_, list_[0], count_);
         else
             k_ir_update<<<flat_grid(n), 256, 0, st_>>>(n, x_, d32_);

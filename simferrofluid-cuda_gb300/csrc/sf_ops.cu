@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "sf_f64_int.cuh"
 #include "sf_ops.h"
 
 namespace sf {
@@ -160,33 +161,34 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
 // the lower x, y and z faces of cell (i, j, k), in one launch over (nx + 1) x (ny + 1) x (nz + 1) points, so phi and
 // p of the cell are loaded once for its three faces.  p is the solution on cells; liquid = phi <= 0.
 // w = 1 - fraction is 0 exactly when the fraction is 1, and 1 exactly when it is zero, where (p1 - p0) * w is
-// p1 - p0: both are tested on the bits, so air faces and open liquid faces take no FP64 operation beyond the
-// update itself.
-__device__ __forceinline__ void project_face(const Dims &d, int a, long long f, long long c0, long long c1, int fa,
-                                             int na, const double *__restrict__ phi, const Faces &frac,
-                                             const Faces &jump, const double *__restrict__ p, double *__restrict__ u,
-                                             double phi1, bool l1) {
-    if (fa <= 0 || fa >= na) return;  // closed boundary face
-    const double fr = frac.p[a][f];
-    if (__double_as_longlong(fr) == kOneBits) return;  // w == 0
-    const double phi0 = phi[c0];
-    const bool l0 = le0(phi0);
-    if (!l0 && !l1) return;
-    double v = u[f];
-    if (l0 && l1 && is_zero(fr)) {
-        v -= p[c1] - p[c0];  // w == 1
-    } else if (l0 && l1) {
-        v -= (p[c1] - p[c0]) * (1. - fr);
-    } else {
-        const double w = 1. - fr;
-        const double theta = phi0 / (phi0 - phi1);
-        const double pin = l0 ? p[c0] : p[c1];
-        const double pj = jump.p[0] ? jump.p[a][f] : 0.;
-        const double t = l0 ? theta : 1 - theta;
-        const double ic = 1. / (t < .001 ? .001 : t);
-        v -= (l0 ? 1.0 : -1.0) * (pj - pin) * ic * w;
-    }
-    u[f] = v;
+// p1 - p0: both are tested on the bits, so open liquid faces take no FP64 operation beyond the update itself.
+// The level set decides first: a face between two air cells (most of a pool's domain) reads nothing more, and the
+// others load fraction, velocity and pressures together.  360 us at 256^3 (20% liquid) when the fraction of every face
+// was read first, each load waiting for the one before; 188 us now, bound by latency and the FP64 pipe (55%).  Two and
+// four planes a thread took 241 and 212 us.
+struct ProjFace {
+    bool on, l0;
+    long long f;
+    double fr, v, p0, phi0;
+};
+// A face at the surface or partly open: its own function, so that its divisions stay out of the common face's way.
+__device__ __noinline__ double project_other(bool l0, bool l1, double fr, double phi0, double phi1, double p0, double p1,
+                                             double pj, double v) {
+    if (l0 && l1) return v - (p1 - p0) * (1. - fr);
+    const double w = 1. - fr;
+    const double theta = f64_div_any(phi0, phi0 - phi1);
+    const double pin = l0 ? p0 : p1;
+    const double t = l0 ? theta : 1 - theta;
+    const double ic = f64_div_any(1., t < .001 ? .001 : t);
+    return v - (l0 ? 1.0 : -1.0) * (pj - pin) * ic * w;
+}
+__device__ __forceinline__ void project_face(const ProjFace &q, int a, bool l1, double p1, double phi1,
+                                             const Faces &jump, double *__restrict__ u) {
+    if (!q.on || __double_as_longlong(q.fr) == kOneBits) return;  // w == 0
+    if (q.l0 && l1 && is_zero(q.fr))
+        u[q.f] = q.v - (p1 - q.p0);  // w == 1
+    else
+        u[q.f] = project_other(q.l0, l1, q.fr, q.phi0, phi1, q.p0, p1, jump.p[0] ? jump.p[a][q.f] : 0., q.v);
 }
 
 __global__ void __launch_bounds__(256) k_apply_projection3(Dims d, const double *__restrict__ phi, Faces frac,
@@ -194,21 +196,32 @@ __global__ void __launch_bounds__(256) k_apply_projection3(Dims d, const double 
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
-    if (k > d.nz || j > d.ny || i > d.nx) return;
-    const bool cell = i < d.nx && j < d.ny && k < d.nz;
-    const long long c1 = cell ? cid(d, i, j, k) : 0;
-    const double phi1 = cell ? phi[c1] : 1.0;  // a face whose upper cell is outside the grid is a boundary face
-    const bool l1 = cell && le0(phi1);
-    const long long sx = (long long)d.ny * d.nz, sy = d.nz;
-    if (j < d.ny && k < d.nz)
-        project_face(d, 0, fid(d, 0, i, j, k), c1 - sx, c1, i, d.nx, phi, frac, jump, p, const_cast<double *>(u.p[0]),
-                     phi1, l1);
-    if (i < d.nx && k < d.nz)
-        project_face(d, 1, fid(d, 1, i, j, k), c1 - sy, c1, j, d.ny, phi, frac, jump, p, const_cast<double *>(u.p[1]),
-                     phi1, l1);
-    if (i < d.nx && j < d.ny)
-        project_face(d, 2, fid(d, 2, i, j, k), c1 - 1, c1, k, d.nz, phi, frac, jump, p, const_cast<double *>(u.p[2]),
-                     phi1, l1);
+    // the lower faces of a cell past the grid's upper end are boundary faces: closed
+    if (k >= d.nz || j >= d.ny) return;
+    const long long c1 = cid(d, i, j, k);
+    const long long st[3] = {(long long)d.ny * d.nz, d.nz, 1};
+    const bool inside[3] = {i > 0, j > 0, k > 0};
+    const double phi1 = phi[c1];
+    ProjFace q[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) q[a].phi0 = inside[a] ? phi[c1 - st[a]] : 1.;
+    const bool l1 = le0(phi1);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        q[a].l0 = le0(q[a].phi0);
+        q[a].on = inside[a] && (q[a].l0 || l1);
+        q[a].f = fid(d, a, i, j, k);
+    }
+    if (!q[0].on && !q[1].on && !q[2].on) return;
+    const double p1 = p[c1];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        q[a].fr = q[a].on ? frac.p[a][q[a].f] : 1.;
+        q[a].v = q[a].on ? u.p[a][q[a].f] : 0.;
+        q[a].p0 = q[a].on ? p[c1 - st[a]] : 0.;
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) project_face(q[a], a, l1, p1, phi1, jump, const_cast<double *>(u.p[a]));
 }
 
 // p_out on cells: solution in liquid cells (D > 0 in the stored operator), 0 elsewhere.
@@ -360,6 +373,18 @@ __global__ void __launch_bounds__(256) k_magnetic_rows(Dims d, Faces hext, doubl
 // the grid, H = Hext on the grid's boundary faces.  One thread per node (i, j, k) of the cell grid writes the lower
 // x, y and z faces of cell (i, j, k), in one launch over (nx + 1) x (ny + 1) x (nz + 1) points, so psi of the cell
 // is loaded once for its three faces.
+// The FP64 pipe bounds it: three operations a face took 307 us at 256^3, where the bytes take 139.  Two remain: the
+// product with 1 / h runs on the integer pipe, or, where 1 / h is a power of two (POW2) and the product exact, joins the
+// sum as a fused multiply-add, which then rounds once as the sum does: 198 us.
+__device__ __noinline__ double mul_plain(double a, double b) { return a * b; }
+template <bool POW2>
+__device__ __forceinline__ double field_face(double p0, double p1, double invh, double h) {
+    const double diff = p0 - p1;
+    if (POW2 && f64_in_range(diff, -500, 500)) return __fma_rn(diff, invh, h);
+    return (f64_in_range(diff, -500, 500) ? f64_mul<true, false>(diff, invh) : mul_plain(diff, invh)) + h;
+}
+
+template <bool POW2>
 __global__ void __launch_bounds__(256) k_total_field3(Dims d, const double *__restrict__ psi, Faces hext, double invh,
                                                       Faces H) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -369,27 +394,23 @@ __global__ void __launch_bounds__(256) k_total_field3(Dims d, const double *__re
     const bool cell = i < d.nx && j < d.ny && k < d.nz;
     const long long c1 = cell ? cid(d, i, j, k) : 0;
     const double p1 = cell ? psi[c1] : 0.0;
-    const long long sx = (long long)d.ny * d.nz, sy = d.nz;
-    if (j < d.ny && k < d.nz) {
-        const long long f = fid(d, 0, i, j, k);
-        double v = 0.;
-        if (i > 0 && i < d.nx) v = (psi[c1 - sx] - p1) * invh;
-        v += hext.p[0][f];
-        const_cast<double *>(H.p[0])[f] = v;
+    const long long st[3] = {(long long)d.ny * d.nz, d.nz, 1};
+    const int at[3] = {i, j, k}, n[3] = {d.nx, d.ny, d.nz};
+    double p0[3], h[3];
+    bool on[3], in[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        on[a] = (a == 0 || i < d.nx) && (a == 1 || j < d.ny) && (a == 2 || k < d.nz);
+        in[a] = on[a] && at[a] > 0 && at[a] < n[a];
+        p0[a] = in[a] ? psi[c1 - st[a]] : 0.;
+        h[a] = on[a] ? hext.p[a][fid(d, a, i, j, k)] : 0.;
     }
-    if (i < d.nx && k < d.nz) {
-        const long long f = fid(d, 1, i, j, k);
-        double v = 0.;
-        if (j > 0 && j < d.ny) v = (psi[c1 - sy] - p1) * invh;
-        v += hext.p[1][f];
-        const_cast<double *>(H.p[1])[f] = v;
-    }
-    if (i < d.nx && j < d.ny) {
-        const long long f = fid(d, 2, i, j, k);
-        double v = 0.;
-        if (k > 0 && k < d.nz) v = (psi[c1 - 1] - p1) * invh;
-        v += hext.p[2][f];
-        const_cast<double *>(H.p[2])[f] = v;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        if (!on[a]) continue;
+        // 0 + Hext on the boundary: Hext, with -0 as +0
+        const double v = in[a] ? field_face<POW2>(p0[a], p1, invh, h[a]) : (is_zero(h[a]) ? 0. : h[a]);
+        const_cast<double *>(H.p[a])[fid(d, a, i, j, k)] = v;
     }
 }
 
@@ -484,7 +505,7 @@ void launch_build_pressure(cudaStream_t st, const Dims &d, const double *phi, co
 
 void launch_apply_projection(cudaStream_t st, const Dims &d, const double *phi, const Faces &frac, const Faces &jump,
                              const double *p, const Faces &u) {
-    k_apply_projection3<<<grid3(d.nx + 1, d.ny + 1, d.nz + 1), blk2(), 0, st>>>(d, phi, frac, jump, p, u);
+    k_apply_projection3<<<grid3(d.nx, d.ny, d.nz), blk2(), 0, st>>>(d, phi, frac, jump, p, u);
 }
 
 void launch_gather_cells(cudaStream_t st, long long n, const double *D, const double *x, double *out) {
@@ -568,7 +589,12 @@ cudaError_t launch_magnetic_residual_noalloc(cudaStream_t st, const Dims &d, con
 
 void launch_total_field(cudaStream_t st, const Dims &d, const double *psi, const Faces &hext, double invh,
                         const Faces &H) {
-    k_total_field3<<<grid3(d.nx + 1, d.ny + 1, d.nz + 1), blk2(), 0, st>>>(d, psi, hext, invh, H);
+    int e = 0;
+    const bool pow2 = std::frexp(invh, &e) == 0.5 && e > -400 && e < 400;
+    if (pow2)
+        k_total_field3<true><<<grid3(d.nx + 1, d.ny + 1, d.nz + 1), blk2(), 0, st>>>(d, psi, hext, invh, H);
+    else
+        k_total_field3<false><<<grid3(d.nx + 1, d.ny + 1, d.nz + 1), blk2(), 0, st>>>(d, psi, hext, invh, H);
 }
 
 __global__ void k_to_f32(long long n, const double *__restrict__ a, float *__restrict__ o) {

@@ -296,17 +296,29 @@ __global__ void __launch_bounds__(256) k_split_to_vec(Dims d, const float *__res
 }
 
 // First refinement step from x = 0 on the split level: r = (float) b in the split layout; slots rr = bb = (b, b).
+// Cells 2m and 2m + 1 of a row are one 16-byte load (rows are whole vectors) and go to m of the two colours.
 __global__ void __launch_bounds__(256) k_cast_rhs_s(Dims d, const double *__restrict__ b, float *__restrict__ r,
                                                     int rr_slot, int bb_slot, double *sc, double *part,
                                                     unsigned *ticket) {
     double v[1] = {0};
-    SPLIT_ROWS(d)
-    const double b0 = b[n0], b1 = b[n1];
-    r[s0] = f64_to_f32(b0);
-    r[s1] = f64_to_f32(b1);
-    v[0] += b0 * b0;
-    v[0] += b1 * b1;
-    SPLIT_ROWS_END
+    const int nh = d.nz >> 1;
+    const long long hn = d.n >> 1, nrows = (long long)d.nx * d.ny;
+    for (long long row = blockIdx.x * (long long)blockDim.y + threadIdx.y; row < nrows;
+         row += (long long)gridDim.x * blockDim.y) {
+        const int i = (int)row / d.ny, j = (int)row - i * d.ny;
+        const bool p = (i + j) & 1;
+        const double2 *src = reinterpret_cast<const double2 *>(b + row * d.nz);
+        float *o = r + row * nh;
+#pragma unroll 4
+        for (int m = threadIdx.x; m < nh; m += 32) {
+            const double2 t = src[m];
+            const float lo = f64_to_f32(t.x), hi = f64_to_f32(t.y);
+            o[m] = p ? hi : lo;
+            o[hn + m] = p ? lo : hi;
+            v[0] += t.x * t.x;
+            v[0] += t.y * t.y;
+        }
+    }
     double tot[1];
     if (grid_reduce<1>(v, part, ticket, tot)) {
         sc[rr_slot] = tot[0];
@@ -314,19 +326,37 @@ __global__ void __launch_bounds__(256) k_cast_rhs_s(Dims d, const double *__rest
     }
 }
 
-// x64 += d32 with d32 in the split layout (zero in inactive rows, which are skipped).
+// x64 += d32 with d32 in the split layout (zero in inactive rows, which are skipped).  A lane takes cells 2m and
+// 2m + 1 as one 16-byte vector.
 __global__ void __launch_bounds__(256) k_ir_update_s(Dims d, double *__restrict__ x, const float *__restrict__ dlt,
                                                      const int *__restrict__ list, const int *__restrict__ count) {
     const int nh = d.nz >> 1;
     const long long hn = d.n >> 1;
-    for_list_items(list, count, 1, (nh + 31) / 32, [&](int, int i, int j, int ch, bool) {
-        const int m = ch * 32 + threadIdx.x;
-        if (m >= nh) return;
+    for_list_items(list, count, 1, (nh + 127) / 128, [&](int, int i, int j, int ch, bool) {
         const long long row = (long long)i * d.ny + j;
-        const int p = (i + j) & 1;
-        const long long nat = row * d.nz + 2 * m, sp = row * nh + m;
-        x[nat + p] += (double)dlt[sp];
-        x[nat + 1 - p] += (double)dlt[hn + sp];
+        const bool p = (i + j) & 1;
+        double2 *xr = reinterpret_cast<double2 *>(x + row * d.nz);
+        const float *dr = dlt + row * nh;
+        double2 t[4];
+        float d0[4], d1[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {  // every load before the first store
+            const int m = ch * 128 + q * 32 + threadIdx.x;
+            if (m < nh) {
+                t[q] = xr[m];
+                d0[q] = dr[m];
+                d1[q] = dr[hn + m];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int m = ch * 128 + q * 32 + threadIdx.x;
+            if (m >= nh) continue;
+            // the conversions on the integer pipe: each would cost as much FP64 time as its sum
+            t[q].x += f32_to_f64(p ? d1[q] : d0[q]);
+            t[q].y += f32_to_f64(p ? d0[q] : d1[q]);
+            xr[m] = t[q];
+        }
     });
 }
 
