@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
     }
     double lower[3] = {0, 0, 0};
     double diag = 0, dexv = 0, div = 0;
+    bool one = liquid;  // every in-grid face fully open to a liquid cell
     if (liquid) {
         const int dn[3] = {d.nx, d.ny, d.nz};
 #pragma unroll
@@ -120,10 +121,12 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
             const bool valid = n3[a] >= 0 && n3[a] < dn[a];
             const long long f = fid(d, a, f3[0], f3[1], f3[2]);
             const double w = valid ? 1. - frac.p[a][f] : 0.0;
+            if (valid && __double_as_longlong(w) != kOneBits) one = false;
             if (w > 0) {
                 if (!rhs_only) {
                     const long long nb = cid(d, n3[0], n3[1], n3[2]);
                     const double pn = phi[nb];
+                    if (!le0(pn)) one = false;
                     if (le0(pn)) {
                         diag += w;
                         if (!up) lower[a] = w;
@@ -154,7 +157,10 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
     cf.dex[c] = dexv;
     cf.D[c] = D;
     if (want_invd) cf.invd[c] = liquid ? (D > 0 ? 1. / D : 0.0) : 0.0;
-    if (so.rows) split_store(so, d, i, j, k, lower[0], lower[1], lower[2], dexv, D > 0);
+    if (so.rows) {
+        split_store(so, d, i, j, k, lower[0], lower[1], lower[2], dexv, D > 0);
+        if (!one) so.other[0][(long long)i * d.ny + j] = 1;  // every writer stores 1
+    }
 }
 
 // Pressure::ApplyProjection (core/Pressure.cpp:137-166).  One thread per node (i, j, k) of the cell grid updates
@@ -299,73 +305,90 @@ __global__ void __launch_bounds__(256) k_magnetic_mu(Dims d, const double *__res
 // mu == 1 add a signed zero, which leaves the sum unchanged, and are skipped).  Row 0 keeps its unpinned value:
 // the reference's pinned row 0 is recovered by the psi[0] = 0 gauge after the solve.
 //
-// Fast paths with the same bits, for interior cells whose six face values are one bit pattern: all 1 (air
-// away from the interface) gives D = 6 (six ones summed exactly) and rhs = 0; all 1 + chi (liquid away from
-// it) gives D = sv6, the six-term sum of 1 + chi formed on the host in the same order, and per face
-// (mu - 1) = m1, also formed on the host; the sign -side is an exact negation.  Bit patterns are compared as
-// integers, so air cells take no FP64 operation.
+// Fast paths with the same bits, for cells whose in-grid face values are one bit pattern: all 1 (air away from the
+// interface) gives D = their number (ones summed exactly) and rhs = 0; all 1 + chi (liquid away from it) gives the sum
+// of that many 1 + chi, formed on the host in the same order (sv[n]), and per face (mu - 1) = m1, also formed on the
+// host; the sign -side is an exact negation.  Bit patterns are compared as integers, so air cells take no FP64
+// operation.  Cells at the grid's ends are in the fast paths too: on the general one they held up their whole warp, whose
+// FP64 instructions are issued for one lane as for 32.
+struct RowSums {
+    double sv[7], inv[7];  // n equal face values 1 + chi summed from 0, and the reciprocals
+};
+// One face's term of the right-hand side on the general path, out of the fast paths' way.
+__device__ __noinline__ double rhs_term(double mu, double hext, double side, double h) {
+    return (mu - 1.) * hext * (-side) * h;
+}
 __global__ void __launch_bounds__(256) k_magnetic_rows(Dims d, Faces hext, double h, Coef<double> cf,
                                                        double *__restrict__ b, int want_invd,
-                                                       long long liq_bits, double m1, double sv6,
-                                                       double inv_sv6, uint8_t *__restrict__ rows) {
+                                                       long long liq_bits, double m1, RowSums rs, SplitOut so) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
     if (k >= d.nz || j >= d.ny) return;
     const long long c = cid(d, i, j, k);
     const long long sx = (long long)d.ny * d.nz, sy = d.nz;
-    if (rows) rows[(long long)i * d.ny + j] = 1;  // D > 0: every in-grid mu is at least 1
-    if (i > 0 && i < d.nx - 1 && j > 0 && j < d.ny - 1 && k > 0 && k < d.nz - 1) {
-        const long long m[6] = {__double_as_longlong(cf.ax[c]), __double_as_longlong(cf.ax[c + sx]),
-                                __double_as_longlong(cf.ay[c]), __double_as_longlong(cf.ay[c + sy]),
-                                __double_as_longlong(cf.az[c]), __double_as_longlong(cf.az[c + 1])};
-        const bool air = (m[0] == kOneBits) & (m[1] == kOneBits) & (m[2] == kOneBits) & (m[3] == kOneBits) &
-                         (m[4] == kOneBits) & (m[5] == kOneBits);
-        const bool liq = (m[0] == liq_bits) & (m[1] == liq_bits) & (m[2] == liq_bits) & (m[3] == liq_bits) &
-                         (m[4] == liq_bits) & (m[5] == liq_bits);
-        if (air) {
-            cf.dex[c] = 0.;
-            cf.D[c] = 6.;
-            if (want_invd) cf.invd[c] = 1. / 6.;
-            b[c] = 0.;
-            return;
-        }
-        if (liq) {
-            double rhs = 0.;
-            rhs += (m1 * hext.p[0][fid(d, 0, i, j, k)]) * h;       // ord -x: -side = +1
-            rhs += -(m1 * hext.p[0][fid(d, 0, i + 1, j, k)]) * h;  // ord +x: -side = -1
-            rhs += (m1 * hext.p[1][fid(d, 1, i, j, k)]) * h;
-            rhs += -(m1 * hext.p[1][fid(d, 1, i, j + 1, k)]) * h;
-            rhs += (m1 * hext.p[2][fid(d, 2, i, j, k)]) * h;
-            rhs += -(m1 * hext.p[2][fid(d, 2, i, j, k + 1)]) * h;
-            cf.dex[c] = 0.;
-            cf.D[c] = sv6;
-            if (want_invd) cf.invd[c] = inv_sv6;
-            b[c] = rhs;
-            return;
-        }
-    }
-    double diag = 0., rhs = 0.;
-    // (mu, valid, face index) in ord order -x, +x, -y, +y, -z, +z
+    const long long row = (long long)i * d.ny + j;
+    if (so.rows) so.rows[row] = 1;  // D > 0: every in-grid mu is at least 1
+    // face order -x, +x, -y, +y, -z, +z
+    const bool in[6] = {i > 0, i < d.nx - 1, j > 0, j < d.ny - 1, k > 0, k < d.nz - 1};
+    double mu[6];
+    bool air = true, liq = true;
+    int n = 0;
 #pragma unroll
-    for (int ord = 0; ord < 6; ord++) {
-        const int a = ord >> 1, up = ord & 1;
-        const int ia = a == 0 ? i : (a == 1 ? j : k);
-        const int na = a == 0 ? d.nx : (a == 1 ? d.ny : d.nz);
-        if (up ? (ia >= na - 1) : (ia <= 0)) continue;
-        const long long st = a == 0 ? sx : (a == 1 ? sy : 1);
-        const double *arr = a == 0 ? cf.ax : (a == 1 ? cf.ay : cf.az);
-        const double mu = up ? arr[c + st] : arr[c];
-        diag += mu;
-        if (__double_as_longlong(mu) != kOneBits) {
-            const int fi = i + (a == 0) * up, fj = j + (a == 1) * up, fk = k + (a == 2) * up;
-            const double side = up ? 1.0 : -1.0;
-            rhs += (mu - 1.) * hext.p[a][fid(d, a, fi, fj, fk)] * (-side) * h;
+    for (int o = 0; o < 6; o++) {
+        const long long st = o < 2 ? sx : (o < 4 ? sy : 1);
+        const double *arr = o < 2 ? cf.ax : (o < 4 ? cf.ay : cf.az);
+        mu[o] = in[o] ? ((o & 1) ? arr[c + st] : arr[c]) : 0.;
+        air = air && (!in[o] || __double_as_longlong(mu[o]) == kOneBits);
+        liq = liq && (!in[o] || __double_as_longlong(mu[o]) == liq_bits);
+        n += in[o] ? 1 : 0;
+    }
+    if (so.rows) {
+        // a warp is part of one row; every writer stores 1
+        const unsigned here = __activemask();
+        const bool some_air = __any_sync(here, !air), some_liq = __any_sync(here, !liq);
+        if ((threadIdx.x & 31) == 0 && some_air) so.other[0][row] = 1;
+        if ((threadIdx.x & 31) == 0 && some_liq) so.other[1][row] = 1;
+    }
+    double diag, inv, rhs = 0.;
+    if (air) {
+        diag = inv = 0.;
+#pragma unroll
+        for (int q = 1; q <= 6; q++)
+            if (n == q) {
+                diag = (double)q;
+                inv = 1. / q;
+            }
+    } else if (liq) {
+        diag = inv = 0.;
+#pragma unroll
+        for (int q = 1; q <= 6; q++)
+            if (n == q) {
+                diag = rs.sv[q];
+                inv = rs.inv[q];
+            }
+        if (in[0]) rhs += (m1 * hext.p[0][fid(d, 0, i, j, k)]) * h;       // ord -x: -side = +1
+        if (in[1]) rhs += -(m1 * hext.p[0][fid(d, 0, i + 1, j, k)]) * h;  // ord +x: -side = -1
+        if (in[2]) rhs += (m1 * hext.p[1][fid(d, 1, i, j, k)]) * h;
+        if (in[3]) rhs += -(m1 * hext.p[1][fid(d, 1, i, j + 1, k)]) * h;
+        if (in[4]) rhs += (m1 * hext.p[2][fid(d, 2, i, j, k)]) * h;
+        if (in[5]) rhs += -(m1 * hext.p[2][fid(d, 2, i, j, k + 1)]) * h;
+    } else {
+        diag = 0.;
+#pragma unroll
+        for (int o = 0; o < 6; o++) {
+            if (!in[o]) continue;
+            const int a = o >> 1, up = o & 1;
+            diag += mu[o];
+            if (__double_as_longlong(mu[o]) != kOneBits)
+                rhs += rhs_term(mu[o], hext.p[a][fid(d, a, i + (a == 0) * up, j + (a == 1) * up, k + (a == 2) * up)],
+                                up ? 1.0 : -1.0, h);
         }
+        inv = want_invd ? (diag > 0 ? f64_div_any(1., diag) : 0.) : 0.;
     }
     cf.dex[c] = 0.;
     cf.D[c] = diag;
-    if (want_invd) cf.invd[c] = diag > 0 ? 1. / diag : 0.;
+    if (want_invd) cf.invd[c] = inv;
     b[c] = rhs;
 }
 
@@ -498,6 +521,8 @@ void launch_build_pressure(cudaStream_t st, const Dims &d, const double *phi, co
     if (so && !rhs_only) {
         o = *so;
         cudaMemsetAsync(o.rows, 0, (size_t)d.nx * d.ny, st);
+        cudaMemsetAsync(o.other[0], 0, (size_t)d.nx * d.ny, st);
+        cudaMemsetAsync(o.other[1], 1, (size_t)d.nx * d.ny, st);  // the projection has no second kind
     }
     k_build_pressure<<<grid3(d.nx, d.ny, d.nz), blk2(), 0, st>>>(d, phi, frac, u, us, jump, vol_error, cf, b,
                                                                   rhs_only ? 1 : 0, want_invd ? 1 : 0, o);
@@ -525,19 +550,25 @@ int launch_build_magnetic(cudaStream_t st, const Dims &d, const double *phi, dou
     const double one_plus_chi = 1. + (1. - 0.) * chi;  // the reference's expression with H = 0
     // the rows kernel's constants for cells whose six faces are 1 + chi: the diagonal summed in face order
     // from 0, its reciprocal, and mu - 1
-    double sv6 = 0.;
-    for (int q = 0; q < 6; q++) sv6 += one_plus_chi;
+    RowSums rs{};
+    for (int q = 1; q <= 6; q++) {
+        rs.sv[q] = rs.sv[q - 1] + one_plus_chi;
+        rs.inv[q] = rs.sv[q] > 0 ? 1. / rs.sv[q] : 0.;
+    }
     const double m1 = one_plus_chi - 1.;
     long long liq_bits;
     std::memcpy(&liq_bits, &one_plus_chi, 8);
     SplitOut o{};
-    if (so) o = *so;
+    if (so) {
+        o = *so;
+        for (uint8_t *p : o.other) cudaMemsetAsync(p, 0, (size_t)d.nx * d.ny, st);
+    }
     // two passes: mu of each face is formed once (band faces take FP64 sinpi, which a fused pass forming the
     // upper faces again would evaluate twice) and the row pass reads it back
     k_magnetic_mu<<<grid3(d.nx, d.ny, d.nz), blk2(), 0, st>>>(d, phi, chi, bw, 1.0 / bw, key(t), key(-t),
                                                               one_plus_chi, cf, o);
     k_magnetic_rows<<<grid3(d.nx, d.ny, d.nz), blk2(), 0, st>>>(d, hext, h, cf, b, want_invd ? 1 : 0, liq_bits, m1,
-                                                                 sv6, sv6 > 0 ? 1. / sv6 : 0., o.rows);
+                                                                 rs, o);
     return 2;
 }
 

@@ -184,6 +184,13 @@ class MGSolver {
     bool split1_ = false;                // level 1 stored colour by colour too
     SplitOut so_{};                      // split_targets()
     bool copies_written_ = false;        // the assembly wrote the split copies and flags
+    uint8_t *other_[2] = {nullptr, nullptr};  // level 0: rows that are not of one exact coupling (SplitOut::other)
+    bool other_ok_ = false;              // they belong to the operator in place
+    unsigned *xmax_ = nullptr;           // upper word of the largest |x|
+    bool xmax_ok_ = false;               // it belongs to the x in place
+    // the FP64 residual of the split form, by rows of one coupling where it can (k_residual_rows)
+    template <class TR>
+    void residual_split(TR *r, bool skip0, int rr_slot, int bb_slot);
     int tail_lt_ = -1, tail_smem_ = 0;   // first level of the fused tail (-1: none), its shared memory
     int tail_nc_ = 0;                    // its cluster size
     std::vector<float *> tail_op_;       // per level of at most 65,536 cells: the tail's FP32 operator (k_tail_op)
