@@ -48,9 +48,9 @@ __device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t addr) {
     return d;
 }
 
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t instr_desc_bf16(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major, M = m (128 or 64), N = n.
+__host__ __device__ constexpr uint32_t instr_desc_bf16(int n, int m = 128) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -271,68 +271,80 @@ __global__ void __launch_bounds__(128, 1) k_conv_tc(const __grid_constant__ CUte
 
 // ------------------------------------------------------------------------------------------------ z lines
 // Forward (and input gradient) for Cin = 16 or 32, Cout <= 32, on grids with nz >= 128: a persistent CTA per SM
-// takes bricks of 128 (z) x 4 (y) x LX (x) voxels (LX = 2 for 16 input channels, 1 for 32), 4 LX M tiles of one
-// z line of 128 voxels each.  A pipeline stage is one z shift dz and one group of 16 channels (K = 16): one TMA box,
-// (16 channels, 128 z, 6 y, LX + 2 x) from (z0 + dz, y0 - 1, x0 - 1), lands as 32-byte rows in the 32-byte swizzled
-// K-major layout and carries the tile rows of all nine (dx, dy) taps: tile (yy, xx) of tap (dx, dy) starts
-// 4 KB x ((yy + 1 + dy) + 6 (xx + 1 + dx)) into the box, so each box is read once for nine taps (the 27-box kernel
-// above reads nine times as many rows, of 16 bytes, each half of a 32-byte sector).  The 27 taps' weights stay in
-// shared memory, swizzled the same way, for the CTA's whole run.  Warp 1 lane 0 issues the TMA loads through two stages, warp 0 lane 0
-// the MMAs (M = 128, N = Cout, K = 16) into one of two TMEM accumulator sets, and warps 2-5 read the other set back
-// (bias + ReLU + BF16, or FP32), so the epilogue of a brick overlaps the MMAs of the next.  Every wait is bounded; a
+// takes bricks of 128 (z) x Y (y) x 2 (x) voxels (Y = 4, or 8 for 16 output channels where that costs less), 2 Y M tiles
+// of one z line of 128 voxels each.  A pipeline stage is one z shift dz, one group of 16 channels (K = 16) and one of
+// the four x planes the brick's taps reach: one TMA box, (16 channels, 128 z, Y + 2 y) from (z0 + dz, y0 - 1) of plane
+// x0 - 1 + xb, lands as 32-byte rows in the 32-byte swizzled K-major layout and carries the tile rows of all its (dx, dy)
+// taps: tile (yy, xx = xb - 1 - dx) of tap (dx, dy) starts 4 KB x (yy + 1 + dy) into the box, so each box is read once
+// for up to six taps (the 27-box kernel above reads a box a tap, of 16-byte rows, each half of a 32-byte sector).  The 27
+// taps' weights stay in shared memory, swizzled the same way and ordered (dz, dx, dy), for the CTA's whole run.
+// One line of the box meets up to three tiles along y, through the taps dy = -1, 0, 1; their weights are consecutive rows
+// and the accumulators stand by descending y, so one MMA of N = 3 Cout does the three: an M = 128 operand costs 4 KB of
+// shared memory reads whatever N is (64 clocks as measured), and those reads bound a tap at a time.  The order of an
+// accumulator's sums, (dz, channels, dx, dy), is the same.  16 to 16 channels at 256^3: 795 us a tap at a time, 626 with
+// three taps an MMA (boxes of four planes, two stages: copies and MMAs half overlapped), 519 with a plane a stage and Y = 8,
+// which reads 2.5 lines a voxel and z shift instead of 3.  What bounds it now is shared memory: a brick's 194 MMAs read
+// 16 k clocks' worth at 64 bytes a clock, the copies write 3.8 k at 128, 19.9 k measured.
+// Warp 1 lane 0 issues the TMA loads through the stages, warp 0 lane 0 the MMAs (M = 128, N up to 3 Cout, K = 16) into
+// one of two TMEM accumulator sets, and warps 2-5 read the other set back (bias + ReLU + BF16, or FP32), so the epilogue
+// of a brick overlaps the MMAs of the next.  Every wait is bounded; a
 // timeout stops all roles, drains the copies in flight and sets the error flag.
 constexpr int kLineZ = 128, kLineY = 4;
 
-template <int CI>
-__host__ __device__ constexpr int line_x() {
-    return CI == 16 ? 2 : 1;
-}
+constexpr int kLineX = 2;
 
-template <int CI, int CO>
+template <int CI, int CO, int Y>
 struct LineLayout {
-    static constexpr int LX = line_x<CI>(), kTiles = kLineY * LX, KP = CI / 16;  // 16-channel groups
-    static constexpr uint32_t kBoxRows = kLineZ * (kLineY + 2) * (LX + 2);
-    static constexpr uint32_t kStageBytes = kBoxRows * 32u;  // 96 KB (LX 2) or 72 KB (LX 1)
+    static constexpr int kTiles = Y * kLineX, KP = CI / 16;  // 16-channel groups
+    static constexpr uint32_t kStageBytes = kLineZ * (Y + 2) * 32u;  // one x plane of one z shift and channel group
     static constexpr uint32_t kWChunkRaw = 27u * CO * 32u;  // [tap][co] rows of 16 channels
     static constexpr uint32_t kWChunk = (kWChunkRaw + 1023u) & ~1023u;
+    static constexpr uint32_t kRest = 1024u + KP * kWChunk + 256u;
+    static constexpr int kStagesRaw = (int)((227u * 1024u - kRest) / kStageBytes);
+    static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
     static constexpr uint32_t kCols = kTiles * CO;  // one accumulator set
     static constexpr uint32_t kAlloc = 2u * kCols <= 256u ? 256u : 512u;
-    static constexpr uint32_t kSmemBytes = 1024u + 2u * kStageBytes + KP * kWChunk + 256u;
-    static_assert(CI % 16 == 0 && 2u * kCols <= 512u && kSmemBytes <= 227u * 1024u, "line layout");
+    static constexpr uint32_t kNeed = kRest + kStages * kStageBytes;
+    // at least 116 KB: one CTA per SM, whose TMEM columns are then always free
+    static constexpr uint32_t kSmemBytes = kNeed > 116u * 1024u ? kNeed : 116u * 1024u;
+    static_assert(CI % 16 == 0 && 2u * kCols <= 512u && kStages >= 3 && kSmemBytes <= 227u * 1024u, "line layout");
 };
 
-template <int CI, int CO, int EPI>
+template <int CI, int CO, int EPI, int Y>
 __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__ CUtensorMap tmap_x,
                                                          const __grid_constant__ CUtensorMap tmap_w, Dims d,
                                                          const float *__restrict__ bias, void *__restrict__ yout,
                                                          int *err) {
-    using L = LineLayout<CI, CO>;
-    constexpr int LX = L::LX, kTiles = L::kTiles, KP = L::KP;
+    using L = LineLayout<CI, CO, Y>;
+    constexpr int LX = kLineX, kTiles = L::kTiles, KP = L::KP, S = L::kStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t *wbuf = smem + 2 * L::kStageBytes;
+    uint8_t *wbuf = smem + S * L::kStageBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(wbuf + KP * L::kWChunk);
-    // barriers: [0,2) stage full, [2,4) stage empty, 4 weights, [5,7) accumulators full, [7,9) accumulators
-    // empty (four epilogue warps), 9 done
-    volatile uint32_t *sh = reinterpret_cast<volatile uint32_t *>(bars + 10);
+    // barriers: [0,S) stage full, [S,2S) stage empty, then weights, two accumulators full, two accumulators
+    // empty (four epilogue warps), done
+    volatile uint32_t *sh = reinterpret_cast<volatile uint32_t *>(bars + 2 * S + 6);
     // sh: [0] TMEM base, [1] abort, [2] stage jobs issued, [3] stage jobs waited, [4] weights waited
-    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + 2), wfull = smem_u32(bars + 4),
-                   tfull0 = smem_u32(bars + 5), tempty0 = smem_u32(bars + 7), done = smem_u32(bars + 9);
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S), wfull = smem_u32(bars + 2 * S),
+                   tfull0 = smem_u32(bars + 2 * S + 1), tempty0 = smem_u32(bars + 2 * S + 3),
+                   done = smem_u32(bars + 2 * S + 5);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bz_n = (d.nz + kLineZ - 1) / kLineZ, by_n = (d.ny + kLineY - 1) / kLineY;
+    const int bz_n = (d.nz + kLineZ - 1) / kLineZ, by_n = (d.ny + Y - 1) / Y;
     const long long nbricks = (long long)bz_n * by_n * ((d.nx + LX - 1) / LX);
     const int nb = nbricks > blockIdx.x ? (int)((nbricks - 1 - blockIdx.x) / gridDim.x + 1) : 0;
     auto brick = [&](int bi, int &z0, int &y0, int &x0) {
         const long long br = blockIdx.x + (long long)bi * gridDim.x;
         z0 = kLineZ * (int)(br % bz_n);
-        y0 = kLineY * (int)((br / bz_n) % by_n);
+        y0 = Y * (int)((br / bz_n) % by_n);
         x0 = LX * (int)(br / ((long long)bz_n * by_n));
     };
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < S; s++) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; s++) {
             mbar_init(tfull0 + 8 * s, 1);
             mbar_init(tempty0 + 8 * s, 4);
         }
@@ -361,20 +373,19 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
         for (int bi = 0; bi < nb && !sh[1]; bi++) {
             int z0, y0, x0;
             brick(bi, z0, y0, x0);
-            for (int st = 0; st < 3 * KP && !sh[1]; st++, q++) {  // stage = (dz, 16-channel group)
-                const int dz = st / KP, jp = st % KP, s = q & 1;
-                if (q >= 2 && !mbar_wait(empty0 + 8 * s, (uint32_t)((q >> 1) - 1) & 1u)) {
+            for (int p = 0; p < 3 * KP * (LX + 2) && !sh[1]; p++, q++) {  // (dz, 16-channel group, x plane)
+                const int xb = p % (LX + 2), st = p / (LX + 2), dz = st / KP, jp = st % KP, s = q % S;
+                if (q >= S && !mbar_wait(empty0 + 8 * s, (uint32_t)(q / S - 1) & 1u)) {
                     sh[1] = 1;
                     break;
                 }
                 mbar_expect_tx(full0 + 8 * s, L::kStageBytes);
                 tma_load_4d(smem_u32(smem + s * L::kStageBytes), &tmap_x, full0 + 8 * s, 16 * jp, z0 + dz - 1, y0 - 1,
-                            x0 - 1);
+                            x0 - 1 + xb);
                 sh[2] = (uint32_t)(q + 1);
             }
         }
     } else if (warp == 0 && lane == 0 && nb > 0) {  // MMA issuer
-        constexpr uint32_t idesc = instr_desc_bf16(CO);
         bool any = false;
         if (!mbar_wait(wfull, 0)) sh[1] = 1;
         else sh[4] = 1;
@@ -386,33 +397,46 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int st = 0; st < 3 * KP; st++, q++) {
-                const int dz = st / KP, jp = st % KP, s = q & 1;
-                if (!mbar_wait(full0 + 8 * s, (uint32_t)(q >> 1) & 1u)) {
-                    sh[1] = 1;
-                    break;
-                }
-                sh[3] = (uint32_t)(q + 1);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // descriptor bases of this stage; every MMA below adds a compile-time offset in 16-byte units (the
-                // start field cannot carry: shared addresses stay below 256 KB)
-                const uint64_t ad0 = smem_desc_sw32(smem_u32(smem + s * L::kStageBytes));
-                const uint64_t bd0 = smem_desc_sw32(smem_u32(wbuf) + jp * L::kWChunk + (uint32_t)dz * CO * 32u);
+            for (int st = 0; st < 3 * KP && !sh[1]; st++) {
+                const int dz = st / KP, jp = st % KP;
+                // weights of this z shift and channel group; every MMA below adds a compile-time offset in 16-byte units
+                // (the start field cannot carry: shared addresses stay below 256 KB)
+                const uint64_t bd0 = smem_desc_sw32(smem_u32(wbuf) + jp * L::kWChunk + (uint32_t)dz * 9u * CO * 32u);
                 const uint32_t tacc = tmem + (uint32_t)(tb * L::kCols);
-                const uint32_t acc0 = st > 0 ? 1u : 0u;
 #pragma unroll
-                for (int pr = 0; pr < 9; pr++) {
-                    const int dx = pr / 3 - 1, dy = pr % 3 - 1;
-                    const uint64_t bd = bd0 + (uint64_t)((9 * (dx + 1) + 3 * (dy + 1)) * CO * 2);
-#pragma unroll
-                    for (int tile = 0; tile < kTiles; tile++) {
-                        const int yy = tile % kLineY, xx = tile / kLineY;
-                        const uint64_t ad = ad0 + (uint64_t)(256 * ((yy + 1 + dy) + (kLineY + 2) * (xx + 1 + dx)));
-                        mma_bf16(tacc + (uint32_t)(tile * CO), ad, bd, idesc, pr > 0 ? 1u : acc0);
+                for (int xb = 0; xb < LX + 2; xb++, q++) {
+                    const int s = q % S;
+                    if (!mbar_wait(full0 + 8 * s, (uint32_t)(q / S) & 1u)) {
+                        sh[1] = 1;
+                        break;
                     }
+                    sh[3] = (uint32_t)(q + 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad0 = smem_desc_sw32(smem_u32(smem + s * L::kStageBytes));
+#pragma unroll
+                    for (int xx = 0; xx < LX; xx++) {
+                        const int dx = xb - xx;  // this plane is tap dx of the tiles of column xx
+                        if (dx < 0 || dx > 2) continue;
+                        const uint64_t bd = bd0 + (uint64_t)(3 * dx * CO * 2);
+                        const bool first = dx == 0 && st == 0;
+                        if (first) {  // the brick's first tap overwrites its accumulator: by itself
+#pragma unroll
+                            for (int yb = 0; yb < Y; yb++)
+                                mma_bf16(tacc + (uint32_t)((xx * Y + Y - 1 - yb) * CO), ad0 + (uint64_t)(256 * yb), bd,
+                                         instr_desc_bf16(CO), 0u);
+                        }
+#pragma unroll
+                        for (int yb = 0; yb < Y + 2; yb++) {  // line yb meets the tiles yb - dy, dy0 <= dy <= dy1
+                            const int lo = yb < Y ? 0 : yb - Y + 1, dy1 = yb < 2 ? yb : 2;
+                            const int dy0 = first && lo == 0 ? 1 : lo;
+                            if (dy0 > dy1) continue;
+                            mma_bf16(tacc + (uint32_t)((xx * Y + Y - 1 - (yb - dy0)) * CO), ad0 + (uint64_t)(256 * yb),
+                                     bd + (uint64_t)(dy0 * CO * 2), instr_desc_bf16((dy1 - dy0 + 1) * CO), 1u);
+                        }
+                    }
+                    any = true;
+                    mma_commit(empty0 + 8 * s);
                 }
-                any = true;
-                mma_commit(empty0 + 8 * s);
             }
             if (sh[1]) break;
             mma_commit(tfull0 + 8 * tb);
@@ -441,13 +465,14 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
             const int z = z0 + 32 * q4 + lane;
 #pragma unroll 1
             for (int tile = 0; tile < kTiles; tile++) {
-                const int yy = y0 + tile % kLineY, xx = x0 + tile / kLineY;
+                const int yy = y0 + tile % Y, xx = x0 + tile / Y;
+                const int col = tile - tile % Y + Y - 1 - tile % Y;  // accumulators by descending y
                 const bool inb = z < d.nz && yy < d.ny && xx < d.nx;
                 const long long v = inb ? cid(d, xx, yy, z) : 0;
 #pragma unroll
                 for (int c0 = 0; c0 < CO; c0 += 16) {
                     float acc[16];
-                    tmem_ld_x16<16>(tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tb * L::kCols + tile * CO + c0),
+                    tmem_ld_x16<16>(tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tb * L::kCols + col * CO + c0),
                                     acc);
                     if (inb && EPI == 0) {
                         uint32_t pk[8];
@@ -476,7 +501,7 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
     }
     __syncthreads();
     if (threadIdx.x == 0 && sh[1]) {  // drain copies still in flight into this CTA's shared memory (bounded)
-        for (uint32_t q = sh[3]; q < sh[2]; q++) mbar_wait(full0 + 8 * (q & 1), (q >> 1) & 1u);
+        for (uint32_t q = sh[3]; q < sh[2]; q++) mbar_wait(full0 + 8 * (q % S), (q / S) & 1u);
         if (!sh[4] && nb > 0) mbar_wait(wfull, 0);
         atomicCAS(err, 0, 1);
     }
@@ -700,12 +725,18 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line64(const __grid_constant
 // N = (dz, Cin), both operands K-major with 8 consecutive z per 16-byte row.  k_to_chmajor makes channel-major copies
 // with z split into 8-voxel rows: dYT[zh][x][y][co][zl] and XT[zh][x][y][s][ci][zl] = X[x][y][8 zh + zl + s - 1][ci]
 // (zero outside), the three z shifts s = dz + 1 interleaved per row so that one TMA box starting on a row boundary
-// carries all three.  A job is one (dx, dy) pair over one brick of 32 (z) x 4 (y) x BX (x) voxels: one 5-D TMA box
-// (8, C, 4, BX, 4) lands as rows c + C k of 16 B, k = y + 4 (x + BX zh) the K index of the 8-voxel core matrices,
-// so consecutive K steps are C x 16 B apart (LBO) and 8-row groups 128 B (SBO); the y and x shifts are box
+// carries all three.  A job is one (dx, dy) pair over one brick of 32 (z) x 4 (y) x BX (x) voxels: one TMA box
+// of 8 z x C x 4 y x BX x x 4 zh lands as rows c + C k of 16 B, k = y + 4 (x + BX zh) the K index of the 8-voxel core
+// matrices, so consecutive K steps are C x 16 B apart (LBO) and 8-row groups 128 B (SBO); the y and x shifts are box
 // coordinates (outside the grid: zero fill).  One MMA (K = 16) then accumulates the three taps (dx, dy, -1..1) into
-// 3 Cin TMEM columns.  M = 128 rows of which the first Cout are dY channels; the rows past them read the next K
-// steps' rows (or a zeroed slack after the buffer) and land in accumulator lanes that are never read.
+// 3 Cin TMEM columns.  M = 64 rows of which the first Cout are dY channels; the rows past them read the next K
+// steps' rows (or a zeroed slack after the buffer) and land in accumulator lanes that are never read (M = 128 reads
+// twice the shared memory for nothing).
+// HALO (16 input channels, grids that hold the box): a job is one zh of a brick with all nine pairs: the box with its
+// halo, 6 y x (BX + 2) x, is read once for them, and as the rows of y, y + 1 and y + 2 follow one another one MMA of
+// N = 144 does the three dy.  16 to 16 channels at 128^3: 405 us with a box a pair and M = 128, 126 so
+// (the 6.5 KB an MMA reads, at 64 bytes a clock).
+// The maps take the contiguous (8 z, channels) as long rows: a row of 16 bytes costs the copy unit as much as one of 512.
 // One CTA (one per SM, 512 TMEM columns) runs a group of (dx, dy) pairs over a strided set of bricks, warp
 // specialised: lane 0 of warp 1 issues the TMA loads (dY of a brick once, into one of two buffers; X per pair through
 // a ring of stages), lane 0 of warp 0 the MMAs, so neither waits on the other's latency.  The CTA writes its partial
@@ -723,11 +754,15 @@ __host__ __device__ constexpr int wg_pairs_per_cta() {
     return CI == 16 ? 9 : CI == 32 ? 5 : 2;
 }
 
-template <int CI, int CO>
+// channels of one row of a box (8 z each, at most 256 elements)
+__host__ __device__ constexpr int wg_row_channels(int c) { return c <= 32 ? c : c % 32 == 0 ? 32 : 24; }
+
+template <int CI, int CO, bool HALO>
 struct WgLayout {
     static constexpr int BX = wg_bx<CI>();
     static constexpr uint32_t kABytes = 256u * CO * BX;  // 8 z x CO x 4 y x BX x x 4 zh, BF16
-    static constexpr uint32_t kBBytes = 768u * CI * BX;  // 8 z x 3 CI x 4 y x BX x x 4 zh
+    // 8 z x 3 CI x 4 y x BX x x 4 zh, or x 6 y x (BX + 2) x
+    static constexpr uint32_t kBBytes = HALO ? 48u * CI * 6u * (BX + 2) : 768u * CI * BX;
     static constexpr uint32_t kAStride = kABytes + kWgSlack;
     static constexpr int kStagesRaw = (int)((216u * 1024u - 2u * kAStride) / kBBytes);
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
@@ -737,46 +772,54 @@ struct WgLayout {
     static_assert(kStages >= 2 && kSmemBytes <= 227u * 1024u, "shared memory");
 };
 
-// dst[zh][x][y][s][c][zl] = src[x][y][8 zh + zl + s + shift0][c] where 8 zh + zl < nz and the shifted z lies in the
-// grid, else 0; s < ns, zh < nzh = ceil(nz / 8).  One thread per (zh, x, y, c): 16-byte stores.
-template <int C>
-__global__ void __launch_bounds__(256) k_to_chmajor(Dims d, int ns, int shift0, const __nv_bfloat16 *__restrict__ src,
+// dst[zh][x][y][s][c][zl] = src[x][y][8 zh + zl + s - (NS - 1) / 2][c] where 8 zh + zl < nz and the shifted z lies in
+// the grid, else 0; s < NS (1 or 3), zh < nzh = ceil(nz / 8).  A thread takes two channels of one (zh, x, y): each z is
+// read once, in 4-byte words, for all its shifts, and 32 bytes are stored per shift (a channel a thread and a read per
+// shift: 32 us for dY and 88 for X of 16 channels at 128^3, 23 and 56 now).
+template <int C, int NS>
+__global__ void __launch_bounds__(256) k_to_chmajor(Dims d, const __nv_bfloat16 *__restrict__ src,
                                                     __nv_bfloat16 *__restrict__ dst) {
-    const int nzh = (d.nz + 7) / 8;
-    const long long m = (long long)nzh * d.nx * d.ny * C;
-    const unsigned short *s16 = reinterpret_cast<const unsigned short *>(src);
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(e % C);
-        const long long r = e / C;  // ((zh nx + x) ny + y)
-        const int y = (int)(r % d.ny);
-        const long long t = r / d.ny;
-        const int x = (int)(t % d.nx), zh = (int)(t / d.nx);
-        const long long row = (((long long)x * d.ny + y) * d.nz) * C + c;  // src index of (x, y, 0, c)
-        for (int s = 0; s < ns; s++) {
-            uint32_t w[4];
+    static_assert(NS == 1 || NS == 3, "z shifts");
+    constexpr int P = C / 2;
+    const long long m = (long long)((d.nz + 7) / 8) * d.nx * d.ny * P;
+    const uint32_t *s32 = reinterpret_cast<const uint32_t *>(src);
+    for (long long e = blockIdx.x * 256LL + threadIdx.x; e < m; e += gridDim.x * 256LL) {
+        const int cp = (int)(e % P);
+        const unsigned r = (unsigned)(e / P), t = r / (unsigned)d.ny;  // r = (zh nx + x) ny + y
+        const int y = (int)(r - t * d.ny), zh = (int)(t / (unsigned)d.nx), x = (int)(t - (unsigned)zh * d.nx);
+        const uint32_t *row = s32 + ((long long)x * d.ny + y) * d.nz * P + cp;
+        uint32_t v[7 + NS];
+#pragma unroll
+        for (int q = 0; q < 7 + NS; q++) {
+            const int z = 8 * zh + q - (NS - 1) / 2;
+            v[q] = z >= 0 && z < d.nz ? row[(long long)z * P] : 0u;
+        }
+        const int nv = d.nz - 8 * zh;  // voxels of this 8-voxel row inside the grid
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            uint32_t lo[4], hi[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                uint32_t h[2];
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int z = 8 * zh + 2 * q + u, zs = z + s + shift0;
-                    h[u] = (z < d.nz && zs >= 0 && zs < d.nz) ? (uint32_t)s16[row + (long long)zs * C] : 0u;
-                }
-                w[q] = h[0] | (h[1] << 16);
+                const uint32_t a = 2 * q < nv ? v[2 * q + s] : 0u, b = 2 * q + 1 < nv ? v[2 * q + 1 + s] : 0u;
+                lo[q] = __byte_perm(a, b, 0x5410);
+                hi[q] = __byte_perm(a, b, 0x7632);
             }
-            *reinterpret_cast<uint4 *>(dst + ((r * ns + s) * C + c) * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+            uint4 *out = reinterpret_cast<uint4 *>(dst) + ((long long)r * NS + s) * C + 2 * cp;
+            out[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            out[1] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         }
     }
 }
 
-template <int CI, int CO>
+template <int CI, int CO, bool HALO>
 __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap tmap_dy,
                                                      const __grid_constant__ CUtensorMap tmap_x, Dims d,
                                                      float *__restrict__ part, int *err) {
     constexpr int NP = wg_pairs_per_cta<CI>();
     constexpr int N = 3 * CI;
-    static_assert(NP * N <= 512 && CO <= 128 && CI % 16 == 0 && CO % 16 == 0 && N <= 256, "shape");
-    using L = WgLayout<CI, CO>;
+    static_assert(NP * N <= 512 && CO <= 64 && CI % 16 == 0 && CO % 16 == 0 && N <= 256, "shape");
+    static_assert(!HALO || (NP == 9 && 3 * N <= 256), "halo form: every pair in one CTA, three of them an MMA");
+    using L = WgLayout<CI, CO, HALO>;
     constexpr int S = L::kStages, BX = L::BX;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -793,7 +836,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
     const int bz_n = (d.nz + 31) / 32, by_n = (d.ny + 3) / 4, bx_n = (d.nx + BX - 1) / BX;
     const long long nbricks = (long long)bz_n * by_n * bx_n;
     const int nb = nbricks > blockIdx.x ? (int)((nbricks - 1 - blockIdx.x) / gridDim.x + 1) : 0;
-    const int J = nb * npair;
+    const int JB = HALO ? 4 : npair, J = nb * JB;  // jobs per brick
 
     // zero the slack after each dY buffer (read by the MMA rows past Cout)
     for (uint32_t i = threadIdx.x; i < kWgSlack / 16; i += blockDim.x) {
@@ -837,7 +880,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
         bool ok = true;
         int a_issued = 0, b_issued = 0;
         for (int q = 0; q < J && ok; q++) {
-            const int bi = q / npair, jj = q % npair;
+            const int bi = q / JB, jj = q % JB;
             int z0, y0, x0;
             brick(bi, z0, y0, x0);
             if (jj == 0) {
@@ -857,18 +900,21 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
                 break;
             }
             mbar_expect_tx(bfull0 + 8 * s, L::kBBytes);
-            tma_load_5d(smem_u32(bbuf + s * L::kBBytes), &tmap_x, bfull0 + 8 * s, 0, 0, y0 + dy, x0 + dx, z0 / 8);
+            if (HALO)
+                tma_load_5d(smem_u32(bbuf + s * L::kBBytes), &tmap_x, bfull0 + 8 * s, 0, 0, y0 - 1, x0 - 1, z0 / 8 + jj);
+            else
+                tma_load_5d(smem_u32(bbuf + s * L::kBBytes), &tmap_x, bfull0 + 8 * s, 0, 0, y0 + dy, x0 + dx, z0 / 8);
             b_issued = q + 1;
         }
         sh[5] = ok ? 1u : 0u;
         sh[6] = (uint32_t)b_issued;
         sh[7] = (uint32_t)a_issued;
     } else if (warp == 0 && lane == 0) {  // MMA issuer
-        constexpr uint32_t idesc = instr_desc_bf16(N);
+        constexpr uint32_t idesc = instr_desc_bf16(HALO ? 3 * N : N, 64);
         bool ok = true;
         int a_waited = 0, b_waited = 0;
         for (int q = 0; q < J; q++) {
-            const int bi = q / npair, jj = q % npair, ab = bi & 1, s = q % S;
+            const int bi = q / JB, jj = q % JB, ab = bi & 1, s = q % S;
             if (jj == 0) {
                 if (!mbar_wait(afull0 + 8 * ab, (uint32_t)(bi >> 1) & 1u)) {
                     ok = false;
@@ -884,12 +930,23 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t ad0 = smem_desc(smem_u32(abuf + ab * L::kAStride), (uint32_t)CO * 16u, 128u);
             const uint64_t bd0 = smem_desc(smem_u32(bbuf + s * L::kBBytes), (uint32_t)N * 16u, 128u);
+            // start addresses advance in 16-byte units (no carry: < 256 KB)
+            if (HALO) {
+                const uint64_t ad = ad0 + (uint64_t)(jj * 4 * BX * CO);
 #pragma unroll
-            for (int p = 0; p < 8 * BX; p++)  // start addresses advance in 16-byte units (no carry: < 256 KB)
-                mma_bf16(tmem + (uint32_t)(jj * N), ad0 + (uint64_t)(2 * p * CO), bd0 + (uint64_t)(2 * p * N), idesc,
-                         (bi > 0 || p > 0) ? 1u : 0u);
+                for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                    for (int p = 0; p < 2 * BX; p++)  // p = y / 2 + 2 x
+                        mma_bf16(tmem + (uint32_t)(3 * dx * N), ad + (uint64_t)(2 * p * CO),
+                                 bd0 + (uint64_t)((2 * (p % 2) + 6 * (p / 2 + dx)) * N), idesc, (q > 0 || p > 0) ? 1u : 0u);
+            } else {
+#pragma unroll
+                for (int p = 0; p < 8 * BX; p++)
+                    mma_bf16(tmem + (uint32_t)(jj * N), ad0 + (uint64_t)(2 * p * CO), bd0 + (uint64_t)(2 * p * N), idesc,
+                             (bi > 0 || p > 0) ? 1u : 0u);
+            }
             mma_commit(bempty0 + 8 * s);
-            if (jj == npair - 1) mma_commit(aempty0 + 8 * ab);
+            if (jj == JB - 1) mma_commit(aempty0 + 8 * ab);
         }
         if (b_waited > 0) {  // completion of every MMA issued (also on the error path, before TMEM is released)
             mma_commit(done);
@@ -912,8 +969,8 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t st = sh[1];
-    if (st != 0 && 32 * warp < CO) {  // 1: the accumulators hold this CTA's sums; 2: no brick, the sums are zero
-        const int co = 32 * warp + lane;  // TMEM lane = dY channel
+    if (st != 0 && 16 * warp < CO) {  // 1: the accumulators hold this CTA's sums; 2: no brick, the sums are zero
+        const int co = lane < 16 ? 16 * warp + lane : CO;  // an M = 64 accumulator: 16 rows in each lane quarter
         for (int jj = 0; jj < npair; jj++) {
 #pragma unroll
             for (int sz = 0; sz < 3; sz++) {

@@ -56,10 +56,18 @@ template <int CI, int CO>
 void launch_conv(cudaStream_t st, int epi, const Dims &d, const bf16 *x, const bf16 *w, const float *b, void *y,
                  int taps) {
     const int blocks = (int)((d.n + 127) / 128);
-    if (epi == 0)
-        k_conv_mma<CI, CO, 0><<<blocks, 128, 0, st>>>(d, x, w, b, y, taps);
-    else
-        k_conv_mma<CI, CO, 1><<<blocks, 128, 0, st>>>(d, x, w, b, y, taps);
+    // 16 channels a block while that leaves each of the 152 SMs at most four blocks: 64 channels at 16^3 took 72 us in
+    // 32 blocks, 30 in 128 with the next tap's weights on their way
+    if (CO > 16 && (long long)blocks * (CO / 16) <= 4 * 152) {
+        if (epi == 0)
+            k_conv_mma<CI, CO, 0, 16><<<dim3(blocks, CO / 16), 128, 0, st>>>(d, x, w, b, y, taps);
+        else
+            k_conv_mma<CI, CO, 1, 16><<<dim3(blocks, CO / 16), 128, 0, st>>>(d, x, w, b, y, taps);
+    } else if (epi == 0) {
+        k_conv_mma<CI, CO, 0, CO><<<blocks, 128, 0, st>>>(d, x, w, b, y, taps);
+    } else {
+        k_conv_mma<CI, CO, 1, CO><<<blocks, 128, 0, st>>>(d, x, w, b, y, taps);
+    }
 }
 
 void conv_dispatch(cudaStream_t st, int ci, int co, int epi, const Dims &d, const bf16 *x, const bf16 *w,
@@ -116,25 +124,29 @@ cudaError_t launch_tc_mt(cudaStream_t st, const Dims &d, const bf16 *x, const bf
     return cudaGetLastError();
 }
 
-// 16 or 32 input channels, at most 32 output channels, on grids holding a 128 x 6 x (LX + 2) box: the z-line
-// kernel (one halo'd box per z shift and chunk for nine taps)
+// 16 or 32 input channels, at most 32 output channels, on grids holding a 128 x 6 box with 4 or 3 planes: the z-line
+// kernel (one halo'd box per z shift, plane and channel group for up to six taps)
 bool line_shape_ok(int ci, int co, const Dims &d) {
-    const int lx = ci == 16 ? tc::line_x<16>() : tc::line_x<32>();
     return (ci == 16 || ci == 32) && (co == 16 || co == 32) && d.nz >= tc::kLineZ && d.ny >= tc::kLineY + 2 &&
-           d.nx >= lx + 2;
+           d.nx >= (ci == 16 ? 4 : 3);
 }
 
-template <int CI, int CO, int EPI>
-cudaError_t launch_tc_line(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *w, const float *b, void *y,
-                           int *err) {
+long long line_bricks(const Dims &d, int y) {
+    return (long long)((d.nz + tc::kLineZ - 1) / tc::kLineZ) * ((d.ny + y - 1) / y) *
+           ((d.nx + tc::kLineX - 1) / tc::kLineX);
+}
+
+template <int CI, int CO, int EPI, int Y>
+cudaError_t launch_tc_line_y(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *wp, const float *b, void *y,
+                             int *err) {
     auto enc = tensor_map_encoder();
-    if (!enc || !aligned16(x) || !aligned16(w) || !aligned16(y)) return cudaErrorInvalidValue;
+    if (!enc || !aligned16(x) || !aligned16(wp) || !aligned16(y)) return cudaErrorInvalidValue;
     CUtensorMap mx, mw;
-    using L = tc::LineLayout<CI, CO>;
+    using L = tc::LineLayout<CI, CO, Y>;
     const cuuint64_t xd[4] = {(cuuint64_t)CI, (cuuint64_t)d.nz, (cuuint64_t)d.ny, (cuuint64_t)d.nx};
     const cuuint64_t xs[3] = {(cuuint64_t)CI * 2, (cuuint64_t)d.nz * CI * 2, (cuuint64_t)d.ny * d.nz * CI * 2};
     // 16 channels (32 bytes) per box row, written in the 32-byte swizzled layout the MMA descriptors read
-    const cuuint32_t xb[4] = {16, tc::kLineZ, tc::kLineY + 2, (cuuint32_t)L::LX + 2};
+    const cuuint32_t xb[4] = {16, tc::kLineZ, Y + 2, 1};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     if (enc(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16 *>(x), xd, xs, xb, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -143,18 +155,31 @@ cudaError_t launch_tc_line(cudaStream_t st, const Dims &d, const bf16 *x, const 
     const cuuint64_t wd[3] = {(cuuint64_t)CI, (cuuint64_t)CO, 27};
     const cuuint64_t ws[2] = {(cuuint64_t)CI * 2, (cuuint64_t)CO * CI * 2};
     const cuuint32_t wb[3] = {16, (cuuint32_t)CO, 27};
-    if (enc(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16 *>(w), wd, ws, wb, es,
+    if (enc(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16 *>(wp), wd, ws, wb, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(tc::k_conv_tc_line<CI, CO, EPI>,
+    cudaError_t e = cudaFuncSetAttribute(tc::k_conv_tc_line<CI, CO, EPI, Y>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmemBytes);
     if (e != cudaSuccess) return e;
-    const long long nbricks = (long long)((d.nz + tc::kLineZ - 1) / tc::kLineZ) *
-                              ((d.ny + tc::kLineY - 1) / tc::kLineY) * ((d.nx + L::LX - 1) / L::LX);
+    const long long nbricks = line_bricks(d, Y);
     const int grid = (int)(nbricks < 152 ? nbricks : 152);
-    tc::k_conv_tc_line<CI, CO, EPI><<<grid, 192, L::kSmemBytes, st>>>(mx, mw, d, b, y, err);
+    tc::k_conv_tc_line<CI, CO, EPI, Y><<<grid, 192, L::kSmemBytes, st>>>(mx, mw, d, b, y, err);
     return cudaGetLastError();
+}
+
+// 16 output channels have tensor memory for bricks eight lines high: taken where the box holds them and the fullest
+// CTA's lines, bricks x (Y + 2), are fewer (256^3: 540 and 648; a ny of 12 has 20 and 18 a column)
+template <int CI, int CO, int EPI>
+cudaError_t launch_tc_line(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *wp, const float *b, void *y,
+                           int *err) {
+    constexpr int Y = tc::kLineY;
+    if constexpr (CO == 16) {
+        const long long lines = (line_bricks(d, Y) + 151) / 152 * (Y + 2),
+                        lines2 = (line_bricks(d, 2 * Y) + 151) / 152 * (2 * Y + 2);
+        if (d.ny >= 2 * Y + 2 && lines2 < lines) return launch_tc_line_y<CI, CO, EPI, 2 * Y>(st, d, x, wp, b, y, err);
+    }
+    return launch_tc_line_y<CI, CO, EPI, Y>(st, d, x, wp, b, y, err);
 }
 
 // grids holding a 64 x 6 x 4 box: the 64-long z-line kernel (weights streamed per stage, taps ordered by z shift)
@@ -199,7 +224,7 @@ template <int CI, int CO, int EPI>
 cudaError_t launch_tc(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *w, const bf16 *wp, const float *b,
                       void *y, int *err) {
     if constexpr ((CI == 16 || CI == 32) && (CO == 16 || CO == 32))
-        if (line_shape_ok(CI, CO, d)) return launch_tc_line<CI, CO, EPI>(st, d, x, w, b, y, err);
+        if (wp && line_shape_ok(CI, CO, d)) return launch_tc_line<CI, CO, EPI>(st, d, x, wp, b, y, err);
     if (wp && line64_shape_ok(CI, CO, d)) return launch_tc_line64<CI, CO, EPI>(st, d, x, wp, b, y, err);
     constexpr int MT = tc::tiles_per_cta<CI, CO>();
     if (d.ny >= tc::kTileY * MT) return launch_tc_mt<CI, CO, EPI, MT>(st, d, x, w, b, y, err);
@@ -207,7 +232,7 @@ cudaError_t launch_tc(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 
 }
 
 // epi 0: forward (bias, ReLU, BF16 y); epi 1: input gradient (FP32 y, no bias).  wp: the weights with taps
-// ordered by z shift (the 64-long z-line kernel), or nullptr
+// ordered by z shift (the z-line kernels), or nullptr
 cudaError_t tc_dispatch(cudaStream_t st, int ci, int co, int epi, const Dims &d, const bf16 *x, const bf16 *w,
                         const bf16 *wp, const float *b, void *y, int *err) {
 #define CASE(A, B)                                                                              \
@@ -227,27 +252,32 @@ bool wgrad_tc_ok(int ci, int co, const Dims &d) {
 
 // channel-major z-row copies of dY and of X with its three z shifts (k_to_chmajor), then k_wgrad_tc over all
 // bricks; chunks receives the number of partial sums written to part
-template <int CI, int CO>
+template <int CI, int CO, bool HALO>
 cudaError_t launch_wgrad_tc(cudaStream_t st, const Dims &d, const bf16 *dy, const bf16 *x, bf16 *dyT, bf16 *xT,
                             float *part, long long part_cap, int &chunks, int *err) {
     auto enc = tensor_map_encoder();
     if (!enc || !aligned16(dyT) || !aligned16(xT) || !aligned16(part)) return cudaErrorInvalidValue;
-    using L = tc::WgLayout<CI, CO>;
+    using L = tc::WgLayout<CI, CO, HALO>;
     const long long nzh = (d.nz + 7) / 8;
     const long long rows = nzh * d.nx * d.ny;  // 8-voxel z rows of one channel
-    auto map5 = [&](CUtensorMap *m, const bf16 *base, int C) {
-        const cuuint64_t dims[5] = {8, (cuuint64_t)C, (cuuint64_t)d.ny, (cuuint64_t)d.nx, (cuuint64_t)nzh};
-        const cuuint64_t str[4] = {16, (cuuint64_t)C * 16, (cuuint64_t)d.ny * C * 16,
+    // (8 z, C) is contiguous and is taken in rows of 8 W elements
+    auto map5 = [&](CUtensorMap *m, const bf16 *base, int C, int by, int bx, int bz) {
+        const cuuint64_t W = (cuuint64_t)tc::wg_row_channels(C);
+        const cuuint64_t dims[5] = {8 * W, C / W, (cuuint64_t)d.ny, (cuuint64_t)d.nx, (cuuint64_t)nzh};
+        const cuuint64_t str[4] = {16 * W, (cuuint64_t)C * 16, (cuuint64_t)d.ny * C * 16,
                                    (cuuint64_t)d.nx * d.ny * C * 16};
-        const cuuint32_t box[5] = {8, (cuuint32_t)C, 4, (cuuint32_t)L::BX, 4};
+        const cuuint32_t box[5] = {(cuuint32_t)(8 * W), (cuuint32_t)(C / W), (cuuint32_t)by, (cuuint32_t)bx,
+                                   (cuuint32_t)bz};
         const cuuint32_t es[5] = {1, 1, 1, 1, 1};
         return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(base), dims, str, box, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
     CUtensorMap mdy, mx;
-    if (!map5(&mdy, dyT, CO) || !map5(&mx, xT, 3 * CI)) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(tc::k_wgrad_tc<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (!map5(&mdy, dyT, CO, 4, L::BX, 4) ||
+        !(HALO ? map5(&mx, xT, 3 * CI, 6, L::BX + 2, 1) : map5(&mx, xT, 3 * CI, 4, L::BX, 4)))
+        return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(tc::k_wgrad_tc<CI, CO, HALO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)L::kSmemBytes);
     if (e != cudaSuccess) return e;
     constexpr int NP = tc::wg_pairs_per_cta<CI>();
@@ -257,18 +287,21 @@ cudaError_t launch_wgrad_tc(cudaStream_t st, const Dims &d, const bf16 *dy, cons
     if (G > nbricks) G = nbricks;
     if (G * 27 * CO * CI > part_cap) G = part_cap / (27LL * CO * CI);
     if (G < 1) return cudaErrorInvalidValue;
-    tc::k_to_chmajor<CO><<<flat_blocks(rows * CO), 256, 0, st>>>(d, 1, 0, dy, dyT);
-    tc::k_to_chmajor<CI><<<flat_blocks(rows * CI), 256, 0, st>>>(d, 3, -1, x, xT);
-    tc::k_wgrad_tc<CI, CO><<<dim3((unsigned)G, groups), 128, L::kSmemBytes, st>>>(mdy, mx, d, part, err);
+    tc::k_to_chmajor<CO, 1><<<flat_blocks(rows * CO / 2), 256, 0, st>>>(d, dy, dyT);
+    tc::k_to_chmajor<CI, 3><<<flat_blocks(rows * CI / 2), 256, 0, st>>>(d, x, xT);
+    tc::k_wgrad_tc<CI, CO, HALO><<<dim3((unsigned)G, groups), 128, L::kSmemBytes, st>>>(mdy, mx, d, part, err);
     chunks = (int)G;
     return cudaGetLastError();
 }
 
 cudaError_t wgrad_tc_dispatch(cudaStream_t st, int ci, int co, const Dims &d, const bf16 *dy, const bf16 *x,
                               bf16 *dyT, bf16 *xT, float *part, long long part_cap, int &chunks, int *err) {
-#define CASE(A, B)                                                                             \
-    if (ci == A && co == B) return launch_wgrad_tc<A, B>(st, d, dy, x, dyT, xT, part, part_cap, chunks, err);
-    CASE(16, 16) CASE(16, 32) CASE(32, 16) CASE(32, 32) CASE(32, 64) CASE(64, 32) CASE(64, 64)
+    const bool halo = d.ny >= 6 && d.nx >= 4;  // the halo'd box lies within the grid's extents, as every other box
+#define CASE(A, B, H)                                                                                     \
+    if (ci == A && co == B && H == (A == 16 && halo))                                                     \
+        return launch_wgrad_tc<A, B, H>(st, d, dy, x, dyT, xT, part, part_cap, chunks, err);
+    CASE(16, 16, true) CASE(16, 32, true) CASE(16, 16, false) CASE(16, 32, false) CASE(32, 16, false)
+    CASE(32, 32, false) CASE(32, 64, false) CASE(64, 32, false) CASE(64, 64, false)
 #undef CASE
     return cudaErrorInvalidValue;
 }
@@ -348,14 +381,16 @@ void *UNet::alloc(size_t bytes) {
 }
 
 void UNet::refresh_bf16() {
+    RefreshLayers R{};
     for (const ConvLayer &L : layers_) {
         if (L.taps != 27) continue;
-        const long long m = (long long)L.taps * L.cout * L.cin;
-        k_f32_to_bf16<<<flat_blocks(m), 256, 0, st_>>>(m, p_ + L.woff, wb_ + L.wbf);
-        k_flip_weights<<<flat_blocks(m), 256, 0, st_>>>(L.taps, L.cout, L.cin, p_ + L.woff, wt_ + L.wbf);
-        k_taps_dz_major<<<flat_blocks(m), 256, 0, st_>>>(m, L.cout * L.cin, wb_ + L.wbf, wbp_ + L.wbf);
-        k_taps_dz_major<<<flat_blocks(m), 256, 0, st_>>>(m, L.cout * L.cin, wt_ + L.wbf, wtp_ + L.wbf);
+        R.ci[R.n] = L.cin;
+        R.co[R.n] = L.cout;
+        R.w[R.n] = L.woff;
+        R.wb[R.n++] = L.wbf;
+        R.wb[R.n] = L.wbf + 27LL * L.cout * L.cin;
     }
+    k_refresh_bf16<<<(unsigned)((R.wb[R.n] + 255) / 256), 256, 0, st_>>>(R, p_, wb_, wt_, wbp_, wtp_);
 }
 
 cudaError_t UNet::set_params(const float *host) {
@@ -532,7 +567,7 @@ void UNet::conv_bwd(const ConvLayer &L, const Dims &d, const bf16 *x, const bf16
                     float *dx) {
     const long long m = d.n * L.cout;
     bf16 *dy = gbf[L.level];
-    k_relu_back<<<flat_blocks(m), 256, 0, st_>>>(m, dpost, post, dy);
+    k_relu_back<<<flat_blocks(m / 8), 256, 0, st_>>>(m / 8, dpost, post, dy);
     long long vchunk = (d.n + 63) / 64;
     if (vchunk < kVchunkMin) vchunk = kVchunkMin;
     const int chunks = (int)((d.n + vchunk - 1) / vchunk);
@@ -565,7 +600,7 @@ void UNet::conv_bwd(const ConvLayer &L, const Dims &d, const bf16 *x, const bf16
         k_bias_grad<32><<<bchunks, 256, 0, st_>>>(d.n, dy, (int)bvchunk, hpart_);
     else
         k_bias_grad<64><<<bchunks, 256, 0, st_>>>(d.n, dy, (int)bvchunk, hpart_);
-    k_reduce_chunks<<<1, 64, 0, st_>>>(hpart_, bchunks, L.cout, g_ + L.boff);
+    k_reduce_long<<<L.cout, 256, 0, st_>>>(hpart_, bchunks, L.cout, g_ + L.boff);
     if (!dx) return;
     // input gradient: the forward convolution with the mirrored, transposed weights (FP32 out, no bias)
     if (mode_ == 1 && L.taps == 27 && tc_shape_ok(L.cout, L.cin, d)) {
@@ -591,8 +626,8 @@ cudaError_t UNet::backward(const Dims &d, const float *dout) {
         long long vchunk = (d0.n + 4095) / 4096;
         if (vchunk < 256) vchunk = 256;
         const int chunks = (int)((d0.n + vchunk - 1) / vchunk);
-        k_head_back<<<chunks, 64, 0, st_>>>(d0.n, 16, D0b, p_ + H.woff, dout, gA[0], (int)vchunk, hpart_);
-        k_reduce_chunks<<<1, 64, 0, st_>>>(hpart_, chunks, 17, g_ + H.woff);  // 16 weights then the bias
+        k_head_back<<<chunks, 64, 0, st_>>>(d0.n, D0b, p_ + H.woff, dout, gA[0], (int)vchunk, hpart_);
+        k_reduce_long<<<17, 256, 0, st_>>>(hpart_, chunks, 17, g_ + H.woff);  // 16 weights then the bias
     }
     conv_bwd(Ls[13], d0, D0a, D0b, gA[0], gB[0]);
     conv_bwd(Ls[12], d0, U0, D0a, gB[0], gU[0]);

@@ -45,14 +45,18 @@ __device__ __forceinline__ void tap_off(int t, int taps, int &dx, int &dy, int &
 
 // --------------------------------------------------------------------------------------------------------
 // y[v][co] = epi( sum_t sum_ci w[t][co][ci] x[v + off_t][ci] ), zero padding.
-// Block: 4 warps, 128 voxels (each warp two m16 tiles); one tap's weights staged in shared memory.
+// Block: 4 warps, 128 voxels (each warp two m16 tiles), CN of the output channels (blockIdx.y of CO / CN); one tap's
+// weights staged in shared memory.  The grids that come here are small (a level of fewer than 32 x 4 cells across): with
+// all 64 channels in one block the 16^3 level had 32 blocks for 152 SMs.
 // EPI 0: + bias, ReLU, BF16 out.  EPI 1: FP32 out, no bias (input gradient).
 // --------------------------------------------------------------------------------------------------------
-template <int CI, int CO, int EPI>
+template <int CI, int CO, int EPI, int CN>
 __global__ void __launch_bounds__(128) k_conv_mma(Dims d, const bf16 *__restrict__ x, const bf16 *__restrict__ w,
                                                   const float *__restrict__ bias, void *__restrict__ yout, int taps) {
-    static_assert(CI % 16 == 0 && CO % 8 == 0, "channel counts");
-    __shared__ __align__(16) bf16 ws[CO][CI + 8];
+    static_assert(CI % 16 == 0 && CN % 8 == 0 && CO % CN == 0, "channel counts");
+    __shared__ __align__(16) bf16 ws[2][CN][CI + 8];
+    constexpr int kW = CN * CI / 8;  // 16-byte groups of a tap's weights
+    const int co0 = blockIdx.y * CN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, tq = lane & 3;
     const long long vbase = (long long)blockIdx.x * 128 + warp * 32;
@@ -67,22 +71,25 @@ __global__ void __launch_bounds__(128) k_conv_mma(Dims d, const bf16 *__restrict
         cj_[r] = (int)((vv / d.nz) % d.ny);
         ci_[r] = (int)(vv / ((long long)d.nz * d.ny));
     }
-    float acc[2][CO / 8][4];
+    float acc[2][CN / 8][4];
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
-        for (int n = 0; n < CO / 8; n++)
+        for (int n = 0; n < CN / 8; n++)
 #pragma unroll
             for (int q = 0; q < 4; q++) acc[m][n][q] = 0.f;
 
+    auto weights = [&](int t, int e) {
+        return *reinterpret_cast<const uint4 *>(w + ((long long)t * CO + co0 + e / (CI / 8)) * CI + e % (CI / 8) * 8);
+    };
+    for (int e = threadIdx.x; e < kW; e += 128)
+        *reinterpret_cast<uint4 *>(&ws[0][e / (CI / 8)][e % (CI / 8) * 8]) = weights(0, e);
     for (int t = 0; t < taps; t++) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < CO * CI / 8; e += 128) {
-            const int co = e / (CI / 8), cc = e % (CI / 8);
-            *reinterpret_cast<uint4 *>(&ws[co][cc * 8]) =
-                *reinterpret_cast<const uint4 *>(w + ((long long)t * CO + co) * CI + cc * 8);
-        }
-        __syncthreads();
+        __syncthreads();  // this tap's weights are staged, and the other buffer is free
+        uint4 next[(kW + 127) / 128];
+#pragma unroll
+        for (int q = 0; q < (kW + 127) / 128; q++)
+            if (t + 1 < taps && (int)threadIdx.x + 128 * q < kW) next[q] = weights(t + 1, threadIdx.x + 128 * q);
         int dx, dy, dz;
         tap_off(t, taps, dx, dy, dz);
         const uint32_t *src[4];
@@ -104,12 +111,18 @@ __global__ void __launch_bounds__(128) k_conv_mma(Dims d, const bf16 *__restrict
                 a[m][3] = rb ? rb[(c0 >> 1) + 4 + tq] : 0u;
             }
 #pragma unroll
-            for (int n = 0; n < CO / 8; n++) {
-                const uint32_t *wr = reinterpret_cast<const uint32_t *>(&ws[n * 8 + g][c0]);
+            for (int n = 0; n < CN / 8; n++) {
+                const uint32_t *wr = reinterpret_cast<const uint32_t *>(&ws[t & 1][n * 8 + g][c0]);
                 const uint32_t b[2] = {wr[tq], wr[4 + tq]};
                 mma16816(acc[0][n], a[0], b);
                 mma16816(acc[1][n], a[1], b);
             }
+        }
+#pragma unroll
+        for (int q = 0; q < (kW + 127) / 128; q++) {
+            const int e = threadIdx.x + 128 * q;
+            if (t + 1 < taps && e < kW)
+                *reinterpret_cast<uint4 *>(&ws[(t + 1) & 1][e / (CI / 8)][e % (CI / 8) * 8]) = next[q];
         }
     }
 #pragma unroll
@@ -119,8 +132,8 @@ __global__ void __launch_bounds__(128) k_conv_mma(Dims d, const bf16 *__restrict
             const long long v = vbase + m * 16 + hh * 8 + g;
             if (v >= d.n) continue;
 #pragma unroll
-            for (int n = 0; n < CO / 8; n++) {
-                const int co = n * 8 + 2 * tq;
+            for (int n = 0; n < CN / 8; n++) {
+                const int co = co0 + n * 8 + 2 * tq;
                 float y0 = acc[m][n][2 * hh], y1 = acc[m][n][2 * hh + 1];
                 if (EPI == 0) {
                     y0 = fmaxf(y0 + bias[co], 0.f);
@@ -145,6 +158,8 @@ __global__ void __launch_bounds__(128) k_wgrad_mma(Dims d, const bf16 *__restric
     constexpr int WPM = 4 / (MT > 4 ? 4 : MT);    // warps per m tile
     static_assert(MT <= 4, "CO <= 64");
     __shared__ float red[4][CO > 16 ? 16 : CO][CI];
+    constexpr int kTile = 512;
+    __shared__ int nb[kTile];  // index of voxel + offset, -1 outside, of a tile of the chunk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, tq = lane & 3;
     const int mt = warp % MT, ks = warp / MT;
@@ -160,18 +175,31 @@ __global__ void __launch_bounds__(128) k_wgrad_mma(Dims d, const bf16 *__restric
         for (int q = 0; q < 4; q++) acc[n][q] = 0.f;
     const int co_a = mt * 16 + g, co_b = co_a + 8;
     const bool oka = co_a < CO, okb = co_b < CO;
-    auto xs = [&](long long v, int ci) -> bf16 {  // x[v + off_t][ci], 0 outside
-        if (v >= v_end) return __float2bfloat16(0.f);
-        const int k = (int)(v % d.nz), j = (int)((v / d.nz) % d.ny), i = (int)(v / ((long long)d.nz * d.ny));
-        const int ii = i + dx, jj = j + dy_, kk = k + dz;
-        if (ii < 0 || ii >= d.nx || jj < 0 || jj >= d.ny || kk < 0 || kk >= d.nz) return __float2bfloat16(0.f);
-        return x[cid(d, ii, jj, kk) * CI + ci];
+    auto xs = [&](int at, int ci) -> bf16 {  // x[v + off_t][ci], 0 outside
+        return at >= 0 ? x[(long long)at * CI + ci] : __float2bfloat16(0.f);
     };
     auto dys = [&](long long v, int co, bool okc) -> bf16 {
         return (okc && v < v_end) ? dy[v * CO + co] : __float2bfloat16(0.f);
     };
-    for (long long v0 = v_begin + 16LL * ks; v0 < v_end; v0 += 16LL * WPM) {
+    // the neighbours' indices once per tile, by the whole block: formed where they are used (twelve 64-bit divisions a
+    // step of 16 voxels) they were most of the kernel, 422 us for 64 x 64 channels at 16^3
+    for (long long tile = v_begin; tile < v_end; tile += kTile) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < kTile; q += 128) {
+        const long long v = tile + q;
+        int at = -1;
+        if (v < v_end) {
+            const int vi = (int)v, row = vi / d.nz, kk = vi - row * d.nz + dz, i = row / d.ny, jj = row - i * d.ny + dy_,
+                      ii = i + dx;
+            if (ii >= 0 && ii < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz) at = (int)cid(d, ii, jj, kk);
+        }
+        nb[q] = at;
+    }
+    __syncthreads();
+    const long long tile_end = min(tile + kTile, v_end);
+    for (long long v0 = tile + 16LL * ks; v0 < tile_end; v0 += 16LL * WPM) {
         const long long va = v0 + 2 * tq, vb = va + 8;
+        const int q0 = (int)(va - tile), na0 = nb[q0], na1 = nb[q0 + 1], nb0 = nb[q0 + 8], nb1 = nb[q0 + 9];
         uint32_t a[4];
         a[0] = pack_raw(dys(va, co_a, oka), dys(va + 1, co_a, oka));
         a[1] = pack_raw(dys(va, co_b, okb), dys(va + 1, co_b, okb));
@@ -180,9 +208,10 @@ __global__ void __launch_bounds__(128) k_wgrad_mma(Dims d, const bf16 *__restric
 #pragma unroll
         for (int n = 0; n < CI / 8; n++) {
             const int ci = n * 8 + g;
-            const uint32_t b[2] = {pack_raw(xs(va, ci), xs(va + 1, ci)), pack_raw(xs(vb, ci), xs(vb + 1, ci))};
+            const uint32_t b[2] = {pack_raw(xs(na0, ci), xs(na1, ci)), pack_raw(xs(nb0, ci), xs(nb1, ci))};
             mma16816(acc[n], a, b);
         }
+    }
     }
     // reduce the WPM warps of each m tile through shared memory (fixed order)
     for (int s = 0; s < WPM; s++) {
@@ -212,13 +241,54 @@ __global__ void __launch_bounds__(128) k_wgrad_mma(Dims d, const bf16 *__restric
     }
 }
 
-// sum over chunks (fixed order): dw[t][co][ci] = sum_c part[c][t][co][ci]
+// sum over chunks (fixed order): dw[t][co][ci] = sum_c part[c][t][co][ci].  The sum of one element is a serial chain; its
+// values are loaded eight at a time ahead of it (43 us for 16 x 16 weights with one load in flight).
 __global__ void k_reduce_chunks(const float *__restrict__ part, int chunks, long long m, float *__restrict__ out) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
         float s = 0.f;
-        for (int c = 0; c < chunks; c++) s += part[(long long)c * m + e];
+        int c = 0;
+        for (; c + 8 <= chunks; c += 8) {
+            float v[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[q] = part[(long long)(c + q) * m + e];
+#pragma unroll
+            for (int q = 0; q < 8; q++) s += v[q];
+        }
+        for (; c < chunks; c++) s += part[(long long)c * m + e];
         out[e] = s;
     }
+}
+
+// The same for few elements and many chunks (the biases and the head: up to 64 elements of up to 4096 chunks): a block an
+// element, which brings 1024 values into shared memory at once for the one thread that adds them in order.  A thread an
+// element, each load waiting for the sum before it, took 330 us for the head and 70 us for a bias; 15 and 5 us now.
+__global__ void __launch_bounds__(256) k_reduce_long(const float *__restrict__ part, int chunks, int m,
+                                                     float *__restrict__ out) {
+    __shared__ __align__(16) float v[1024];
+    const int e = blockIdx.x;
+    float s = 0.f;
+    for (int c0 = 0; c0 < chunks; c0 += 1024) {
+        const int n = min(1024, chunks - c0);
+        __syncthreads();
+        for (int q = threadIdx.x; q < n; q += 256) v[q] = part[(long long)(c0 + q) * m + e];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int q = 0;
+            for (; q + 8 <= n; q += 8) {
+                const float4 a = *reinterpret_cast<const float4 *>(v + q), b = *reinterpret_cast<const float4 *>(v + q + 4);
+                s += a.x;
+                s += a.y;
+                s += a.z;
+                s += a.w;
+                s += b.x;
+                s += b.y;
+                s += b.z;
+                s += b.w;
+            }
+            for (; q < n; q++) s += v[q];
+        }
+    }
+    if (threadIdx.x == 0) out[e] = s;
 }
 
 // bias gradient partials: part[chunk][co] = sum_{v in chunk} dy[v][co].  256 threads per chunk: thread t sums
@@ -343,11 +413,17 @@ __global__ void __launch_bounds__(256) k_up_back(Dims d, Dims dc, const float *_
     *reinterpret_cast<float4 *>(dcoarse + cid(dc, I, J, K) * C + 4 * g) = s;
 }
 
-// dpre = dpost * (post > 0), BF16 out (input of the MMA gradient kernels)
-__global__ void k_relu_back(long long m, const float *__restrict__ dpost, const bf16 *__restrict__ post,
-                            bf16 *__restrict__ dpre) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x)
-        dpre[e] = __float2bfloat16(__bfloat162float(post[e]) > 0.f ? dpost[e] : 0.f);
+// dpre = dpost * (post > 0), BF16 out (input of the MMA gradient kernels); m8 groups of eight channels
+__global__ void __launch_bounds__(256) k_relu_back(long long m8, const float *__restrict__ dpost,
+                                                   const bf16 *__restrict__ post, bf16 *__restrict__ dpre) {
+    for (long long e = blockIdx.x * 256LL + threadIdx.x; e < m8; e += gridDim.x * 256LL) {
+        const float4 a = reinterpret_cast<const float4 *>(dpost)[2 * e], b = reinterpret_cast<const float4 *>(dpost)[2 * e + 1];
+        float p[8], f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        bf16x8_to_f32(reinterpret_cast<const uint4 *>(post)[e], p);
+#pragma unroll
+        for (int q = 0; q < 8; q++) f[q] = p[q] > 0.f ? f[q] : 0.f;
+        reinterpret_cast<uint4 *>(dpre)[e] = f32_to_bf16x8(f);
+    }
 }
 
 // 1x1 head: out[v] = b + sum_c w[c] a[v][c]  (FP32 out), 16 channels read as two 16-byte groups
@@ -370,28 +446,41 @@ __global__ void __launch_bounds__(256) k_head_fwd(long long n, const bf16 *__res
     }
 }
 
-// head backward: da[v][c] = dout[v] w[c] (FP32); weight/bias partials per block chunk
-__global__ void k_head_back(long long n, int C, const bf16 *__restrict__ a, const float *__restrict__ w,
-                            const float *__restrict__ dout, float *__restrict__ da, int vchunk,
-                            float *__restrict__ part /*[chunks][C+1]*/) {
+// head backward (16 channels): da[v][c] = dout[v] w[c] (FP32); weight/bias partials per block chunk.  A thread takes whole
+// voxels in 16-byte pieces (a channel at a time it was 162 us at 128^3, 43 now: 268 MB).
+__global__ void __launch_bounds__(64) k_head_back(long long n, const bf16 *__restrict__ a, const float *__restrict__ w,
+                                                  const float *__restrict__ dout, float *__restrict__ da, int vchunk,
+                                                  float *__restrict__ part /*[chunks][17]*/) {
     const long long v0 = (long long)blockIdx.x * vchunk, v1 = min(v0 + vchunk, n);
     __shared__ float sh[64][17];
-    float acc[17];
-    for (int c = 0; c <= C; c++) acc[c] = 0.f;
-    for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-        const float g = dout[v];
-        for (int c = 0; c < C; c++) {
-            da[v * C + c] = g * w[c];
-            acc[c] += g * __bfloat162float(a[v * C + c]);
-        }
-        acc[C] += g;
+    float acc[17], wr[16];
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+        acc[c] = 0.f;
+        wr[c] = w[c];
     }
-    for (int c = 0; c <= C; c++) sh[threadIdx.x][c] = acc[c];
+    acc[16] = 0.f;
+#pragma unroll 2
+    for (long long v = v0 + threadIdx.x; v < v1; v += 64) {
+        const float g = dout[v];
+        float f[16];
+        bf16x8_to_f32(reinterpret_cast<const uint4 *>(a)[2 * v], *reinterpret_cast<float(*)[8]>(f));
+        bf16x8_to_f32(reinterpret_cast<const uint4 *>(a)[2 * v + 1], *reinterpret_cast<float(*)[8]>(f + 8));
+#pragma unroll
+        for (int c = 0; c < 16; c += 4)
+            reinterpret_cast<float4 *>(da)[4 * v + c / 4] =
+                make_float4(g * wr[c], g * wr[c + 1], g * wr[c + 2], g * wr[c + 3]);
+#pragma unroll
+        for (int c = 0; c < 16; c++) acc[c] += g * f[c];
+        acc[16] += g;
+    }
+#pragma unroll
+    for (int c = 0; c <= 16; c++) sh[threadIdx.x][c] = acc[c];
     __syncthreads();
-    if (threadIdx.x <= C) {
+    if (threadIdx.x <= 16) {
         float s = 0.f;
-        for (int t = 0; t < (int)blockDim.x; t++) s += sh[t][threadIdx.x];
-        part[(long long)blockIdx.x * (C + 1) + threadIdx.x] = s;
+        for (int t = 0; t < 64; t++) s += sh[t][threadIdx.x];
+        part[(long long)blockIdx.x * 17 + threadIdx.x] = s;
     }
 }
 
@@ -411,27 +500,31 @@ __global__ void k_adam(long long m, float *__restrict__ p, const float *__restri
     }
 }
 
-// weights for the input gradient: wt[t'][ci][co] = w[taps-1-t'][co][ci] (mirrored taps, transposed channels)
-__global__ void k_flip_weights(int taps, int CO, int CI, const float *__restrict__ w, bf16 *__restrict__ wt) {
-    const long long m = (long long)taps * CO * CI;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
-        const int ci = (int)(e % CI), co = (int)((e / CI) % CO), t = (int)(e / ((long long)CI * CO));
-        wt[((long long)(taps - 1 - t) * CI + ci) * CO + co] = __float2bfloat16(w[e]);
-    }
-}
-
-// wp[9 dz + pr][co][ci] = w[3 pr + dz][co][ci]: the 27 taps reordered so that those of one z shift are
-// consecutive (pr = 3 (dx + 1) + (dy + 1), dz the z shift + 1)
-__global__ void k_taps_dz_major(long long m, int coci, const bf16 *__restrict__ w, bf16 *__restrict__ wp) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
-        const int tp = (int)(e / coci), r = (int)(e % coci);
-        wp[e] = w[(long long)(3 * (tp % 9) + tp / 9) * coci + r];
-    }
-}
-
-__global__ void k_f32_to_bf16(long long m, const float *__restrict__ a, bf16 *__restrict__ b) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x)
-        b[e] = __float2bfloat16(a[e]);
+// The BF16 copies of every 27-tap layer's weights in one launch (56 launches of 3 us before):
+//   wb  as stored, [tap][co][ci];
+//   wt  for the input gradient: wt[26 - t][ci][co] = w[t][co][ci] (mirrored taps, transposed channels);
+//   wbp, wtp  the same two with the taps of one z shift consecutive: tap 3 pr + dz goes to 9 dz + pr
+//   (pr = 3 (dx + 1) + (dy + 1), dz the z shift + 1).
+struct RefreshLayers {
+    int n;
+    int ci[16], co[16];
+    long long w[16], wb[17];  // offsets of the FP32 weights and of the copies (ascending)
+};
+__global__ void __launch_bounds__(256) k_refresh_bf16(RefreshLayers L, const float *__restrict__ p, bf16 *__restrict__ wb,
+                                                      bf16 *__restrict__ wt, bf16 *__restrict__ wbp,
+                                                      bf16 *__restrict__ wtp) {
+    const long long e = blockIdx.x * 256LL + threadIdx.x;
+    if (e >= L.wb[L.n]) return;
+    int l = 0;
+    while (e >= L.wb[l + 1]) l++;
+    const int r = (int)(e - L.wb[l]), CI = L.ci[l], CO = L.co[l], cc = CI * CO;
+    const int t = r / cc, rr = r - t * cc, co = rr / CI, ci = rr - co * CI, tm = 26 - t;
+    const bf16 v = __float2bfloat16(p[L.w[l] + r]);
+    const long long o = L.wb[l], tr = (long long)ci * CO + co;
+    wb[o + r] = v;
+    wt[o + (long long)tm * cc + tr] = v;
+    wbp[o + (long long)(9 * (t % 3) + t / 3) * cc + rr] = v;
+    wtp[o + (long long)(9 * (tm % 3) + tm / 3) * cc + tr] = v;
 }
 
 }  // namespace sf
