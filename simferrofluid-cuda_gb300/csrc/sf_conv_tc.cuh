@@ -775,7 +775,7 @@ struct WgLayout {
 // dst[zh][x][y][s][c][zl] = src[x][y][8 zh + zl + s - (NS - 1) / 2][c] where 8 zh + zl < nz and the shifted z lies in
 // the grid, else 0; s < NS (1 or 3), zh < nzh = ceil(nz / 8).  A thread takes two channels of one (zh, x, y): each z is
 // read once, in 4-byte words, for all its shifts, and 32 bytes are stored per shift (a channel a thread and a read per
-// shift: 32 us for dY and 88 for X of 16 channels at 128^3, 23 and 56 now).
+// shift: 32 us for dY and 76 for X of 16 channels at 128^3, 23 and 56 now).
 template <int C, int NS>
 __global__ void __launch_bounds__(256) k_to_chmajor(Dims d, const __nv_bfloat16 *__restrict__ src,
                                                     __nv_bfloat16 *__restrict__ dst) {

@@ -153,33 +153,30 @@ __device__ __forceinline__ typename Acc<C>::T diag_of(const Coef<C> &cf, long lo
 // --------------------------------------------------------------------------------------------------------
 constexpr int kRedThreads = 256;
 
-template <int K>
-__device__ __forceinline__ void warp_sum(double (&v)[K]) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int q = 0; q < K; q++) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-}
-
-// Fixed-order tree sum of one value per thread over a kRedThreads block; result valid in tid 0.
+// Fixed-order sum of one value per thread over a kRedThreads block; result valid in tid 0.  The block's values go
+// through shared memory to its first warp: 12 FP64 instructions a value, where a shuffle tree in every warp issues 48
+// (each costs the SM's FP64 pipe 16 clocks whatever the lanes, and all blocks of a launch end together).
 template <int K>
 __device__ __forceinline__ void block_sum(double (&acc)[K], int tid) {
     __shared__ double sh2[K][kRedThreads];
 #pragma unroll
     for (int q = 0; q < K; q++) sh2[q][tid] = acc[q];
     __syncthreads();
-    for (int s = kRedThreads / 2; s > 0; s >>= 1) {
-        if (tid < s)
+    if (tid < 32) {
 #pragma unroll
-            for (int q = 0; q < K; q++) sh2[q][tid] += sh2[q][tid + s];
-        __syncthreads();
+        for (int w = 1; w < kRedThreads / 32; w++)
+#pragma unroll
+            for (int q = 0; q < K; q++) acc[q] += sh2[q][32 * w + tid];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < K; q++) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
     }
-#pragma unroll
-    for (int q = 0; q < K; q++) acc[q] = sh2[q][0];
     __syncthreads();
 }
 
 constexpr int kRedGroup = 256;  // blocks per first-level group
+constexpr int kRedFlat = 2048;  // grids of at most so many blocks are one group: the second level costs 1.5 us
 
 // Warp sum of FP32 values as an unevaluated (hi, lo) pair of floats: each shuffle stage adds the partner's pair
 // with the exact two-sum (Knuth), keeps the rounding error in lo and renormalises, so the sum carries about 48
@@ -207,85 +204,94 @@ __device__ __forceinline__ void warp_sum_df(const float (&v)[K], float (&hi_out)
     }
 }
 
-// Deterministic grid-wide sum.  Blocks write partials; the last block of each group of kRedGroup blocks sums
-// its group in block order; the last group to finish sums the group partials in group order.  Returns true in
-// exactly one thread (linear thread 0 of that block) with `tot` holding the totals.  Blocks must have
-// kRedThreads threads (any shape).  part: K * (nblk + ngroups) doubles; ticket: 1 + ngroups counters, zero on
-// entry and re-armed on exit.  Per-thread values are doubles (warp stage in FP64) or floats (warp stage as a
-// float pair, warp_sum_df); the block and grid stages are FP64.
+// Deterministic grid-wide sum.  Blocks write partials; the last block of each group of kRedGroup blocks (of the whole
+// grid up to kRedFlat blocks) sums its group in a fixed order; the last group to finish sums the group partials in group
+// order.  Returns true in exactly one thread (linear thread 0 of that block) with `tot` holding the totals.  Blocks must
+// have kRedThreads threads (any shape).  part: K * (nblk + ngroups) doubles; ticket: 1 + ngroups counters, zero on
+// entry and re-armed on exit.  Per-thread values are doubles or floats (warp stage as a float pair, warp_sum_df); the
+// block and grid stages are FP64, in the first warp only: with the warps' pairs converted and added by one thread,
+// (r, z) and (z, q) of a 256^3 potential took 43 us, 37 so (of a pool half full, 24 and 17).
 template <int K, class V>
 __device__ __forceinline__ bool grid_reduce(V (&v)[K], double *part, unsigned *ticket, double (&tot)[K]) {
-    __shared__ double sh[K][kRedThreads / 32];
-    __shared__ float shf[K][2][kRedThreads / 32];
     __shared__ bool last;
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     const int nblk = gridDim.x * gridDim.y * gridDim.z;
     const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int ngroups = (nblk + kRedGroup - 1) / kRedGroup;
-    const int grp = bid / kRedGroup;
-    const int gsize = min(kRedGroup, nblk - grp * kRedGroup);
+    const int group = nblk <= kRedFlat ? nblk : kRedGroup;
+    const int ngroups = (nblk + group - 1) / group;
+    const int grp = bid / group;
+    const int gsize = min(group, nblk - grp * group);
     double *gpart = part + (long long)K * nblk;
-    const int lane = tid & 31, wid = tid >> 5;
-    constexpr bool kFloat = std::is_same<V, float>::value;
-    if constexpr (kFloat) {
+    double acc[K];
+    if constexpr (std::is_same<V, float>::value) {
+        __shared__ float shf[K][2][kRedThreads / 32];
         float hi[K], lo[K];
         warp_sum_df<K>(v, hi, lo);
-        if (lane == 0)
+        if ((tid & 31) == 0)
 #pragma unroll
             for (int q = 0; q < K; q++) {
-                shf[q][0][wid] = hi[q];
-                shf[q][1][wid] = lo[q];
+                shf[q][0][tid >> 5] = hi[q];
+                shf[q][1][tid >> 5] = lo[q];
             }
-    } else {
-        warp_sum<K>(v);
-        if (lane == 0)
+        __syncthreads();
+        if (tid < 32) {
 #pragma unroll
-            for (int q = 0; q < K; q++) sh[q][wid] = v[q];
+            for (int q = 0; q < K; q++) {
+                const int w = tid & (kRedThreads / 32 - 1);
+                acc[q] = (double)shf[q][0][w] + (double)shf[q][1][w];
+            }
+#pragma unroll
+            for (int o = kRedThreads / 64; o > 0; o >>= 1)
+#pragma unroll
+                for (int q = 0; q < K; q++) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < K; q++) acc[q] = v[q];
+        block_sum<K>(acc, tid);
     }
-    __syncthreads();
     if (tid == 0) {
 #pragma unroll
-        for (int q = 0; q < K; q++) {
-            double b = 0;
-            for (int w = 0; w < kRedThreads / 32; w++)
-                b += kFloat ? ((double)shf[q][0][w] + (double)shf[q][1][w]) : sh[q][w];
-            part[(long long)q * nblk + bid] = b;
-        }
+        for (int q = 0; q < K; q++) part[(long long)q * nblk + bid] = acc[q];
         __threadfence();
         const unsigned t = atomicAdd(&ticket[1 + grp], 1u);
         last = (t == (unsigned)gsize - 1);
     }
     __syncthreads();
     if (!last) return false;
-    // last block of the group: sum the group's partials in block order
-    __threadfence();
-    double acc[K];
-#pragma unroll
-    for (int q = 0; q < K; q++)
-        acc[q] = tid < gsize ? ((volatile double *)part)[(long long)q * nblk + grp * kRedGroup + tid] : 0.0;
-    block_sum<K>(acc, tid);
-    if (tid == 0) {
-#pragma unroll
-        for (int q = 0; q < K; q++) gpart[(long long)q * ngroups + grp] = acc[q];
-        ticket[1 + grp] = 0u;
-        __threadfence();
-        const unsigned t = atomicAdd(&ticket[0], 1u);
-        last = (t == (unsigned)ngroups - 1);
-    }
-    __syncthreads();
-    if (!last) return false;
-    // last group: sum the group partials in group order
+    // last block of the group: sum the group's partials
     __threadfence();
 #pragma unroll
     for (int q = 0; q < K; q++) acc[q] = 0;
-    for (int g = tid; g < ngroups; g += kRedThreads)
+#pragma unroll 4
+    for (int t = tid; t < gsize; t += kRedThreads)
 #pragma unroll
-        for (int q = 0; q < K; q++) acc[q] += ((volatile double *)gpart)[(long long)q * ngroups + g];
+        for (int q = 0; q < K; q++) acc[q] += __ldcg(&part[(long long)q * nblk + grp * group + t]);
     block_sum<K>(acc, tid);
+    if (tid == 0) ticket[1 + grp] = 0u;
+    if (ngroups > 1) {
+        if (tid == 0) {
+#pragma unroll
+            for (int q = 0; q < K; q++) gpart[(long long)q * ngroups + grp] = acc[q];
+            __threadfence();
+            const unsigned t = atomicAdd(&ticket[0], 1u);
+            last = (t == (unsigned)ngroups - 1);
+        }
+        __syncthreads();
+        if (!last) return false;
+        // last group: sum the group partials in group order
+        __threadfence();
+#pragma unroll
+        for (int q = 0; q < K; q++) acc[q] = 0;
+        for (int g = tid; g < ngroups; g += kRedThreads)
+#pragma unroll
+            for (int q = 0; q < K; q++) acc[q] += __ldcg(&gpart[(long long)q * ngroups + g]);
+        block_sum<K>(acc, tid);
+        if (tid == 0) ticket[0] = 0u;
+    }
     if (tid != 0) return false;
 #pragma unroll
     for (int q = 0; q < K; q++) tot[q] = acc[q];
-    ticket[0] = 0u;
     return true;
 }
 

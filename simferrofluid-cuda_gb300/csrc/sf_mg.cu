@@ -72,6 +72,12 @@ dim3 tile_grid(const Dims &d, int &xpb, int max_blocks) {
     return dim3((unsigned)(items < max_blocks ? items : max_blocks), 1, 1);
 }
 
+// VEC_ROWS kernels: a warp a row
+static unsigned vec_grid(const Dims &d) {
+    const long long g = ((long long)d.nx * d.ny + 7) / 8;
+    return (unsigned)(g < kMaxRedBlocks ? g : kMaxRedBlocks);
+}
+
 void Tracker::before(cudaStream_t st, bool fine) {
     launches++;
     if (!prof || !fine) return;
@@ -691,39 +697,42 @@ __global__ void __launch_bounds__(256) k_rbgs_pipe(Dims d, Coef<T> cf, const T *
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// r = b - A x on the fine level, summed over each coarse cell's (up to) 8 children -> coarse rhs.
+// r = b - A x on the fine level, summed over each coarse cell's (up to) 8 children, in the order (di, dj, dk) -> coarse
+// rhs.  Four threads a coarse cell: with one, a 64^3 level has seven warps an SM and the kernel is the latency of eight
+// residuals in turn (11.0 us for FP64, 6.4 with four).
+constexpr int kRestrictJ = 2;  // coarse rows of a block
 template <class T, class C>
 __global__ void __launch_bounds__(256) k_resid_restrict(Dims d, Coef<C> cf, const T *__restrict__ x,
                                                         const T *__restrict__ b, Dims dc, T *__restrict__ bc,
                                                         const uint8_t *__restrict__ rows = nullptr,
                                                         const uint8_t *__restrict__ rows_c = nullptr) {
     pdl_entry();
-    const int K = blockIdx.x * blockDim.x + threadIdx.x;
-    const int J = blockIdx.y * blockDim.y + threadIdx.y;
-    const int I = blockIdx.z;
-    if (K >= dc.nz || J >= dc.ny || !row_on(rows_c, dc, I, J)) return;
-    T acc = 0;
+    // thread (K, child row sub, J): the residuals of the two children k = 2K, 2K + 1 of child row sub = 2 di + dj
+    __shared__ T sh[kRestrictJ][4][2][32];
+    const int K = blockIdx.x * 32 + threadIdx.x, sub = threadIdx.y & 3, jl = threadIdx.y >> 2;
+    const int J = blockIdx.y * kRestrictJ + jl, I = blockIdx.z;
+    const bool on = K < dc.nz && J < dc.ny && row_on(rows_c, dc, I, J);
+    const int i = 2 * I + (sub >> 1), j = 2 * J + (sub & 1);
+    T res[2] = {T(0), T(0)};
+    if (on && i < d.nx && j < d.ny && row_on(rows, d, i, j)) {  // else residual zero
 #pragma unroll
-    for (int di = 0; di < 2; di++) {
-        const int i = 2 * I + di;
-        if (i >= d.nx) break;
-#pragma unroll
-        for (int dj = 0; dj < 2; dj++) {
-            const int j = 2 * J + dj;
-            if (j >= d.ny) break;
-            if (!row_on(rows, d, i, j)) continue;  // residual zero
-#pragma unroll
-            for (int dk = 0; dk < 2; dk++) {
-                const int k = 2 * K + dk;
-                if (k >= d.nz) break;
-                const long long c = cid(d, i, j, k);
-                T sa;
-                T s = nbsum<T, C, sizeof(C) != 8>(d, cf, x, i, j, k, c, sa);
-                T D = (T)diag_of<C>(cf, c, (typename Acc<C>::T)sa);
-                acc += (b[c] - D * x[c]) + s;
-            }
+        for (int dk = 0; dk < 2; dk++) {
+            const int k = 2 * K + dk;
+            if (k >= d.nz) break;
+            const long long c = cid(d, i, j, k);
+            T sa;
+            T s = nbsum<T, C, sizeof(C) != 8>(d, cf, x, i, j, k, c, sa);
+            T D = (T)diag_of<C>(cf, c, (typename Acc<C>::T)sa);
+            res[dk] = (b[c] - D * x[c]) + s;
         }
     }
+    sh[jl][sub][0][threadIdx.x] = res[0];
+    sh[jl][sub][1][threadIdx.x] = res[1];
+    __syncthreads();
+    if (!on || sub != 0) return;
+    T acc = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) acc += sh[jl][q >> 1][q & 1][threadIdx.x];
     bc[cid(dc, I, J, K)] = acc;
 }
 
@@ -750,46 +759,46 @@ constexpr int kCoarseMax = 1024, kCoarseThreads = 1024;
 // that by rounding, and Gauss-Seidel sweeps then drift along the constant, the further the more sweeps run (which
 // degrades the preconditioner).  coarse_consistent subtracts the mean of b over the active cells (D > 0) on such
 // a level and returns b unchanged on any other.  Every thread of the block calls it, one cell each; the sums run
-// in a fixed order (warp shuffles, then the warps in order), so equal inputs give equal bits.
+// in a fixed order (warp shuffles, then the warps in order by one thread: 32 FP64 sums and a division in each of 32 warps
+// were 12 of k_coarse_smem<double>'s 48 us), so equal inputs give equal bits.
 template <class R>
 __device__ __forceinline__ R coarse_consistent(R bc, bool active, bool excess) {
-    __shared__ R s_sum[32];
+    __shared__ R s_sum[32], s_mean;
     __shared__ int s_cnt[32];
     if (__syncthreads_or(excess ? 1 : 0)) return bc;
     R s = active ? bc : R(0);
-    int m = active ? 1 : 0;
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_down_sync(0xffffffffu, s, o);
-        m += __shfl_down_sync(0xffffffffu, m, o);
-    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    const int m = __popc(__ballot_sync(0xffffffffu, active));
     if ((threadIdx.x & 31) == 0) {
         s_sum[threadIdx.x >> 5] = s;
         s_cnt[threadIdx.x >> 5] = m;
     }
     __syncthreads();
-    R tot = 0;
-    int cnt = 0;
-    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); w++) {
-        tot += s_sum[w];
-        cnt += s_cnt[w];
+    if (threadIdx.x == 0) {
+        R tot = 0;
+        int cnt = 0;
+        for (int w = 0; w < (int)((blockDim.x + 31) >> 5); w++) {
+            tot += s_sum[w];
+            cnt += s_cnt[w];
+        }
+        s_mean = cnt > 0 ? tot / R(cnt) : R(0);
     }
-    return active && cnt > 0 ? bc - tot / R(cnt) : bc;
+    __syncthreads();
+    return active ? bc - s_mean : bc;
 }
 
-template <class T, class C>
-__global__ void __launch_bounds__(kCoarseThreads) k_coarse_smem(Dims d, Coef<C> cf, T *__restrict__ x,
-                                                                const T *__restrict__ b, int pairs) {
-    pdl_entry();
-    using R = typename Acc<C>::T;
-    __shared__ T xs[kCoarseMax];
+// The coarsest solve of at most kCoarseMax cells by one block of at least d.n threads (the others only help with the
+// barriers): b made consistent, x = 0, then the sequence red, (black, red) x pairs.  xs: the solution, in shared memory.
+// b is read before xs is written.  A thread then owns a pair k = 2 m, 2 m + 1 of a row, one cell of either colour, so
+// that every lane of half the warps works in each half sweep and only those warps meet at its barrier (17 half sweeps of
+// 8^3 cells in FP64: 23 us with a cell a thread, bound by the FP64 pipe, 14 so; 97 of 5 x 4 x 4 cells, bound by the chain
+// of eight operations, 36 either way).
+template <class R, class T, class C>
+__device__ __forceinline__ void coarse_pairs(const Dims &d, const Coef<C> &cf, const T *b, T *xs, int pairs) {
+    static_assert(std::is_same<R, T>::value, "b waits in xs");
     const int sx = d.ny * d.nz, sy = d.nz;
-    const int c = threadIdx.x;
-    R a[6], inv = 0, bc = 0;
-    int has = 0, col = -1;
-    if (c < d.n) {
-        const int k = c % d.nz, j = (c / d.nz) % d.ny, i = c / (d.nz * d.ny);
-        col = (i + j + k) & 1;
-        // neighbour order and guards of nbsum: -x, +x, -y, +y, -z, +z
+    // neighbour order and guards of nbsum: -x, +x, -y, +y, -z, +z
+    auto cell = [&](int c, int i, int j, int k, int &has, R(&a)[6], R &inv) {  // a: 0 where there is no neighbour
         has = (i > 0) | ((i < d.nx - 1) << 1) | ((j > 0) << 2) | ((j < d.ny - 1) << 3) | ((k > 0) << 4) |
               ((k < d.nz - 1) << 5);
         R sum = 0;
@@ -805,26 +814,77 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse_smem(Dims d, Coef<C> 
             }
             a[f] = av;
         }
-        inv = inv_diag<C>(cf, c, sum);
-        bc = (R)b[c];
-        xs[c] = T(0);
-    }
-    bc = coarse_consistent<R>(bc, c < d.n && inv > R(0), c < d.n && ldv(cf.dex, c) != R(0));
-    __syncthreads();
-    const int nh = 1 + 2 * pairs;
-    for (int h = 0; h < nh; h++) {
-        if (col == (h & 1)) {
-            R s = 0;
-#pragma unroll
-            for (int f = 0; f < 6; f++) {
-                const int st = f < 2 ? sx : (f < 4 ? sy : 1);
-                if (has & (1 << f)) s += a[f] * (R)xs[(f & 1) ? c + st : c - st];
-            }
-            xs[c] = (T)((bc + s) * inv);
+        inv = (R)inv_diag<C>(cf, c, sum);
+    };
+    R a[2][6], inv[2] = {0, 0}, bc[2] = {0, 0};
+    int cc[2] = {-1, -1}, nb[2][6];
+    {
+        const int c = threadIdx.x;
+        R bn = 0, in = 0;
+        bool excess = false;
+        if (c < d.n) {
+            const int k = c % d.nz, j = (c / d.nz) % d.ny, i = c / (d.nz * d.ny);
+            R t[6];
+            int h;
+            cell(c, i, j, k, h, t, in);
+            bn = (R)b[c];
+            excess = ldv(cf.dex, c) != (decltype(ldv(cf.dex, c)))0;
         }
+        bn = coarse_consistent<R>(bn, c < d.n && in > R(0), excess);
+        if (c < d.n) xs[c] = (T)bn;
         __syncthreads();
     }
-    if (c < d.n) x[c] = xs[c];
+    const int np = (d.nz + 1) >> 1, own = d.nx * d.ny * np;  // pairs of a row, of the grid
+    if ((int)threadIdx.x < own) {
+        const int row = threadIdx.x / np, m = threadIdx.x - row * np, i = row / d.ny, j = row - i * d.ny;
+#pragma unroll
+        for (int col = 0; col < 2; col++) {
+            const int k = 2 * m + ((i + j + col) & 1);
+            if (k >= d.nz) continue;
+            cc[col] = row * d.nz + k;
+            int has;
+            cell(cc[col], i, j, k, has, a[col], inv[col]);
+            bc[col] = xs[cc[col]];
+#pragma unroll
+            for (int f = 0; f < 6; f++) {  // a missing neighbour is the cell itself, times 0: no branch in the sweeps
+                const int st = f < 2 ? sx : (f < 4 ? sy : 1);
+                nb[col][f] = cc[col] + ((has >> f) & 1 ? ((f & 1) ? st : -st) : 0);
+            }
+        }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < d.n) xs[threadIdx.x] = T(0);
+    __syncthreads();
+    const int nthr = (own + 31) & ~31;
+    if ((int)threadIdx.x < nthr) {
+        auto half = [&](int col) {
+            const int c = cc[col];
+            if (c >= 0) {
+                R v[6], s = 0;
+#pragma unroll
+                for (int f = 0; f < 6; f++) v[f] = xs[nb[col][f]];
+#pragma unroll
+                for (int f = 0; f < 6; f++) s += a[col][f] * v[f];
+                xs[c] = (T)((bc[col] + s) * inv[col]);
+            }
+            asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+        };
+        half(0);
+        for (int h = 0; h < pairs; h++) {
+            half(1);
+            half(0);
+        }
+    }
+    __syncthreads();
+}
+
+template <class T, class C>
+__global__ void __launch_bounds__(kCoarseThreads) k_coarse_smem(Dims d, Coef<C> cf, T *__restrict__ x,
+                                                                const T *__restrict__ b, int pairs) {
+    pdl_entry();
+    __shared__ T xs[kCoarseMax];
+    coarse_pairs<typename Acc<C>::T>(d, cf, b, xs, pairs);
+    if ((int)threadIdx.x < d.n) x[threadIdx.x] = xs[threadIdx.x];
 }
 
 template <class T, class C>
@@ -1103,7 +1163,7 @@ static void apply_dot32(cudaStream_t st, const Dims &d, const Coef<float> &cf, c
     for (long long row_ = blockIdx.x * 8LL + threadIdx.y, nrows_ = (long long)(d).nx * (d).ny; row_ < nrows_; \
          row_ += (long long)gridDim.x * 8) {                                                                  \
         if ((rows) && !(rows)[row_]) continue;                                                                \
-        for (int k_ = threadIdx.x; k_ < (d).nz; k_ += 32) {                                                   \
+        _Pragma("unroll 4") for (int k_ = threadIdx.x; k_ < (d).nz; k_ += 32) {                               \
             const long long c = row_ * (d).nz + k_;
 #define VEC_ROWS_END \
     }                \
@@ -1776,14 +1836,15 @@ static void restrict_res(cudaStream_t st, Tracker &tk, const Dims &d, const Coef
             return;
         }
     }
-    launch_pdl(k_resid_restrict<T, C>, grid_cells(dc), blk2(), st, d, cf, x, b, dc, bc, rows, rows_c);
+    const dim3 g((dc.nz + 31) / 32, (dc.ny + kRestrictJ - 1) / kRestrictJ, dc.nx);
+    launch_pdl(k_resid_restrict<T, C>, g, dim3(32, 4 * kRestrictJ), st, d, cf, x, b, dc, bc, rows, rows_c);
 }
 
 template <class T, class C>
 static void coarse_solve(cudaStream_t st, Tracker &tk, const Dims &d, const Coef<C> &cf, T *x, const T *b, int pairs) {
     tk.launches++;
     if (d.n <= kCoarseMax) {
-        launch_pdl(k_coarse_smem<T, C>, 1, kCoarseThreads, st, d, cf, x, b, pairs);
+        launch_pdl(k_coarse_smem<T, C>, 1, (unsigned)((d.n + 31) / 32 * 32), st, d, cf, x, b, pairs);
         return;
     }
     int nt = d.n >= 1024 ? 1024 : (int)((d.n + 31) / 32 * 32);
@@ -2316,11 +2377,11 @@ void MGSolver::enqueue_iter64(bool copy_slots) {
     vcycle<double, double, double, double>(st_, tk_, lev_dims_, c64_[0], c64_[0], c64_, z_, r_, x64_, b64_,
                                            prm_.smoother == 1 ? t64_ : std::vector<double *>(t64_.size(), nullptr),
                                            prm_, false, rows64_ ? &rs : nullptr);
-    launch_pdl(k_dot_rz<double>, kMaxRedBlocks, dim3(32, 8), st_, d, r0, r_, z_, q_, prm_.flexible ? 1 : 0, sc_,
+    launch_pdl(k_dot_rz<double>, vec_grid(d), dim3(32, 8), st_, d, r0, r_, z_, q_, prm_.flexible ? 1 : 0, sc_,
                part_, ticket_);
-    launch_pdl(k_xpby<double>, kMaxRedBlocks, dim3(32, 8), st_, d, r0, z_, p_, sc_);
+    launch_pdl(k_xpby<double>, vec_grid(d), dim3(32, 8), st_, d, r0, z_, p_, sc_);
     launch_pdl(k_apply_dot<double, double>, tg, dim3(32, 8), st_, d, xpb, c64_[0], p_, q_, sc_, part_, ticket_, r0);
-    launch_pdl(k_update<double>, kMaxRedBlocks, dim3(32, 8), st_, d, r0, x_, r_, p_, q_, sc_, part_, ticket_);
+    launch_pdl(k_update<double>, vec_grid(d), dim3(32, 8), st_, d, r0, x_, r_, p_, q_, sc_, part_, ticket_);
     tk_.launches += 4;
     iter_launches64_ = tk_.launches - l0;
     if (copy_slots) cudaMemcpyAsync(sc_host_, sc_, 8 * S_NSLOTS, cudaMemcpyDeviceToHost, st_);
@@ -2358,10 +2419,10 @@ void MGSolver::enqueue_iter32(bool copy_slots) {
         vcycle<float, float, __half, float>(st_, tk_, lev_dims_, c32_, c32_, c16_, z32_, ri32_, x32_, b32_, ts,
                                             prm_, false, nullptr, tail_lt_, tail_smem_, tail_nc_, tail_op_.data());
     const uint8_t *nr = nullptr;
-    launch_pdl(k_dot_rz<float>, kMaxRedBlocks, dim3(32, 8), st_, d, nr, ri32_, z32_, q32_, 1, sc_, part_, ticket_);
-    launch_pdl(k_xpby<float>, kMaxRedBlocks, dim3(32, 8), st_, d, nr, z32_, p32_, sc_);
+    launch_pdl(k_dot_rz<float>, vec_grid(d), dim3(32, 8), st_, d, nr, ri32_, z32_, q32_, 1, sc_, part_, ticket_);
+    launch_pdl(k_xpby<float>, vec_grid(d), dim3(32, 8), st_, d, nr, z32_, p32_, sc_);
     apply_dot32(st_, d, c32_, p32_, q32_, sc_, part_, ticket_);
-    launch_pdl(k_update<float>, kMaxRedBlocks, dim3(32, 8), st_, d, nr, d32_, ri32_, p32_, q32_, sc_, part_, ticket_);
+    launch_pdl(k_update<float>, vec_grid(d), dim3(32, 8), st_, d, nr, d32_, ri32_, p32_, q32_, sc_, part_, ticket_);
     tk_.launches += 4;
     iter_launches32_ = tk_.launches - l0;
     if (copy_slots) cudaMemcpyAsync(sc_host_, sc_, 8 * S_NSLOTS, cudaMemcpyDeviceToHost, st_);

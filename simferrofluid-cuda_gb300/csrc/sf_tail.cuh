@@ -363,60 +363,9 @@ __device__ void tail_prolong(cg::cluster_group &cl, const TailLv &f, const TailL
     cl.sync();
 }
 
-// The coarsest level solved on CTA 0 as k_coarse_smem does: b made consistent on a pure-Neumann level
-// (coarse_consistent), x = 0, then the palindromic sequence red, (black, red) x pairs, each cell's couplings (FP16,
-// global memory) pre-multiplied by the level's unscale.  x and b are the
-// level's arrays in CTA 0, in natural order.
+// The coarsest level solved on CTA 0 as k_coarse_smem does.  x and b are the level's arrays in CTA 0, in natural order.
 __device__ void tail_coarse(cg::cluster_group &cl, const TailLv &v, int rank, int pairs) {
-    const Dims &d = v.d;
-    const Coef<__half> &cf = v.L->cf;
-    if (rank == 0) {
-        float *xs = v.a.x;
-        const int sx = d.ny * d.nz, sy = d.nz;
-        const int c = threadIdx.x;
-        float a[6], inv = 0.f, bc = 0.f;
-        int has = 0, col = -1;
-        if (c < d.n) {
-            const int k = c % d.nz, j = (c / d.nz) % d.ny, i = c / (d.nz * d.ny);
-            col = (i + j + k) & 1;
-            has = (i > 0) | ((i < d.nx - 1) << 1) | ((j > 0) << 2) | ((j < d.ny - 1) << 3) | ((k > 0) << 4) |
-                  ((k < d.nz - 1) << 5);
-            float sum = 0.f;
-#pragma unroll
-            for (int f = 0; f < 6; f++) {
-                const __half *arr = f < 2 ? cf.ax : (f < 4 ? cf.ay : cf.az);
-                const int st = f < 2 ? sx : (f < 4 ? sy : 1);
-                float av = 0.f;
-                if (has & (1 << f)) {
-                    av = __half2float(arr[(f & 1) ? c + st : c]);
-                    av *= cf.unscale;
-                    sum += av;
-                }
-                a[f] = av;
-            }
-            float e = __half2float(cf.dex[c]);
-            e *= cf.unscale;
-            const float D = sum + e;
-            inv = D > 0.f ? 1.f / D : 0.f;
-            bc = v.a.b[c];
-            xs[c] = 0.f;
-        }
-        bc = coarse_consistent<float>(bc, c < d.n && inv > 0.f, c < d.n && __half2float(cf.dex[c]) != 0.f);
-        __syncthreads();
-        const int nh = 1 + 2 * pairs;
-        for (int h = 0; h < nh; h++) {
-            if (col == (h & 1)) {
-                float s = 0.f;
-#pragma unroll
-                for (int f = 0; f < 6; f++) {
-                    const int st = f < 2 ? sx : (f < 4 ? sy : 1);
-                    if (has & (1 << f)) s += a[f] * xs[(f & 1) ? c + st : c - st];
-                }
-                xs[c] = (bc + s) * inv;
-            }
-            __syncthreads();
-        }
-    }
+    if (rank == 0) coarse_pairs<float>(v.d, v.L->cf, (const float *)v.a.b, v.a.x, pairs);
     cl.sync();
 }
 
