@@ -492,57 +492,49 @@ __device__ __forceinline__ float c_of(const Coef<C> &cf, float c32) {
     return c32;
 }
 
-// Loads of a uniform-row update: the other colour's x around the colour-`col` cells m0 .. m0 + 3 of row (i, j).
+// Loads of a uniform-row update: the other colour's x around the colour-`col` cells m0 .. m0 + 3 of row (i, j), 0 outside
+// the grid.
 struct Nb4 {
     float xm[4] = {0, 0, 0, 0}, xp[4] = {0, 0, 0, 0}, ym[4] = {0, 0, 0, 0}, yp[4] = {0, 0, 0, 0}, zo[4] = {0, 0, 0, 0};
     float zx = 0.f;  // the other colour's entry just outside the vector (m0 - 1 for even k, m0 + 4 for odd)
 };
-__device__ __forceinline__ void load_nb4(const Dims &d, const float *__restrict__ x, long long oth, int i, int j,
-                                         int m0, int qz, Nb4 &v) {
-    const int nh = d.nz >> 1;
-    const long long sx = (long long)d.ny * nh, sy = nh;
-    if (i > 0) ld4(x + oth - sx, v.xm);
-    if (i < d.nx - 1) ld4(x + oth + sx, v.xp);
-    if (j > 0) ld4(x + oth - sy, v.ym);
-    if (j < d.ny - 1) ld4(x + oth + sy, v.yp);
-    ld4(x + oth, v.zo);
+// at: the other colour's entry m0 of row (i, j)
+__device__ __forceinline__ void load_nb4(const Dims &d, const float *__restrict__ at, int i, int j, int m0, int qz,
+                                         Nb4 &v) {
+    const int nh = d.nz >> 1, sx = d.ny * nh;
+    if (i > 0) ld4(at - sx, v.xm);
+    if (i < d.nx - 1) ld4(at + sx, v.xp);
+    if (j > 0) ld4(at - nh, v.ym);
+    if (j < d.ny - 1) ld4(at + nh, v.yp);
+    ld4(at, v.zo);
     if (qz == 0) {
-        if (m0 > 0) v.zx = x[oth - 1];
+        if (m0 > 0) v.zx = at[-1];
     } else if (m0 + 4 < nh) {
-        v.zx = x[oth + 4];
+        v.zx = at[4];
     }
 }
-// sum of the in-grid neighbours of cell t (face order of the general path) and their count
+// Sum of the neighbours of cell t in the face order of the general path.  Those outside the grid are added as the zeros
+// that load_nb4 left, which changes no sum (a test and a count per face and cell: 383 instructions for the 8 cells a lane of
+// the product, and registers that the restriction lacked for four blocks an SM: 33.8 us at 256^3, 25.3 so).
 template <int QZ, int t>
-__device__ __forceinline__ void nb_sum(const Dims &d, const Nb4 &v, int i, int j, int m0, bool use_x, float &s,
-                                       float &n) {
-    const int k = 2 * (m0 + t) + QZ;
-    s = 0.f;
-    n = 0.f;
-    if (i > 0) {
-        if (use_x) s += v.xm[t];
-        n += 1.f;
-    }
-    if (i < d.nx - 1) {
-        if (use_x) s += v.xp[t];
-        n += 1.f;
-    }
-    if (j > 0) {
-        if (use_x) s += v.ym[t];
-        n += 1.f;
-    }
-    if (j < d.ny - 1) {
-        if (use_x) s += v.yp[t];
-        n += 1.f;
-    }
-    if (k > 0) {
-        if (use_x) s += QZ == 0 ? (t == 0 ? v.zx : v.zo[t == 0 ? 0 : t - 1]) : v.zo[t];
-        n += 1.f;
-    }
-    if (k < d.nz - 1) {
-        if (use_x) s += QZ == 0 ? v.zo[t] : (t == 3 ? v.zx : v.zo[t == 3 ? 3 : t + 1]);
-        n += 1.f;
-    }
+__device__ __forceinline__ float nb_sum(const Nb4 &v) {
+    float s = v.xm[t] + v.xp[t];
+    s += v.ym[t];
+    s += v.yp[t];
+    s += QZ == 0 ? (t == 0 ? v.zx : v.zo[t == 0 ? 0 : t - 1]) : v.zo[t];
+    s += QZ == 0 ? v.zo[t] : (t == 3 ? v.zx : v.zo[t == 3 ? 3 : t + 1]);
+    return s;
+}
+// whether cell t is an end of its row (k = 0 or nz - 1)
+template <int QZ, int t>
+__device__ __forceinline__ bool row_end(const Dims &d, int m0) {
+    return QZ == 0 ? t == 0 && m0 == 0 : t == 3 && m0 + 4 == d.nz >> 1;
+}
+// c times the number of in-grid neighbours, of the row's inner cells and of its two ends
+__device__ __forceinline__ void row_diag(const Dims &d, float c, int i, int j, float &in, float &end) {
+    const float nxy = (float)((i > 0) + (i < d.nx - 1) + (j > 0) + (j < d.ny - 1));
+    in = c * (nxy + 2.f);
+    end = c * (nxy + 1.f);
 }
 template <class Fn>
 __device__ __forceinline__ void for_cells4(int qz, Fn &&fn) {
@@ -563,8 +555,8 @@ __device__ __forceinline__ void for_cells4(int qz, Fn &&fn) {
 // 1 / (c n) for the row's interior cells (n = the in-grid x and y faces + 2) and for its two end cells (k = 0,
 // k = nz - 1: one z face fewer); c n is exact, as in the general path.
 __device__ __forceinline__ void row_inv(const Dims &d, float c, int i, int j, float &inv_in, float &inv_end) {
-    const float nxy = (float)((i > 0) + (i < d.nx - 1) + (j > 0) + (j < d.ny - 1));
-    const float di = c * (nxy + 2.f), de = c * (nxy + 1.f);
+    float di, de;
+    row_diag(d, c, i, j, di, de);
     inv_in = di > 0.f ? __frcp_rn(di) : 0.f;  // IEEE round-to-nearest reciprocal: the value of 1.f / di
     inv_end = de > 0.f ? __frcp_rn(de) : 0.f;
 }
@@ -636,14 +628,11 @@ __device__ __forceinline__ void rbgs4s_uniform(const Dims &d, float4 rcv, float 
     float bv[4], out[4];
     ld4(b + own, bv);
     Nb4 v;
-    if (!ZERO) load_nb4(d, x, oth, i, j, m0, qz, v);
+    if (!ZERO) load_nb4(d, x + oth, i, j, m0, qz, v);
     for_cells4(qz, [&](auto qc, auto tc) {
         constexpr int QZ = decltype(qc)::value, t = decltype(tc)::value;
-        float s, n;
-        nb_sum<QZ, t>(d, v, i, j, m0, !ZERO, s, n);
-        const int k = 2 * (m0 + t) + QZ;
-        const float inv = (k == 0 || k == d.nz - 1) ? inv_end : inv_in;
-        out[t] = (bv[t] + c * s) * inv;
+        const float inv = row_end<QZ, t>(d, m0) ? inv_end : inv_in;
+        out[t] = (bv[t] + c * (ZERO ? 0.f : nb_sum<QZ, t>(v))) * inv;
     });
     *reinterpret_cast<float4 *>(x + own) = make_float4(out[0], out[1], out[2], out[3]);
 }
@@ -651,71 +640,47 @@ __device__ __forceinline__ void rbgs4s_uniform(const Dims &d, float4 rcv, float 
 __device__ __forceinline__ void resid4_uniform(const Dims &d, float c, const float *__restrict__ x,
                                                const float *__restrict__ b, int col, int i, int j, int m0,
                                                float (&r)[4]) {
-    const int nh = d.nz >> 1;
-    const long long row = ((long long)i * d.ny + j) * nh + m0;
-    const long long own = (long long)col * (d.n >> 1) + row, oth = (long long)(col ^ 1) * (d.n >> 1) + row;
+    const unsigned nh = (unsigned)d.nz >> 1, hn = (unsigned)(d.n >> 1);
+    const unsigned row = ((unsigned)i * (unsigned)d.ny + (unsigned)j) * nh + (unsigned)m0;
+    const unsigned own = (col ? hn : 0u) + row, oth = (col ? 0u : hn) + row;
     const int qz = (i + j + col) & 1;
-    float xc[4], bv[4];
+    float xc[4], bv[4], d_in, d_end;
     ld4(x + own, xc);
     ld4(b + own, bv);
     Nb4 v;
-    load_nb4(d, x, oth, i, j, m0, qz, v);
+    load_nb4(d, x + oth, i, j, m0, qz, v);
+    row_diag(d, c, i, j, d_in, d_end);
     for_cells4(qz, [&](auto qc, auto tc) {
         constexpr int QZ = decltype(qc)::value, t = decltype(tc)::value;
-        float s, n;
-        nb_sum<QZ, t>(d, v, i, j, m0, true, s, n);
-        r[t] = (bv[t] - (c * n) * xc[t]) + c * s;
+        const float D = row_end<QZ, t>(d, m0) ? d_end : d_in;
+        r[t] = (bv[t] - D * xc[t]) + c * nb_sum<QZ, t>(v);
     });
 }
 
-__device__ __forceinline__ void apply4s_uniform(const Dims &d, float c, const float *__restrict__ p,
-                                                float *__restrict__ q, int col, int i, int j, int m0, float &acc) {
-    const int nh = d.nz >> 1;
-    const long long row = ((long long)i * d.ny + j) * nh + m0;
-    const long long own = (long long)col * (d.n >> 1) + row, oth = (long long)(col ^ 1) * (d.n >> 1) + row;
-    const int qz = (i + j + col) & 1;
-    float pc[4], out[4];
-    ld4(p + own, pc);
-    Nb4 v;
-    load_nb4(d, p, oth, i, j, m0, qz, v);
-    for_cells4(qz, [&](auto qc, auto tc) {
-        constexpr int QZ = decltype(qc)::value, t = decltype(tc)::value;
-        float s, n;
-        nb_sum<QZ, t>(d, v, i, j, m0, true, s, n);
-        out[t] = (c * n) * pc[t] - c * s;
-        acc += pc[t] * out[t];
-    });
-    *reinterpret_cast<float4 *>(q + own) = make_float4(out[0], out[1], out[2], out[3]);
-}
-
-// Both colours of a uniform row at once: cells m0 .. m0 + 3 of colour 0 and of colour 1 of row (i, j).  The
+// q = A p of both colours of a uniform row at once: cells m0 .. m0 + 3 of colour 0 and of colour 1 of row (i, j).  The
 // neighbour rows of one colour are the other colour's, so the two colours' loads serve each other (the own
-// values are the other colour's z row) and p is read from DRAM once per launch instead of once per colour.  Each
-// cell's q is apply4s_uniform's.
+// values are the other colour's z row) and p is read from DRAM once per launch instead of once per colour.
 __device__ __forceinline__ void apply4s_uniform2(const Dims &d, float c, const float *__restrict__ p,
                                                  float *__restrict__ q, int i, int j, int m0, float &acc) {
     const int nh = d.nz >> 1;
     const long long row = ((long long)i * d.ny + j) * nh + m0, hn = d.n >> 1;
     const int qz0 = (i + j) & 1;
     Nb4 v0, v1;  // v0: the colour-1 rows around colour 0 (v0.zo = colour 1's own row); v1 the converse
-    load_nb4(d, p, hn + row, i, j, m0, qz0, v0);
-    load_nb4(d, p, row, i, j, m0, qz0 ^ 1, v1);
-    float out0[4], out1[4];
+    load_nb4(d, p + hn + row, i, j, m0, qz0, v0);
+    load_nb4(d, p + row, i, j, m0, qz0 ^ 1, v1);
+    float out0[4], out1[4], d_in, d_end;
+    row_diag(d, c, i, j, d_in, d_end);
     for_cells4(qz0, [&](auto qc, auto tc) {
         constexpr int QZ = decltype(qc)::value, t = decltype(tc)::value;
-        float s, n;
-        nb_sum<QZ, t>(d, v0, i, j, m0, true, s, n);
-        out0[t] = (c * n) * v1.zo[t] - c * s;
+        out0[t] = (row_end<QZ, t>(d, m0) ? d_end : d_in) * v1.zo[t] - c * nb_sum<QZ, t>(v0);
         acc += v1.zo[t] * out0[t];
     });
+    *reinterpret_cast<float4 *>(q + row) = make_float4(out0[0], out0[1], out0[2], out0[3]);
     for_cells4(qz0 ^ 1, [&](auto qc, auto tc) {
         constexpr int QZ = decltype(qc)::value, t = decltype(tc)::value;
-        float s, n;
-        nb_sum<QZ, t>(d, v1, i, j, m0, true, s, n);
-        out1[t] = (c * n) * v0.zo[t] - c * s;
+        out1[t] = (row_end<QZ, t>(d, m0) ? d_end : d_in) * v0.zo[t] - c * nb_sum<QZ, t>(v1);
         acc += v0.zo[t] * out1[t];
     });
-    *reinterpret_cast<float4 *>(q + row) = make_float4(out0[0], out0[1], out0[2], out0[3]);
     *reinterpret_cast<float4 *>(q + hn + row) = make_float4(out1[0], out1[1], out1[2], out1[3]);
 }
 
@@ -941,7 +906,7 @@ __device__ __forceinline__ void resid_restrict_s_cells(const Dims &d, const Coef
 }
 
 template <class C, bool SOUT>
-__global__ void __launch_bounds__(256) k_resid_restrict_s(Dims d, Coef<C> cf, const float *__restrict__ x,
+__global__ void __launch_bounds__(256, 4) k_resid_restrict_s(Dims d, Coef<C> cf, const float *__restrict__ x,
                                                              const float *__restrict__ b, Dims dc,
                                                              float *__restrict__ bc, const uint8_t *__restrict__ rows,
                                                              const float *__restrict__ crow,
@@ -956,8 +921,8 @@ __global__ void __launch_bounds__(256) k_resid_restrict_s(Dims d, Coef<C> cf, co
     });
 }
 
-// x += P xc on the split level 0 (piecewise constant): both colours' entries m of row (i, j) take coarse cell
-// (i/2, j/2, m).
+// x += P xc on a split level (piecewise constant), colour 0 only: the post-smoothing that always follows begins by writing
+// colour 1, without reading it.  Entry m of row (i, j) takes coarse cell (i/2, j/2, m).
 __global__ void __launch_bounds__(256) k_prolong_s(Dims d, float *__restrict__ x, Dims dc, const float *__restrict__ xc,
                                                    const int *__restrict__ list, const int *__restrict__ count) {
     pdl_entry();
@@ -970,20 +935,17 @@ __global__ void __launch_bounds__(256) k_prolong_s(Dims d, float *__restrict__ x
         float v[4];
         ld4(xc + cid(dc, i >> 1, j >> 1, m0), v);
         const long long row = r * nh + m0;
-#pragma unroll
-        for (int col = 0; col < 2; col++) {
-            float *p = x + (long long)col * (d.n >> 1) + row;
-            float4 t = *reinterpret_cast<float4 *>(p);
-            t.x += v[0];
-            t.y += v[1];
-            t.z += v[2];
-            t.w += v[3];
-            *reinterpret_cast<float4 *>(p) = t;
-        }
+        float4 t = *reinterpret_cast<float4 *>(x + row);
+        t.x += v[0];
+        t.y += v[1];
+        t.z += v[2];
+        t.w += v[3];
+        *reinterpret_cast<float4 *>(x + row) = t;
     });
 }
 
-// x += P xc with both levels split: fine entries m0 .. m0 + 3 of row (i, j) (either colour, k = 2m or 2m + 1) take
+// k_prolong_s with both levels split (256^3: 19.0 us for both colours, 13.0 for one): fine entries m0 .. m0 + 3 of
+// row (i, j) (k = 2m or 2m + 1) take
 // coarse cells K = m0 .. m0 + 3 of coarse row (i/2, j/2): even K of colour (i/2 + j/2) & 1, odd K of the other,
 // at entries K / 2 (two float2 loads).
 __global__ void __launch_bounds__(256) k_prolong_ss(Dims d, float *__restrict__ x, Dims dc,
@@ -1003,16 +965,12 @@ __global__ void __launch_bounds__(256) k_prolong_ss(Dims d, float *__restrict__ 
         const float2 od = *reinterpret_cast<const float2 *>(xc + (long long)(pc ^ 1) * hc + base);
         const float v[4] = {ev.x, od.x, ev.y, od.y};
         const long long row = r * nh + m0;
-#pragma unroll
-        for (int col = 0; col < 2; col++) {
-            float *p = x + (long long)col * (d.n >> 1) + row;
-            float4 t = *reinterpret_cast<float4 *>(p);
-            t.x += v[0];
-            t.y += v[1];
-            t.z += v[2];
-            t.w += v[3];
-            *reinterpret_cast<float4 *>(p) = t;
-        }
+        float4 t = *reinterpret_cast<float4 *>(x + row);
+        t.x += v[0];
+        t.y += v[1];
+        t.z += v[2];
+        t.w += v[3];
+        *reinterpret_cast<float4 *>(x + row) = t;
     });
 }
 
@@ -1020,7 +978,7 @@ __global__ void __launch_bounds__(256) k_prolong_ss(Dims d, float *__restrict__ 
 // k_apply_dot).  Persistent: warps over (colour row, chunk of 32 vectors), rows without an active cell skipped
 // (q stays zero there).  Uniform rows are done for both colours in the colour-0 pass (apply4s_uniform2), so the
 // colour-1 pass reads only the general rows again.
-__global__ void __launch_bounds__(256, 3) k_apply_dot4s(Dims d, Coef<float> cf, const float *__restrict__ p,
+__global__ void __launch_bounds__(256, 2) k_apply_dot4s(Dims d, Coef<float> cf, const float *__restrict__ p,
                                                      float *__restrict__ q, const int *__restrict__ list,
                                                      const int *__restrict__ count, const float *__restrict__ crow,
                                                      double *sc, double *part, unsigned *ticket) {
