@@ -310,11 +310,23 @@ struct LineLayout {
     static_assert(CI % 16 == 0 && 2u * kCols <= 512u && kStages >= 3 && kSmemBytes <= 227u * 1024u, "line layout");
 };
 
+// EPI 2: as 0, and the 2x2x2 average pooling of y besides (a brick holds whole 2x2x2 cells; sums in k_pool's order).
+// EPI 3 (Cout = 16): the 1x1 head applied to y, which is not stored.  256^3: pooling and head by themselves read the 537
+// MB again, 92 and 87 us; in these epilogues, which run beside the next brick's MMAs, the convolutions take 523 and 474
+// us (531 without either).
+struct LineEpi {
+    __nv_bfloat16 *pool;
+    Dims dc;               // of the pooled grid
+    const float *hw, *hb;  // head
+    float *out;
+};
+
 template <int CI, int CO, int EPI, int Y>
 __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__ CUtensorMap tmap_x,
                                                          const __grid_constant__ CUtensorMap tmap_w, Dims d,
                                                          const float *__restrict__ bias, void *__restrict__ yout,
-                                                         int *err) {
+                                                         int *err, LineEpi ep) {
+    static_assert(EPI != 3 || CO == 16, "head");
     using L = LineLayout<CI, CO, Y>;
     constexpr int LX = kLineX, kTiles = L::kTiles, KP = L::KP, S = L::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -447,6 +459,12 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
         }
     } else if (warp >= 2 && nb > 0) {  // epilogue
         const int q4 = warp & 3;  // TMEM lane quarter of this warp
+        float hw[EPI == 3 ? 16 : 1], hb = 0.f;
+        if (EPI == 3) {
+#pragma unroll
+            for (int c = 0; c < 16; c++) hw[EPI == 3 ? c : 0] = ep.hw[c];
+            hb = ep.hb[0];
+        }
         for (int bi = 0; bi < nb; bi++) {
             const int tb = bi & 1;
             const uint32_t par = (uint32_t)(bi >> 1) & 1u;
@@ -463,34 +481,112 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
             int z0, y0, x0;
             brick(bi, z0, y0, x0);
             const int z = z0 + 32 * q4 + lane;
+            // 16 channels c0 .. of tile (yy, xx), after bias and ReLU, as BF16 pairs
+            auto relu16 = [&](int yy, int xx, int c0, uint32_t(&pk)[8]) {
+                float acc[16];
+                tmem_ld_x16<16>(tmem + ((uint32_t)(32 * q4) << 16) +
+                                    (uint32_t)(tb * L::kCols + (xx * Y + Y - 1 - yy) * CO + c0),
+                                acc);  // accumulators by descending y
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const float a0 = fmaxf(acc[2 * k] + bias[c0 + 2 * k], 0.f);
+                    const float a1 = fmaxf(acc[2 * k + 1] + bias[c0 + 2 * k + 1], 0.f);
+                    __nv_bfloat162 h2 = __floats2bfloat162_rn(a0, a1);
+                    pk[k] = *reinterpret_cast<uint32_t *>(&h2);
+                }
+            };
+            auto put16 = [&](long long v, int c0, const uint32_t(&pk)[8]) {
+                uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(yout) + v * CO + c0);
+                dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            };
+            if constexpr (EPI == 2) {
+                // lanes 2K and 2K + 1 hold the two z of coarse cell K: the even one takes channels 0-7 of both, the odd
+                // one 8-15; the lower z of the four columns first, then the upper (held in up)
+                const bool odd = lane & 1;
 #pragma unroll 1
-            for (int tile = 0; tile < kTiles; tile++) {
-                const int yy = y0 + tile % Y, xx = x0 + tile / Y;
-                const int col = tile - tile % Y + Y - 1 - tile % Y;  // accumulators by descending y
-                const bool inb = z < d.nz && yy < d.ny && xx < d.nx;
-                const long long v = inb ? cid(d, xx, yy, z) : 0;
+                for (int yp = 0; yp < Y; yp += 2) {
 #pragma unroll
-                for (int c0 = 0; c0 < CO; c0 += 16) {
-                    float acc[16];
-                    tmem_ld_x16<16>(tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tb * L::kCols + col * CO + c0),
-                                    acc);
-                    if (inb && EPI == 0) {
-                        uint32_t pk[8];
+                    for (int c0 = 0; c0 < CO; c0 += 16) {
+                        float sum[8];
+                        uint32_t up[4][4];
 #pragma unroll
-                        for (int k = 0; k < 8; k++) {
-                            const float a0 = fmaxf(acc[2 * k] + bias[c0 + 2 * k], 0.f);
-                            const float a1 = fmaxf(acc[2 * k + 1] + bias[c0 + 2 * k + 1], 0.f);
-                            __nv_bfloat162 h2 = __floats2bfloat162_rn(a0, a1);
-                            pk[k] = *reinterpret_cast<uint32_t *>(&h2);
+                        for (int q = 0; q < 8; q++) sum[q] = 0.f;
+                        auto add = [&](const uint32_t(&w)[4]) {
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                sum[2 * q] += __uint_as_float(w[q] << 16);
+                                sum[2 * q + 1] += __uint_as_float(w[q] & 0xffff0000u);
+                            }
+                        };
+#pragma unroll
+                        for (int t = 0; t < 4; t++) {
+                            const int xx = t & 1, yy = yp + (t >> 1);
+                            uint32_t pk[8], lo[4];
+                            relu16(yy, xx, c0, pk);
+                            if (z < d.nz && y0 + yy < d.ny && x0 + xx < d.nx) {
+                                put16(cid(d, x0 + xx, y0 + yy, z), c0, pk);
+                            } else {  // absent
+#pragma unroll
+                                for (int q = 0; q < 8; q++) pk[q] = 0u;
+                            }
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? pk[q] : pk[4 + q], 1);
+                                lo[q] = odd ? got : pk[q];
+                                up[t][q] = odd ? pk[4 + q] : got;
+                            }
+                            add(lo);
                         }
-                        uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(yout) + v * CO + c0);
-                        dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                        dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                    } else if (inb) {
-                        float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(yout) + v * CO + c0);
 #pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            dst[k] = make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                        for (int t = 0; t < 4; t++) add(up[t]);
+                        const int I = x0 >> 1, J = (y0 + yp) >> 1, K = z >> 1;
+                        if (I < ep.dc.nx && J < ep.dc.ny && K < ep.dc.nz) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                __nv_bfloat162 h2 = __floats2bfloat162_rn(sum[2 * q] * 0.125f, sum[2 * q + 1] * 0.125f);
+                                w[q] = *reinterpret_cast<uint32_t *>(&h2);
+                            }
+                            *reinterpret_cast<uint4 *>(ep.pool + cid(ep.dc, I, J, K) * CO + c0 + (odd ? 8 : 0)) =
+                                make_uint4(w[0], w[1], w[2], w[3]);
+                        }
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int tile = 0; tile < kTiles; tile++) {
+                    const int yt = tile % Y, xt = tile / Y, yy = y0 + yt, xx = x0 + xt;
+                    const bool inb = z < d.nz && yy < d.ny && xx < d.nx;
+                    const long long v = inb ? cid(d, xx, yy, z) : 0;
+#pragma unroll
+                    for (int c0 = 0; c0 < CO; c0 += 16) {
+                        if constexpr (EPI == 1) {
+                            float acc[16];
+                            tmem_ld_x16<16>(tmem + ((uint32_t)(32 * q4) << 16) +
+                                                (uint32_t)(tb * L::kCols + (xt * Y + Y - 1 - yt) * CO + c0),
+                                            acc);
+                            if (!inb) continue;
+                            float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(yout) + v * CO + c0);
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                dst[k] = make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                        } else {
+                            uint32_t pk[8];
+                            relu16(yt, xt, c0, pk);
+                            if (!inb) continue;
+                            if constexpr (EPI == 3) {
+                                float s = hb;
+#pragma unroll
+                                for (int k = 0; k < 8; k++) {
+                                    s += hw[2 * k] * __uint_as_float(pk[k] << 16);
+                                    s += hw[2 * k + 1] * __uint_as_float(pk[k] & 0xffff0000u);
+                                }
+                                ep.out[v] = s;
+                            } else {
+                                put16(v, c0, pk);
+                            }
+                        }
                     }
                 }
             }

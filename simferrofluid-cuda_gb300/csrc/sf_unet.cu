@@ -138,7 +138,7 @@ long long line_bricks(const Dims &d, int y) {
 
 template <int CI, int CO, int EPI, int Y>
 cudaError_t launch_tc_line_y(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *wp, const float *b, void *y,
-                             int *err) {
+                             int *err, const tc::LineEpi &ep) {
     auto enc = tensor_map_encoder();
     if (!enc || !aligned16(x) || !aligned16(wp) || !aligned16(y)) return cudaErrorInvalidValue;
     CUtensorMap mx, mw;
@@ -164,7 +164,7 @@ cudaError_t launch_tc_line_y(cudaStream_t st, const Dims &d, const bf16 *x, cons
     if (e != cudaSuccess) return e;
     const long long nbricks = line_bricks(d, Y);
     const int grid = (int)(nbricks < 152 ? nbricks : 152);
-    tc::k_conv_tc_line<CI, CO, EPI, Y><<<grid, 192, L::kSmemBytes, st>>>(mx, mw, d, b, y, err);
+    tc::k_conv_tc_line<CI, CO, EPI, Y><<<grid, 192, L::kSmemBytes, st>>>(mx, mw, d, b, y, err, ep);
     return cudaGetLastError();
 }
 
@@ -172,14 +172,14 @@ cudaError_t launch_tc_line_y(cudaStream_t st, const Dims &d, const bf16 *x, cons
 // CTA's lines, bricks x (Y + 2), are fewer (256^3: 540 and 648; a ny of 12 has 20 and 18 a column)
 template <int CI, int CO, int EPI>
 cudaError_t launch_tc_line(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *wp, const float *b, void *y,
-                           int *err) {
+                           int *err, const tc::LineEpi &ep = {}) {
     constexpr int Y = tc::kLineY;
     if constexpr (CO == 16) {
         const long long lines = (line_bricks(d, Y) + 151) / 152 * (Y + 2),
                         lines2 = (line_bricks(d, 2 * Y) + 151) / 152 * (2 * Y + 2);
-        if (d.ny >= 2 * Y + 2 && lines2 < lines) return launch_tc_line_y<CI, CO, EPI, 2 * Y>(st, d, x, wp, b, y, err);
+        if (d.ny >= 2 * Y + 2 && lines2 < lines) return launch_tc_line_y<CI, CO, EPI, 2 * Y>(st, d, x, wp, b, y, err, ep);
     }
-    return launch_tc_line_y<CI, CO, EPI, Y>(st, d, x, wp, b, y, err);
+    return launch_tc_line_y<CI, CO, EPI, Y>(st, d, x, wp, b, y, err, ep);
 }
 
 // grids holding a 64 x 6 x 4 box: the 64-long z-line kernel (weights streamed per stage, taps ordered by z shift)
@@ -241,6 +241,15 @@ cudaError_t tc_dispatch(cudaStream_t st, int ci, int co, int epi, const Dims &d,
                         : launch_tc<A, B, 1>(st, d, x, w, wp, b, y, err);
     CASE(16, 16) CASE(16, 32) CASE(32, 16) CASE(32, 32) CASE(32, 64) CASE(64, 32) CASE(64, 64)
 #undef CASE
+    return cudaErrorInvalidValue;
+}
+
+// the z-line kernel with a fused epilogue; refused (as an unsupported shape) where the layer does not run on it
+cudaError_t line_fused(cudaStream_t st, int ci, int co, int epi, const Dims &d, const bf16 *x, const bf16 *wp,
+                       const float *b, void *y, int *err, const tc::LineEpi &ep) {
+    if (epi == 2 && ci == 16 && co == 16) return launch_tc_line<16, 16, 2>(st, d, x, wp, b, y, err, ep);
+    if (epi == 2 && ci == 32 && co == 32) return launch_tc_line<32, 32, 2>(st, d, x, wp, b, y, err, ep);
+    if (epi == 3 && ci == 16 && co == 16) return launch_tc_line<16, 16, 3>(st, d, x, wp, b, y, err, ep);
     return cudaErrorInvalidValue;
 }
 
@@ -516,6 +525,22 @@ void UNet::conv_fwd(const ConvLayer &L, const Dims &d, const bf16 *x, bf16 *y) {
     conv_dispatch(st_, L.cin, L.cout, 0, d, x, wb_ + L.wbf, p_ + L.boff, y, L.taps);
 }
 
+bool UNet::conv_fwd_fused(const ConvLayer &L, const Dims &d, const bf16 *x, bf16 *y, int epi, const Dims &dc, bf16 *pool,
+                          float *out) {
+    if (mode_ != 1 || L.taps != 27 || !line_shape_ok(L.cin, L.cout, d)) return false;
+    const ConvLayer &H = layers_.back();
+    const tc::LineEpi ep{pool, dc, p_ + H.woff, p_ + H.boff, out};
+    const cudaError_t e =
+        line_fused(st_, L.cin, L.cout, epi, d, x, wbp_ + L.wbf, p_ + L.boff, y, err_, ep);
+    if (e == cudaSuccess) {
+        tc_launches_++;
+        return true;
+    }
+    last_error = std::string("tcgen05 convolution not launched: ") + cudaGetErrorString(e);
+    cudaGetLastError();  // the separate kernels run instead: the refused launch is not an error
+    return false;
+}
+
 cudaError_t UNet::check_device_errors() {
     int h = 0;
     cudaError_t e = cudaMemcpyAsync(&h, err_, sizeof(int), cudaMemcpyDeviceToHost, st_);
@@ -538,11 +563,15 @@ cudaError_t UNet::forward(const Dims &d, const bf16 *feat, float *out, bool trai
     const ConvLayer *Ls = layers_.data();
     const Dims &d0 = dims_[0], &d1 = dims_[1], &d2 = dims_[2], &d3 = dims_[3];
     conv_fwd(Ls[0], d0, feat, A0a);
-    conv_fwd(Ls[1], d0, A0a, S0);
-    k_pool<16><<<line_grid(d1, 2), 256, 0, st_>>>(d0, d1, S0, P1);
+    if (!conv_fwd_fused(Ls[1], d0, A0a, S0, 2, d1, P1, nullptr)) {
+        conv_fwd(Ls[1], d0, A0a, S0);
+        k_pool<16><<<line_grid(d1, 2), 256, 0, st_>>>(d0, d1, S0, P1);
+    }
     conv_fwd(Ls[2], d1, P1, A1a);
-    conv_fwd(Ls[3], d1, A1a, S1);
-    k_pool<32><<<line_grid(d2, 4), 256, 0, st_>>>(d1, d2, S1, P2);
+    if (!conv_fwd_fused(Ls[3], d1, A1a, S1, 2, d2, P2, nullptr)) {
+        conv_fwd(Ls[3], d1, A1a, S1);
+        k_pool<32><<<line_grid(d2, 4), 256, 0, st_>>>(d1, d2, S1, P2);
+    }
     conv_fwd(Ls[4], d2, P2, A2a);
     conv_fwd(Ls[5], d2, A2a, S2);
     k_pool<64><<<line_grid(d3, 8), 256, 0, st_>>>(d2, d3, S2, P3);
@@ -556,6 +585,8 @@ cudaError_t UNet::forward(const Dims &d, const bf16 *feat, float *out, bool trai
     conv_fwd(Ls[11], d1, D1a, D1b);
     k_up_add<16><<<line_grid(d0, 2), 256, 0, st_>>>(d0, d1, D1b, S0, U0);
     conv_fwd(Ls[12], d0, U0, D0a);
+    // the backward pass reads the last activations: fused into their convolution in inference only
+    if (!training && conv_fwd_fused(Ls[13], d0, D0a, nullptr, 3, d0, nullptr, out)) return cudaGetLastError();
     conv_fwd(Ls[13], d0, D0a, D0b);
     const ConvLayer &H = Ls[14];
     k_head_fwd<<<flat_blocks(d0.n), 256, 0, st_>>>(d0.n, D0b, p_ + H.woff, p_ + H.boff, out ? out : out_);

@@ -66,6 +66,10 @@ class UNet {
     cudaError_t ensure(const Dims &d, bool training);
     cudaError_t ensure_wgrad_ws();
     void conv_fwd(const ConvLayer &L, const Dims &d, const __nv_bfloat16 *x, __nv_bfloat16 *y);
+    // conv_fwd with the pooling (epi 2: into pool, of extents dc) or the head (epi 3: into out, y not stored) in its
+    // epilogue; false, with nothing launched, where the layer does not run on the z-line kernel
+    bool conv_fwd_fused(const ConvLayer &L, const Dims &d, const __nv_bfloat16 *x, __nv_bfloat16 *y, int epi,
+                        const Dims &dc, __nv_bfloat16 *pool, float *out);
     void conv_bwd(const ConvLayer &L, const Dims &d, const __nv_bfloat16 *x, const __nv_bfloat16 *post,
                   const float *dpost, float *dx /* nullable */);
     void refresh_bf16();
