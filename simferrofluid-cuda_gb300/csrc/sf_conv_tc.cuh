@@ -314,6 +314,7 @@ struct LineLayout {
 // EPI 3 (Cout = 16): the 1x1 head applied to y, which is not stored.  256^3: pooling and head by themselves read the 537
 // MB again, 92 and 87 us; in these epilogues, which run beside the next brick's MMAs, the convolutions take 523 and 474
 // us (531 without either).
+// (The upsampling and skip sum in the epilogue of the layer before it: 280 us, 131 and 165 by themselves.)
 struct LineEpi {
     __nv_bfloat16 *pool;
     Dims dc;               // of the pooled grid
@@ -468,6 +469,9 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
         for (int bi = 0; bi < nb; bi++) {
             const int tb = bi & 1;
             const uint32_t par = (uint32_t)(bi >> 1) & 1u;
+            int z0, y0, x0;
+            brick(bi, z0, y0, x0);
+            const int z = z0 + 32 * q4 + lane;
             // lane 0 decides for the warp, so that the warp-collective TMEM loads below are never divergent
             int go = 0;
             if (lane == 0) go = (!sh[1] && mbar_wait(tfull0 + 8 * tb, par)) ? 1 : 0;
@@ -478,9 +482,6 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
             }
             mbar_wait(tfull0 + 8 * tb, par);  // completed: returns at once, with this thread's acquire
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            int z0, y0, x0;
-            brick(bi, z0, y0, x0);
-            const int z = z0 + 32 * q4 + lane;
             // 16 channels c0 .. of tile (yy, xx), after bias and ReLU, as BF16 pairs
             auto relu16 = [&](int yy, int xx, int c0, uint32_t(&pk)[8]) {
                 float acc[16];
@@ -868,15 +869,14 @@ struct WgLayout {
     static_assert(kStages >= 2 && kSmemBytes <= 227u * 1024u, "shared memory");
 };
 
-// dst[zh][x][y][s][c][zl] = src[x][y][8 zh + zl + s - (NS - 1) / 2][c] where 8 zh + zl < nz and the shifted z lies in
-// the grid, else 0; s < NS (1 or 3), zh < nzh = ceil(nz / 8).  A thread takes two channels of one (zh, x, y): each z is
+// dst[zh][x][y][s][c][zl] = src[x][y][8 zh + zl + s - 1][c] where 8 zh + zl < nz and the shifted z lies in
+// the grid, else 0; s < 3, zh < nzh = ceil(nz / 8).  A thread takes two channels of one (zh, x, y): each z is
 // read once, in 4-byte words, for all its shifts, and 32 bytes are stored per shift (a channel a thread and a read per
-// shift: 32 us for dY and 76 for X of 16 channels at 128^3, 23 and 56 now).
-template <int C, int NS>
+// shift: 76 us for 16 channels at 128^3, 56 now).
+template <int C>
 __global__ void __launch_bounds__(256) k_to_chmajor(Dims d, const __nv_bfloat16 *__restrict__ src,
                                                     __nv_bfloat16 *__restrict__ dst) {
-    static_assert(NS == 1 || NS == 3, "z shifts");
-    constexpr int P = C / 2;
+    constexpr int P = C / 2, NS = 3;
     const long long m = (long long)((d.nz + 7) / 8) * d.nx * d.ny * P;
     const uint32_t *s32 = reinterpret_cast<const uint32_t *>(src);
     for (long long e = blockIdx.x * 256LL + threadIdx.x; e < m; e += gridDim.x * 256LL) {
@@ -887,7 +887,7 @@ __global__ void __launch_bounds__(256) k_to_chmajor(Dims d, const __nv_bfloat16 
         uint32_t v[7 + NS];
 #pragma unroll
         for (int q = 0; q < 7 + NS; q++) {
-            const int z = 8 * zh + q - (NS - 1) / 2;
+            const int z = 8 * zh + q - 1;
             v[q] = z >= 0 && z < d.nz ? row[(long long)z * P] : 0u;
         }
         const int nv = d.nz - 8 * zh;  // voxels of this 8-voxel row inside the grid
@@ -904,6 +904,41 @@ __global__ void __launch_bounds__(256) k_to_chmajor(Dims d, const __nv_bfloat16 
             out[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             out[1] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         }
+    }
+}
+
+// dY = dpost (post > 0) as BF16 [voxel][C], and its channel-major copy [zh][x][y][c][zl], zero past nz, in one pass (37
+// and 23 us for 16 channels at 128^3 by themselves, 52 together).
+template <int C>
+__global__ void __launch_bounds__(256) k_relu_chmajor(Dims d, const float *__restrict__ dpost,
+                                                      const __nv_bfloat16 *__restrict__ post,
+                                                      __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ dyT) {
+    constexpr int P = C / 2;
+    const long long m = (long long)((d.nz + 7) / 8) * d.nx * d.ny * P;
+    for (long long e = blockIdx.x * 256LL + threadIdx.x; e < m; e += gridDim.x * 256LL) {
+        const int cp = (int)(e % P);
+        const unsigned r = (unsigned)(e / P), t = r / (unsigned)d.ny;  // r = (zh nx + x) ny + y
+        const int y = (int)(r - t * d.ny), zh = (int)(t / (unsigned)d.nx), x = (int)(t - (unsigned)zh * d.nx);
+        const long long row = (((long long)x * d.ny + y) * d.nz + 8 * zh) * P + cp;  // in channel pairs
+        const int nv = d.nz - 8 * zh;
+        uint32_t v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            v[q] = 0u;
+            if (q < nv) {
+                const float2 g = reinterpret_cast<const float2 *>(dpost)[row + q * P];
+                const uint32_t a = reinterpret_cast<const uint32_t *>(post)[row + q * P];
+                __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(a << 16) > 0.f ? g.x : 0.f,
+                                                          __uint_as_float(a & 0xffff0000u) > 0.f ? g.y : 0.f);
+                v[q] = *reinterpret_cast<uint32_t *>(&h2);
+                reinterpret_cast<uint32_t *>(dy)[row + q * P] = v[q];
+            }
+        }
+        uint4 *out = reinterpret_cast<uint4 *>(dyT) + (long long)r * C + 2 * cp;
+        out[0] = make_uint4(__byte_perm(v[0], v[1], 0x5410), __byte_perm(v[2], v[3], 0x5410),
+                            __byte_perm(v[4], v[5], 0x5410), __byte_perm(v[6], v[7], 0x5410));
+        out[1] = make_uint4(__byte_perm(v[0], v[1], 0x7632), __byte_perm(v[2], v[3], 0x7632),
+                            __byte_perm(v[4], v[5], 0x7632), __byte_perm(v[6], v[7], 0x7632));
     }
 }
 

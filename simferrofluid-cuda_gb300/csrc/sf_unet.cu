@@ -259,10 +259,10 @@ bool wgrad_tc_ok(int ci, int co, const Dims &d) {
     return ch && (d.nz + 7) / 8 >= 4 && d.ny >= 4 && d.nx >= 2;
 }
 
-// channel-major z-row copies of dY and of X with its three z shifts (k_to_chmajor), then k_wgrad_tc over all
-// bricks; chunks receives the number of partial sums written to part
+// the channel-major z-row copy of X with its three z shifts (k_to_chmajor; dY's is there, k_relu_chmajor), then k_wgrad_tc
+// over all bricks; chunks receives the number of partial sums written to part
 template <int CI, int CO, bool HALO>
-cudaError_t launch_wgrad_tc(cudaStream_t st, const Dims &d, const bf16 *dy, const bf16 *x, bf16 *dyT, bf16 *xT,
+cudaError_t launch_wgrad_tc(cudaStream_t st, const Dims &d, const bf16 *x, const bf16 *dyT, bf16 *xT,
                             float *part, long long part_cap, int &chunks, int *err) {
     auto enc = tensor_map_encoder();
     if (!enc || !aligned16(dyT) || !aligned16(xT) || !aligned16(part)) return cudaErrorInvalidValue;
@@ -296,19 +296,18 @@ cudaError_t launch_wgrad_tc(cudaStream_t st, const Dims &d, const bf16 *dy, cons
     if (G > nbricks) G = nbricks;
     if (G * 27 * CO * CI > part_cap) G = part_cap / (27LL * CO * CI);
     if (G < 1) return cudaErrorInvalidValue;
-    tc::k_to_chmajor<CO, 1><<<flat_blocks(rows * CO / 2), 256, 0, st>>>(d, dy, dyT);
-    tc::k_to_chmajor<CI, 3><<<flat_blocks(rows * CI / 2), 256, 0, st>>>(d, x, xT);
+    tc::k_to_chmajor<CI><<<flat_blocks(rows * CI / 2), 256, 0, st>>>(d, x, xT);
     tc::k_wgrad_tc<CI, CO, HALO><<<dim3((unsigned)G, groups), 128, L::kSmemBytes, st>>>(mdy, mx, d, part, err);
     chunks = (int)G;
     return cudaGetLastError();
 }
 
-cudaError_t wgrad_tc_dispatch(cudaStream_t st, int ci, int co, const Dims &d, const bf16 *dy, const bf16 *x,
-                              bf16 *dyT, bf16 *xT, float *part, long long part_cap, int &chunks, int *err) {
+cudaError_t wgrad_tc_dispatch(cudaStream_t st, int ci, int co, const Dims &d, const bf16 *x, const bf16 *dyT,
+                              bf16 *xT, float *part, long long part_cap, int &chunks, int *err) {
     const bool halo = d.ny >= 6 && d.nx >= 4;  // the halo'd box lies within the grid's extents, as every other box
 #define CASE(A, B, H)                                                                                     \
     if (ci == A && co == B && H == (A == 16 && halo))                                                     \
-        return launch_wgrad_tc<A, B, H>(st, d, dy, x, dyT, xT, part, part_cap, chunks, err);
+        return launch_wgrad_tc<A, B, H>(st, d, x, dyT, xT, part, part_cap, chunks, err);
     CASE(16, 16, true) CASE(16, 32, true) CASE(16, 16, false) CASE(16, 32, false) CASE(32, 16, false)
     CASE(32, 32, false) CASE(32, 64, false) CASE(64, 32, false) CASE(64, 64, false)
 #undef CASE
@@ -598,22 +597,29 @@ void UNet::conv_bwd(const ConvLayer &L, const Dims &d, const bf16 *x, const bf16
                     float *dx) {
     const long long m = d.n * L.cout;
     bf16 *dy = gbf[L.level];
-    k_relu_back<<<flat_blocks(m / 8), 256, 0, st_>>>(m / 8, dpost, post, dy);
     long long vchunk = (d.n + 63) / 64;
     if (vchunk < kVchunkMin) vchunk = kVchunkMin;
     const int chunks = (int)((d.n + vchunk - 1) / vchunk);
     int wchunks = 0;
-    if (mode_ >= 1 && L.taps == 27 && wgrad_tc_ok(L.cin, L.cout, d)) {
-        cudaError_t e = ensure_wgrad_ws();
-        if (e == cudaSuccess)
-            e = wgrad_tc_dispatch(st_, L.cin, L.cout, d, dy, x, wg_dy_, wg_x_, wpart_, wpart_elems_, wchunks, err_);
-        if (e == cudaSuccess)
-            tc_launches_++;
-        else {
-            wchunks = 0;
-            last_error = std::string("tcgen05 weight gradient not launched: ") + cudaGetErrorString(e);
-            cudaGetLastError();  // the warp-MMA kernel runs instead
-        }
+    const bool tc_shape = mode_ >= 1 && L.taps == 27 && wgrad_tc_ok(L.cin, L.cout, d);
+    cudaError_t e = tc_shape ? ensure_wgrad_ws() : cudaSuccess;
+    if (tc_shape && e == cudaSuccess) {
+        const int blocks = flat_blocks(m / 16);
+        if (L.cout == 16)
+            tc::k_relu_chmajor<16><<<blocks, 256, 0, st_>>>(d, dpost, post, dy, wg_dy_);
+        else if (L.cout == 32)
+            tc::k_relu_chmajor<32><<<blocks, 256, 0, st_>>>(d, dpost, post, dy, wg_dy_);
+        else
+            tc::k_relu_chmajor<64><<<blocks, 256, 0, st_>>>(d, dpost, post, dy, wg_dy_);
+        e = wgrad_tc_dispatch(st_, L.cin, L.cout, d, x, wg_dy_, wg_x_, wpart_, wpart_elems_, wchunks, err_);
+        if (e == cudaSuccess) tc_launches_++;
+    } else {
+        k_relu_back<<<flat_blocks(m / 8), 256, 0, st_>>>(m / 8, dpost, post, dy);
+    }
+    if (e != cudaSuccess) {
+        wchunks = 0;
+        last_error = std::string("tcgen05 weight gradient not launched: ") + cudaGetErrorString(e);
+        cudaGetLastError();  // the warp-MMA kernel runs instead
     }
     if (wchunks == 0) {
         wgrad_dispatch(st_, L.cin, L.cout, d, dy, x, wpart_, L.taps, (int)vchunk, chunks);
