@@ -282,8 +282,8 @@ __global__ void __launch_bounds__(128, 1) k_conv_tc(const __grid_constant__ CUte
 // and the accumulators stand by descending y, so one MMA of N = 3 Cout does the three: an M = 128 operand costs 4 KB of
 // shared memory reads whatever N is (64 clocks as measured), and those reads bound a tap at a time.  The order of an
 // accumulator's sums, (dz, channels, dx, dy), is the same.  16 to 16 channels at 256^3: 795 us a tap at a time, 626 with
-// three taps an MMA (boxes of four planes, two stages: copies and MMAs half overlapped), 519 with a plane a stage and Y = 8,
-// which reads 2.5 lines a voxel and z shift instead of 3.  What bounds it now is shared memory: a brick's 194 MMAs read
+// three taps an MMA (boxes of four planes, two stages: copies and MMAs half overlapped), 515 with a plane a stage and
+// Y = 8, which reads 2.5 lines a voxel and z shift instead of 3.  What bounds it now is shared memory: a brick's 194 MMAs read
 // 16 k clocks' worth at 64 bytes a clock, the copies write 3.8 k at 128, 19.9 k measured.
 // Warp 1 lane 0 issues the TMA loads through the stages, warp 0 lane 0 the MMAs (M = 128, N up to 3 Cout, K = 16) into
 // one of two TMEM accumulator sets, and warps 2-5 read the other set back (bias + ReLU + BF16, or FP32), so the epilogue
@@ -312,8 +312,8 @@ struct LineLayout {
 
 // EPI 2: as 0, and the 2x2x2 average pooling of y besides (a brick holds whole 2x2x2 cells; sums in k_pool's order).
 // EPI 3 (Cout = 16): the 1x1 head applied to y, which is not stored.  256^3: pooling and head by themselves read the 537
-// MB again, 92 and 87 us; in these epilogues, which run beside the next brick's MMAs, the convolutions take 523 and 474
-// us (531 without either).
+// MB again, 92 and 87 us; in these epilogues, which run beside the next brick's MMAs, the convolutions take 514 and 474
+// us (515 without either).
 // (The upsampling and skip sum in the epilogue of the layer before it: 280 us, 131 and 165 by themselves.)
 struct LineEpi {
     __nv_bfloat16 *pool;
@@ -466,6 +466,9 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
             for (int c = 0; c < 16; c++) hw[EPI == 3 ? c : 0] = ep.hw[c];
             hb = ep.hb[0];
         }
+        float bs[EPI == 1 ? 1 : CO];
+#pragma unroll
+        for (int c = 0; c < (EPI == 1 ? 0 : CO); c++) bs[c] = bias[c];
         for (int bi = 0; bi < nb; bi++) {
             const int tb = bi & 1;
             const uint32_t par = (uint32_t)(bi >> 1) & 1u;
@@ -490,8 +493,8 @@ __global__ void __launch_bounds__(192, 1) k_conv_tc_line(const __grid_constant__
                                 acc);  // accumulators by descending y
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
-                    const float a0 = fmaxf(acc[2 * k] + bias[c0 + 2 * k], 0.f);
-                    const float a1 = fmaxf(acc[2 * k + 1] + bias[c0 + 2 * k + 1], 0.f);
+                    const float a0 = fmaxf(acc[2 * k] + bs[EPI == 1 ? 0 : c0 + 2 * k], 0.f);
+                    const float a1 = fmaxf(acc[2 * k + 1] + bs[EPI == 1 ? 0 : c0 + 2 * k + 1], 0.f);
                     __nv_bfloat162 h2 = __floats2bfloat162_rn(a0, a1);
                     pk[k] = *reinterpret_cast<uint32_t *>(&h2);
                 }
