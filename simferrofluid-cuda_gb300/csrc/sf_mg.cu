@@ -1286,12 +1286,11 @@ __device__ __forceinline__ double from_fixed(long long t, int emax) {
 // partial sums at every step of the FP64 form.  Such a row (91% of the potential's) also reads no coefficient: 20 bytes
 // a cell instead of 60.  Two FP64 operations a cell remain (the product with c, the square).
 //
-// A block owns a 64 (z) x 8 (y) tile and marches along x, two cells of a row a thread; each value is converted once and
-// shared through two planes of shared memory, zero outside the grid.  209 us (200 without an output, 315 before), now
-// bound by the latency of a plane between its barriers: the FP64 pipe is 45% busy.  Every neighbour converted where it
-// is needed, without shared memory: 250 us; eight planes an item: 194 us, but the pressure's uneven rows then take 204
-// instead of 140; values loaded a plane ahead: 286 us (92 registers, two blocks an SM).
-constexpr int kResPlanes = 4;  // x planes of a block's item
+// A block owns a 64 (z) x 8 (y) tile and marches along x (`planes` of them an item), two cells of a row a thread; each
+// value is converted once and shared through two planes of shared memory, zero outside the grid.  189 us (184 without an
+// output, 315 before), now bound by the latency of a plane between its barriers: the FP64 pipe is 55% busy, the integer
+// pipe 50%.  Every neighbour converted where it is needed, without shared memory: 250 us; values loaded a plane ahead:
+// 286 us (92 registers, two blocks an SM).
 // b - A x of one cell in FP64; a call, so that its registers are not the common rows'.
 __device__ __noinline__ double residual_cell(const Dims &d, const Coef<double> &cf, const double *x, double bc, int i,
                                              int j, int k) {
@@ -1308,7 +1307,7 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
                                                        const unsigned *__restrict__ xmax,
                                                        const double *__restrict__ x, const double *__restrict__ b,
                                                        TR *__restrict__ r, int skip0, int rr_slot, int bb_slot,
-                                                       double *sc, double *part, unsigned *ticket) {
+                                                       double *sc, double *part, unsigned *ticket, int planes) {
     // [row + 1][cell + 2]: one row of halo in y, one cell (at 1 and 66) in z
     __shared__ __align__(16) long long plane[2][10][68];
     double v[2] = {0, 0};
@@ -1321,14 +1320,14 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
     const bool pair = tid < 64;
     const int hy = tid < 32 ? 0 : (pair ? 9 : 1 + ((tid - 64) & 7)), hz = pair ? 2 + 2 * (tid & 31) : (tid < 72 ? 1 : 66);
     const unsigned tz_n = (d.nz + 63) / 64, ty_n = (d.ny + 7) / 8;
-    const unsigned items = tz_n * ty_n * ((d.nx + kResPlanes - 1) / kResPlanes);
+    const unsigned items = tz_n * ty_n * ((d.nx + planes - 1) / planes);
     for (unsigned w = blockIdx.x; w < items; w += gridDim.x) {
         const unsigned tzi = w % tz_n, rest = w / tz_n, tyi = rest % ty_n, chunk = rest / ty_n;
         const int k = (int)tzi * 64 + 2 * tx, j = (int)tyi * 8 + ty;
         const int jh = (int)tyi * 8 + hy - 1, kh = (int)tzi * 64 + hz - 2;
         const bool in = k < d.nz && j < d.ny;  // nz is even: both cells or none
         const bool halo = tid < 80 && jh >= 0 && jh < d.ny && kh >= 0 && kh < d.nz;
-        const int i0 = (int)chunk * kResPlanes, i_end = min(d.nx, i0 + kResPlanes);
+        const int i0 = (int)chunk * planes, i_end = min(d.nx, i0 + planes);
         bool any = false;
         if (tx < i_end - i0 && j < d.ny) any = rows[(i0 + tx) * d.ny + j] != 0;
         const int m0 = in ? (i0 * d.ny + j) * nh + (k >> 1) : 0;  // split index of the pair, plane i0
@@ -2237,7 +2236,8 @@ void MGSolver::plan_tail() {
     }
 }
 
-const SplitOut *MGSolver::split_targets() {
+const SplitOut *MGSolver::split_targets(bool dense) {
+    dense_ = dense;
     if (!split0_) return nullptr;
     so_.c32 = c32_;
     so_.c16 = c16s0_;
@@ -2830,12 +2830,14 @@ void MGSolver::residual_split(TR *r, bool skip0, int rr_slot, int bb_slot) {
         xmax_ok_ = true;
         tk_.launches++;
     }
-    const long long items =
-        (long long)((d.nz + 63) / 64) * ((d.ny + 7) / 8) * ((d.nx + kResPlanes - 1) / kResPlanes);
+    // planes an item: eight where every row has work (256^3 potential: 189 us against 205 with four); the pressure's
+    // active rows then fall unevenly to the blocks (199 us against 134)
+    const int planes = dense_ ? 8 : 4;
+    const long long items = (long long)((d.nz + 63) / 64) * ((d.ny + 7) / 8) * ((d.nx + planes - 1) / planes);
     auto go = [&](auto kernel) {
         const int grid = (int)std::min<long long>(items, std::min(resident_grid((const void *)kernel), kMaxRedGrid));
         kernel<<<grid, dim3(32, 8), 0, st_>>>(d, c64_[0], rows_[0], other_[0], other_[1], xmax_, x_, b_, r,
-                                              skip0 ? 1 : 0, rr_slot, bb_slot, sc_, part_, ticket_);
+                                              skip0 ? 1 : 0, rr_slot, bb_slot, sc_, part_, ticket_, planes);
     };
     if (bb_slot >= 0)
         go(k_residual_rows<TR, true>);
