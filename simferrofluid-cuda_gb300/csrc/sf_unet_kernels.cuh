@@ -149,17 +149,24 @@ __global__ void __launch_bounds__(128) k_conv_mma(Dims d, const bf16 *__restrict
 // --------------------------------------------------------------------------------------------------------
 // Weight gradient, partial over a voxel chunk: part[chunk][t][co][ci] = sum_{v in chunk} dy[v][co] x[v+off_t][ci]
 // Block: 4 warps, one tap (blockIdx.y), one chunk of `vchunk` voxels (blockIdx.x).  M = co (m16 tiles), N = ci,
-// K = voxels; warps split the m tiles and, when CO < 64, the voxels.
+// K = voxels; warps split the m tiles and, when CO < 64, the voxels.  Tiles of 128 voxels are staged in shared memory by
+// 16-byte loads and read as transposed fragments; the voxels' neighbours are found once a tile.  With each fragment
+// gathered by 2-byte loads, 64 x 64 channels at 16^3 took 422 us, 45 with the neighbours once a tile, 20 so.
 // --------------------------------------------------------------------------------------------------------
 template <int CI, int CO>
 __global__ void __launch_bounds__(128) k_wgrad_mma(Dims d, const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
                                                    float *__restrict__ part, int taps, int vchunk) {
-    constexpr int MT = CO / 16 > 0 ? CO / 16 : 1;  // m16 tiles (CO = 8 uses one padded tile)
-    constexpr int WPM = 4 / (MT > 4 ? 4 : MT);    // warps per m tile
-    static_assert(MT <= 4, "CO <= 64");
-    __shared__ float red[4][CO > 16 ? 16 : CO][CI];
-    constexpr int kTile = 512;
-    __shared__ int nb[kTile];  // index of voxel + offset, -1 outside, of a tile of the chunk
+    constexpr int MT = CO / 16;                   // m16 tiles
+    constexpr int WPM = 4 / MT;                   // warps per m tile
+    static_assert(CO % 16 == 0 && MT <= 4 && CI % 16 == 0, "channel counts");
+    // rows of the two operands of a tile of voxels, 16 bytes of padding each (the fragments' loads are then without bank
+    // conflicts); afterwards the warps' sums
+    constexpr int kTile = 128, LX = CI + 8, LY = CO + 8;
+    constexpr int kRows = kTile * (LX + LY) * 2, kRed = 4 * 16 * CI * 4;
+    __shared__ __align__(16) unsigned char buf[kRows > kRed ? kRows : kRed];
+    bf16 *sx = reinterpret_cast<bf16 *>(buf), *sy = sx + kTile * LX;
+    float(*red)[16][CI] = reinterpret_cast<float(*)[16][CI]>(buf);
+    __shared__ int nb[kTile];  // index of voxel + offset, -1 outside
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, tq = lane & 3;
     const int mt = warp % MT, ks = warp / MT;
@@ -173,46 +180,69 @@ __global__ void __launch_bounds__(128) k_wgrad_mma(Dims d, const bf16 *__restric
     for (int n = 0; n < CI / 8; n++)
 #pragma unroll
         for (int q = 0; q < 4; q++) acc[n][q] = 0.f;
-    const int co_a = mt * 16 + g, co_b = co_a + 8;
-    const bool oka = co_a < CO, okb = co_b < CO;
-    auto xs = [&](int at, int ci) -> bf16 {  // x[v + off_t][ci], 0 outside
-        return at >= 0 ? x[(long long)at * CI + ci] : __float2bfloat16(0.f);
+    // this lane's row of the four 8 x 8 matrices of a transposing load: A (k, m) as k 0-7 | 8-15 of m 0-7 and 8-15, B
+    // (k, n) as k 0-7 and 8-15 of two n tiles
+    const int mat = lane >> 3, r8 = lane & 7;
+    const uint32_t a_at = (uint32_t)__cvta_generic_to_shared(sy + (((mat >> 1) * 8 + r8) * LY + mt * 16 + (mat & 1) * 8));
+    const uint32_t b_at = (uint32_t)__cvta_generic_to_shared(sx + (((mat & 1) * 8 + r8) * LX + (mat >> 1) * 8));
+    const bool wide = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    auto load_t = [](uint32_t at, uint32_t(&v)[4]) {
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                     : "r"(at)
+                     : "memory");
     };
-    auto dys = [&](long long v, int co, bool okc) -> bf16 {
-        return (okc && v < v_end) ? dy[v * CO + co] : __float2bfloat16(0.f);
-    };
-    // the neighbours' indices once per tile, by the whole block: formed where they are used (twelve 64-bit divisions a
-    // step of 16 voxels) they were most of the kernel, 422 us for 64 x 64 channels at 16^3
     for (long long tile = v_begin; tile < v_end; tile += kTile) {
-    __syncthreads();
-    for (int q = threadIdx.x; q < kTile; q += 128) {
-        const long long v = tile + q;
-        int at = -1;
-        if (v < v_end) {
-            const int vi = (int)v, row = vi / d.nz, kk = vi - row * d.nz + dz, i = row / d.ny, jj = row - i * d.ny + dy_,
-                      ii = i + dx;
-            if (ii >= 0 && ii < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz) at = (int)cid(d, ii, jj, kk);
+        __syncthreads();
+        {
+            const long long v = tile + threadIdx.x;
+            int at = -1;
+            if (v < v_end) {
+                const int vi = (int)v, row = vi / d.nz, kk = vi - row * d.nz + dz, i = row / d.ny,
+                          jj = row - i * d.ny + dy_, ii = i + dx;
+                if (ii >= 0 && ii < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz) at = (int)cid(d, ii, jj, kk);
+            }
+            nb[threadIdx.x] = at;
         }
-        nb[q] = at;
-    }
-    __syncthreads();
-    const long long tile_end = min(tile + kTile, v_end);
-    for (long long v0 = tile + 16LL * ks; v0 < tile_end; v0 += 16LL * WPM) {
-        const long long va = v0 + 2 * tq, vb = va + 8;
-        const int q0 = (int)(va - tile), na0 = nb[q0], na1 = nb[q0 + 1], nb0 = nb[q0 + 8], nb1 = nb[q0 + 9];
-        uint32_t a[4];
-        a[0] = pack_raw(dys(va, co_a, oka), dys(va + 1, co_a, oka));
-        a[1] = pack_raw(dys(va, co_b, okb), dys(va + 1, co_b, okb));
-        a[2] = pack_raw(dys(vb, co_a, oka), dys(vb + 1, co_a, oka));
-        a[3] = pack_raw(dys(vb, co_b, okb), dys(vb + 1, co_b, okb));
+        __syncthreads();
 #pragma unroll
-        for (int n = 0; n < CI / 8; n++) {
-            const int ci = n * 8 + g;
-            const uint32_t b[2] = {pack_raw(xs(na0, ci), xs(na1, ci)), pack_raw(xs(nb0, ci), xs(nb1, ci))};
-            mma16816(acc[n], a, b);
+        for (int e = threadIdx.x; e < kTile * CI / 8; e += 128) {
+            const int r = e / (CI / 8), q = e % (CI / 8), at = nb[r];
+            uint4 u = make_uint4(0u, 0u, 0u, 0u);
+            if (at >= 0) {
+                const bf16 *src = x + (long long)at * CI + 8 * q;
+                if (wide) {
+                    u = *reinterpret_cast<const uint4 *>(src);
+                } else {  // the caller's features may stand on any 4-byte boundary
+                    const uint32_t *w = reinterpret_cast<const uint32_t *>(src);
+                    u = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+            *reinterpret_cast<uint4 *>(sx + r * LX + 8 * q) = u;
+        }
+#pragma unroll
+        for (int e = threadIdx.x; e < kTile * CO / 8; e += 128) {
+            const int r = e / (CO / 8), q = e % (CO / 8);
+            *reinterpret_cast<uint4 *>(sy + r * LY + 8 * q) =
+                tile + r < v_end ? *reinterpret_cast<const uint4 *>(dy + (tile + r) * CO + 8 * q)
+                                 : make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        const int steps = (int)((min(tile + kTile, v_end) - tile + 15) / 16);
+        for (int k = ks; k < steps; k += WPM) {
+            uint32_t a[4];
+            load_t(a_at + (uint32_t)(16 * k * LY * 2), a);
+#pragma unroll
+            for (int n = 0; n < CI / 8; n += 2) {
+                uint32_t b[4];
+                load_t(b_at + (uint32_t)((16 * k * LX + 8 * n) * 2), b);
+                const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+                mma16816(acc[n], a, b0);
+                mma16816(acc[n + 1], a, b1);
+            }
         }
     }
-    }
+    __syncthreads();
     // reduce the WPM warps of each m tile through shared memory (fixed order)
     for (int s = 0; s < WPM; s++) {
         if (ks == s) {
