@@ -344,11 +344,13 @@ __global__ void __launch_bounds__(256) k_magnetic_rows(Dims d, Faces hext, doubl
         n += in[o] ? 1 : 0;
     }
     if (so.rows) {
-        // a warp is part of one row; every writer stores 1
-        const unsigned here = __activemask();
+        // A warp is part of one row, and its lanes with k < nz, the first one among them, all come here.  The vote names
+        // them: the lanes that happen to be converged might leave out the first one, which stores for all.
+        const int left = d.nz - (int)(blockIdx.x * blockDim.x);
+        const unsigned here = left >= 32 ? 0xffffffffu : (1u << left) - 1u;
         const bool some_air = __any_sync(here, !air), some_liq = __any_sync(here, !liq);
-        if ((threadIdx.x & 31) == 0 && some_air) so.other[0][row] = 1;
-        if ((threadIdx.x & 31) == 0 && some_liq) so.other[1][row] = 1;
+        if (threadIdx.x == 0 && some_air) so.other[0][row] = 1;  // every writer stores 1
+        if (threadIdx.x == 0 && some_liq) so.other[1][row] = 1;
     }
     double diag, inv, rhs = 0.;
     if (air) {
