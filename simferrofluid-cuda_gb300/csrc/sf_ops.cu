@@ -399,17 +399,20 @@ __global__ void __launch_bounds__(256) k_magnetic_rows(Dims d, Faces hext, doubl
 // x, y and z faces of cell (i, j, k), in one launch over (nx + 1) x (ny + 1) x (nz + 1) points, so psi of the cell
 // is loaded once for its three faces.
 // The FP64 pipe bounds it: three operations a face took 307 us at 256^3, where the bytes take 139.  Two remain: the
-// product with 1 / h runs on the integer pipe, or, where 1 / h is a power of two (POW2) and the product exact, joins the
-// sum as a fused multiply-add, which then rounds once as the sum does: 198 us.
+// product with 1 / h runs on the integer pipe, or, where 1 / h is a power of two and the product exact, joins the sum as a
+// fused multiply-add, which then rounds once as the sum does: 198 us.  Both want a normal product: differences outside
+// [2^-500, 2^500), and every difference where 1 / h lies outside [2^-400, 2^399), are multiplied as they stand.
+enum FieldForm { kFieldPlain, kFieldInt, kFieldFused };
 __device__ __noinline__ double mul_plain(double a, double b) { return a * b; }
-template <bool POW2>
+template <FieldForm FORM>
 __device__ __forceinline__ double field_face(double p0, double p1, double invh, double h) {
     const double diff = p0 - p1;
-    if (POW2 && f64_in_range(diff, -500, 500)) return __fma_rn(diff, invh, h);
-    return (f64_in_range(diff, -500, 500) ? f64_mul<true, false>(diff, invh) : mul_plain(diff, invh)) + h;
+    if (FORM == kFieldPlain || !f64_in_range(diff, -500, 500)) return mul_plain(diff, invh) + h;
+    if (FORM == kFieldFused) return __fma_rn(diff, invh, h);
+    return f64_mul<true, false>(diff, invh) + h;
 }
 
-template <bool POW2>
+template <FieldForm FORM>
 __global__ void __launch_bounds__(256) k_total_field3(Dims d, const double *__restrict__ psi, Faces hext, double invh,
                                                       Faces H) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(256) k_total_field3(Dims d, const double *__re
     for (int a = 0; a < 3; a++) {
         if (!on[a]) continue;
         // 0 + Hext on the boundary: Hext, with -0 as +0
-        const double v = in[a] ? field_face<POW2>(p0[a], p1, invh, h[a]) : (is_zero(h[a]) ? 0. : h[a]);
+        const double v = in[a] ? field_face<FORM>(p0[a], p1, invh, h[a]) : (is_zero(h[a]) ? 0. : h[a]);
         const_cast<double *>(H.p[a])[fid(d, a, i, j, k)] = v;
     }
 }
@@ -623,11 +626,14 @@ cudaError_t launch_magnetic_residual_noalloc(cudaStream_t st, const Dims &d, con
 void launch_total_field(cudaStream_t st, const Dims &d, const double *psi, const Faces &hext, double invh,
                         const Faces &H) {
     int e = 0;
-    const bool pow2 = std::frexp(invh, &e) == 0.5 && e > -400 && e < 400;
-    if (pow2)
-        k_total_field3<true><<<grid3(d.nx + 1, d.ny + 1, d.nz + 1), blk2(), 0, st>>>(d, psi, hext, invh, H);
+    const bool power = std::frexp(invh, &e) == 0.5, inside = std::isnormal(invh) && e > -400 && e < 400;
+    const dim3 g = grid3(d.nx + 1, d.ny + 1, d.nz + 1);
+    if (!inside)
+        k_total_field3<kFieldPlain><<<g, blk2(), 0, st>>>(d, psi, hext, invh, H);
+    else if (power)
+        k_total_field3<kFieldFused><<<g, blk2(), 0, st>>>(d, psi, hext, invh, H);
     else
-        k_total_field3<false><<<grid3(d.nx + 1, d.ny + 1, d.nz + 1), blk2(), 0, st>>>(d, psi, hext, invh, H);
+        k_total_field3<kFieldInt><<<g, blk2(), 0, st>>>(d, psi, hext, invh, H);
 }
 
 __global__ void k_to_f32(long long n, const double *__restrict__ a, float *__restrict__ o) {
