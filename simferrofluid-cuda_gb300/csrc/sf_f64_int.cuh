@@ -41,6 +41,13 @@ SF_CONV_FN double f64_fma(double a, double b, double c) { return __fma_rn(a, b, 
 SF_CONV_FN uint32_t mulhi_u32(uint32_t a, uint32_t b) { return __umulhi(a, b); }
 SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) { return __funnelshift_l(lo, hi, n); }
 SF_CONV_FN uint32_t shf_r(uint32_t lo, uint32_t hi, int n) { return __funnelshift_r(lo, hi, n); }
+SF_CONV_FN int clz_u64(uint64_t v) { return __clzll((long long)v); }
+// v >> n of a signed integer, n >= 0 of any size (PTX clamps the amount; in C++ 64 and more are undefined)
+SF_CONV_FN int64_t shr_s64(int64_t v, int n) {
+    int64_t r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
 #else
 #if defined(SF_F64_TEST_RCP)
 // a test's own approximations, off by as much as the device's may be
@@ -62,6 +69,8 @@ SF_CONV_FN uint32_t shf_l(uint32_t lo, uint32_t hi, int n) {
     return (uint32_t)(((((uint64_t)hi << 32) | lo) << n) >> 32);
 }
 SF_CONV_FN uint32_t shf_r(uint32_t lo, uint32_t hi, int n) { return (uint32_t)((((uint64_t)hi << 32) | lo) >> n); }
+SF_CONV_FN int clz_u64(uint64_t v) { return v ? __builtin_clzll(v) : 64; }
+SF_CONV_FN int64_t shr_s64(int64_t v, int n) { return v >> (n < 63 ? n : 63); }
 #endif
 
 constexpr uint32_t kF64Exp = 0x7ff00000u, kF64Frac = 0xfffffu, kF64One = 0x100000u, kF64Sign = 0x80000000u;
@@ -337,5 +346,52 @@ SF_CONV_FN double f64_sqrt_any(double a) {
     return !f64_lt0(a) && f64_in_range(a, -1000, 1000) && !f64_is_zero(a) ? f64_sqrt(a) : std::sqrt(a);
 }
 SF_CONV_FN double f64_third_any(double a) { return f64_in_range(a, -1000, 1000) ? f64_third(a) : a / 3; }
+
+// A double as its significand times 2^6, with the sign, and its exponent field: v = m 2^(e - 1081), |m| < 2^59 (a zero or a
+// subnormal number, of field 0, comes out as one near 2^-1023).
+struct F64Fixed {
+    int64_t m;
+    int e;
+};
+SF_CONV_FN F64Fixed f64_fixed(double v) {
+    uint32_t h, l;
+    f64_words(v, h, l);
+    const int64_t t = (int64_t)(((uint64_t)shf_l(l, (h & kF64Frac) | kF64One, 6) << 32) | (l << 6));
+    return F64Fixed{(int)h < 0 ? -t : t, (int)((h >> 20) & 0x7ffu)};
+}
+// In units of 2^(e - 1081), towards minus infinity; e at least the value's own field.
+SF_CONV_FN int64_t fixed_at(const F64Fixed &v, int e) { return shr_s64(v.m, e - v.e); }
+
+// t 2^(e - 1081), rounded to nearest even, |t| < 2^63 (the conversion instruction takes the FP64 pipe twice).
+SF_CONV_FN double fixed_to_f64(int64_t t, int e) {
+    const uint64_t m = t < 0 ? 0ull - (uint64_t)t : (uint64_t)t;
+    const int z = clz_u64(m);          // >= 1
+    const uint64_t a = m << (z & 63);  // 64-bit significand, the top bit set
+    // the 53 kept bits and the exponent field of 2^(e - 1081) 2^(63 - z), less the implicit bit, rounded by adding just
+    // under a half of the eleven dropped bits and the kept part's parity
+    const uint64_t kept = (a >> 11) + ((uint64_t)(uint32_t)(e + 4 - z) << 52);
+    const uint64_t up = ((a & 0x7ffull) + 0x3ffull + ((a >> 11) & 1ull)) >> 11;
+    const uint64_t bits = (kept + up) | ((uint64_t)t & 0x8000000000000000ull);
+    return m == 0 ? 0. : f64_from_words((uint32_t)(bits >> 32), (uint32_t)bits);
+}
+
+// s = n x - (a + b + c + d + e + f), n <= 6, in 64-bit integers of one unit, 2^-58 of the largest magnitude M among the seven:
+// what is lost is less than a unit a value, 6 2^-58 M in all, and the last rounding, against a rounding of up to
+// 2^-53 of the partial sum at each of seven FP64 operations.  The unit is this sum's own, so that holds wherever
+// the seven stand in a field of any range.  False (s unset) where M is below 2^-823, infinite or NaN.
+SF_CONV_FN bool fixed_stencil(int n, const F64Fixed &x, const F64Fixed &a, const F64Fixed &b, const F64Fixed &c,
+                              const F64Fixed &d, const F64Fixed &e, const F64Fixed &f, double &s) {
+    int top = x.e > a.e ? x.e : a.e;
+    top = top > b.e ? top : b.e;
+    top = top > c.e ? top : c.e;
+    top = top > d.e ? top : d.e;
+    top = top > e.e ? top : e.e;
+    top = top > f.e ? top : f.e;
+    if (top < 200 || top > 2040) return false;
+    s = fixed_to_f64(fixed_at(x, top) * n - (fixed_at(a, top) + fixed_at(b, top) + fixed_at(c, top) + fixed_at(d, top) +
+                                             fixed_at(e, top) + fixed_at(f, top)),
+                     top);
+    return true;
+}
 
 }  // namespace sf

@@ -59,8 +59,9 @@ __host__ __device__ __forceinline__ long long split_index(const Dims &d, int i, 
 
 // Where the assembly kernels also write the split level 0's FP32 and FP16 operator copies and its row flags
 // (1 on a row with an active cell; cleared by the launcher first).  rows == nullptr: not written.
-// other[q][row] (cleared by the launcher first) is set by any cell of the row whose FP64 operator is not exactly that of
-// kind q: in-grid couplings all one value and D their sum -- kind 0 the value 1, kind 1 the potential's 1 + chi.  A row
+// other[q][row] (the potential's assembly only; cleared by the launcher first) is set by any cell of the row whose FP64
+// operator is not exactly that of kind q: in-grid couplings all one value and D their sum -- kind 0 the value 1, kind 1 the
+// liquid's 1 + chi.  A row
 // without the mark of one kind has one coupling throughout (stored, for instance, at its second cell's lower z face).
 struct SplitOut {
     Coef<float> c32;

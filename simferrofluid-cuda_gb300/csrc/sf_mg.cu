@@ -27,6 +27,7 @@
 #include <tuple>
 #include <type_traits>
 
+#include "sf_f64_int.cuh"
 #include "sf_rbgs_tma.cuh"
 #include "sf_solver.h"
 
@@ -1254,43 +1255,21 @@ __global__ void __launch_bounds__(256) k_residual64(Dims d, int xpb, Coef<double
     }
 }
 
-// An integer multiple of 2^(emax - 1081) next to v towards zero, |v| < 2^(emax - 1022): the significand moved to the
-// place that its exponent has below the field's largest, emax.
-__device__ __forceinline__ long long to_fixed(double v, int emax) {
-    uint32_t h, l;
-    f64_words(v, h, l);
-    const uint32_t m = (h & 0xfffffu) | 0x100000u;
-    const unsigned long long t = ((unsigned long long)__funnelshift_l(l, m, 6) << 32) | (l << 6);
-    const long long s = (long long)(t >> min((unsigned)(emax - (int)((h >> 20) & 0x7ffu)), 63u));
-    return (int)h < 0 ? -s : s;
-}
-// t * 2^(emax - 1081), rounded to nearest even, |t| < 2^63 (the conversion instruction takes the FP64 pipe twice).
-__device__ __forceinline__ double from_fixed(long long t, int emax) {
-    const unsigned long long m = t < 0 ? 0ull - (unsigned long long)t : (unsigned long long)t;
-    const int z = __clzll((long long)m);  // >= 1
-    const unsigned long long a = m << z;  // 64-bit significand, the top bit set
-    // the 53 kept bits and the exponent field of 2^(emax - 1081) * 2^(63 - z), less the implicit bit, rounded by adding
-    // just under a half of the eleven dropped bits and the kept part's parity
-    const unsigned long long kept = (a >> 11) + ((unsigned long long)(unsigned)(emax + 4 - z) << 52);
-    const unsigned long long up = ((a & 0x7ffull) + 0x3ffull + ((a >> 11) & 1ull)) >> 11;
-    const unsigned long long bits = kept + up;
-    return m == 0 ? 0. : __longlong_as_double((long long)(bits | ((unsigned long long)t & 0x8000000000000000ull)));
-}
-
-// k_residual64 for the split form: rows of one exact coupling c (SplitOut::other) as r = b - c sum (x - x_neighbour),
-// the sum in 64-bit integers.
+// k_residual64 for the potential in the split form: rows of one exact coupling c (SplitOut::other) as
+// r = b - c sum (x - x_neighbour), the sum in 64-bit integers (fixed_stencil).
 //
-// The seven-point sum in FP64 arithmetic bound this kernel (nine operations and a conversion a cell: 359 us at 256^3
-// for the potential, 87% of the FP64 pipe).  x as an integer multiple of a power of two, 2^59 at the field's largest
-// magnitude, sums exactly: what is lost is what lies below 2^-58 of the largest |x|, once per value, against 2^-53 of the
-// partial sums at every step of the FP64 form.  Such a row (91% of the potential's) also reads no coefficient: 20 bytes
-// a cell instead of 60.  Two FP64 operations a cell remain (the product with c, the square).
+// The seven-point sum in FP64 arithmetic bounds k_residual64 (nine operations and a conversion a cell: 348 us at 256^3, 306
+// without an output, 87% of the FP64 pipe).  Such a row (91% of the potential's) also reads no coefficient: 20 bytes a
+// cell instead of 60.  Two FP64 operations a cell remain (the product with c, the square).
 //
-// A block owns a 64 (z) x 8 (y) tile and marches along x (`planes` of them an item), two cells of a row a thread; each
-// value is converted once and shared through two planes of shared memory, zero outside the grid.  189 us (184 without an
-// output, 315 before), now bound by the latency of a plane between its barriers: the FP64 pipe is 55% busy, the integer
-// pipe 50%.  Every neighbour converted where it is needed, without shared memory: 250 us; values loaded a plane ahead:
-// 286 us (92 registers, two blocks an SM).
+// A block owns a 64 (z) x 8 (y) tile and marches along x, kResidPlanes an item, two cells of a row a thread; each value is
+// taken apart once (f64_fixed) and shared through two planes of shared memory, zero outside the grid; a cell's sum is
+// formed in the unit of its own seven values.  234 us (225 without an output), bound by the latency of a plane between its
+// barriers and the integer pipe; 244 us with five blocks an SM (48 registers, spilled).  One unit for the whole field takes
+// 189 us, but parts of a field far below its largest value lose bits; one for an item, with the cells below an eighth of it
+// left to FP64, 275 us.  The pressure, whose rows mostly lie across the surface or outside the liquid, takes 162 us here and
+// 147 by k_residual64, which it keeps.
+constexpr int kResidPlanes = 8;
 // b - A x of one cell in FP64; a call, so that its registers are not the common rows'.
 __device__ __noinline__ double residual_cell(const Dims &d, const Coef<double> &cf, const double *x, double bc, int i,
                                              int j, int k) {
@@ -1301,59 +1280,47 @@ __device__ __noinline__ double residual_cell(const Dims &d, const Coef<double> &
 }
 
 template <class TR, bool BB>
-__global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> cf, const uint8_t *__restrict__ rows,
+__global__ void __launch_bounds__(256, 4) k_residual_rows(Dims d, Coef<double> cf,
                                                        const uint8_t *__restrict__ other0,
                                                        const uint8_t *__restrict__ other1,
-                                                       const unsigned *__restrict__ xmax,
                                                        const double *__restrict__ x, const double *__restrict__ b,
                                                        TR *__restrict__ r, int skip0, int rr_slot, int bb_slot,
-                                                       double *sc, double *part, unsigned *ticket, int planes) {
+                                                       double *sc, double *part, unsigned *ticket) {
     // [row + 1][cell + 2]: one row of halo in y, one cell (at 1 and 66) in z
-    __shared__ __align__(16) long long plane[2][10][68];
+    __shared__ __align__(16) int64_t plane[2][10][68];
+    __shared__ __align__(8) int expo[2][10][68];
     double v[2] = {0, 0};
     const int sx = d.ny * d.nz, nh = d.nz >> 1;
     const long long hn = d.n >> 1;
-    const int emax = (int)(*xmax >> 20);
-    const bool scaled = emax >= 200 && emax <= 2000;  // else x is zero, tiny or not finite: the FP64 form
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     // halo of this thread: tids 0..63 a pair of the row below or above, 64..79 one cell beside
     const bool pair = tid < 64;
     const int hy = tid < 32 ? 0 : (pair ? 9 : 1 + ((tid - 64) & 7)), hz = pair ? 2 + 2 * (tid & 31) : (tid < 72 ? 1 : 66);
     const unsigned tz_n = (d.nz + 63) / 64, ty_n = (d.ny + 7) / 8;
-    const unsigned items = tz_n * ty_n * ((d.nx + planes - 1) / planes);
+    const unsigned items = tz_n * ty_n * ((d.nx + kResidPlanes - 1) / kResidPlanes);
     for (unsigned w = blockIdx.x; w < items; w += gridDim.x) {
         const unsigned tzi = w % tz_n, rest = w / tz_n, tyi = rest % ty_n, chunk = rest / ty_n;
         const int k = (int)tzi * 64 + 2 * tx, j = (int)tyi * 8 + ty;
         const int jh = (int)tyi * 8 + hy - 1, kh = (int)tzi * 64 + hz - 2;
         const bool in = k < d.nz && j < d.ny;  // nz is even: both cells or none
         const bool halo = tid < 80 && jh >= 0 && jh < d.ny && kh >= 0 && kh < d.nz;
-        const int i0 = (int)chunk * planes, i_end = min(d.nx, i0 + planes);
-        bool any = false;
-        if (tx < i_end - i0 && j < d.ny) any = rows[(i0 + tx) * d.ny + j] != 0;
+        const int i0 = (int)chunk * kResidPlanes, i_end = min(d.nx, i0 + kResidPlanes);
         const int m0 = in ? (i0 * d.ny + j) * nh + (k >> 1) : 0;  // split index of the pair, plane i0
-        if (!__syncthreads_or(any)) {  // residual zero
-            if (r && in)
-                for (int i = i0, m = m0; i < i_end; i++, m += d.ny * nh) {
-                    if (sizeof(TR) == 4) {
-                        r[m] = (TR)0;
-                        r[hn + m] = (TR)0;
-                    } else {
-                        r[2 * (long long)m] = r[2 * (long long)m + 1] = (TR)0;
-                    }
-                }
-            continue;
-        }
         const double2 *xo = reinterpret_cast<const double2 *>(x) + m0, *bo = reinterpret_cast<const double2 *>(b) + m0;
         const double *xh = x + (halo ? (i0 * d.ny + jh) * d.nz + kh : 0);
-        const uint8_t *f = rows + i0 * d.ny + j, *f0 = other0 + i0 * d.ny + j, *f1 = other1 + i0 * d.ny + j;
+        const uint8_t *f0 = other0 + i0 * d.ny + j, *f1 = other1 + i0 * d.ny + j;
         const double *az = cf.az + (in ? (i0 * d.ny + j) * d.nz + 1 : 0);  // the coupling of a row of one
         const int ps = d.ny * nh;  // pairs of a plane
         const double2 zero2 = make_double2(0., 0.);
+        auto put1 = [&](int q, int row, int col, const F64Fixed &v) {
+            plane[q][row][col] = v.m;
+            expo[q][row][col] = v.e;
+        };
+        auto at = [&](int q, int row, int col) { return F64Fixed{plane[q][row][col], expo[q][row][col]}; };
         auto put = [&](int q, const double2 &h2) {  // the halo values of one plane
             if (!(tid < 80)) return;
-            const long long h0 = to_fixed(h2.x, emax);
-            plane[q][hy][hz] = h0;
-            if (pair) plane[q][hy][hz + 1] = to_fixed(h2.y, emax);
+            put1(q, hy, hz, f64_fixed(h2.x));
+            if (pair) put1(q, hy, hz + 1, f64_fixed(h2.y));
         };
         auto beside = [&](int p) {
             double2 h2 = zero2;
@@ -1366,19 +1333,10 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
             }
             return h2;
         };
-        long long xm0 = 0, xm1 = 0, xc0, xc1;
-        if (in && i0 > 0) {
-            const double2 t = xo[-ps];
-            xm0 = to_fixed(t.x, emax);
-            xm1 = to_fixed(t.y, emax);
-        }
-        {
-            const double2 t = in ? xo[0] : zero2;
-            xc0 = to_fixed(t.x, emax);
-            xc1 = to_fixed(t.y, emax);
-        }
-        plane[0][ty + 1][2 * tx + 2] = xc0;
-        plane[0][ty + 1][2 * tx + 3] = xc1;
+        const double2 tm = in && i0 > 0 ? xo[-ps] : zero2, tc = in ? xo[0] : zero2;
+        F64Fixed xm0 = f64_fixed(tm.x), xm1 = f64_fixed(tm.y), xc0 = f64_fixed(tc.x), xc1 = f64_fixed(tc.y);
+        put1(0, ty + 1, 2 * tx + 2, xc0);
+        put1(0, ty + 1, 2 * tx + 3, xc1);
         put(0, beside(0));
         const int nyz = (j > 0) + (j < d.ny - 1) + 1;  // in-grid faces in y, and the one between the two cells
         const int n0 = nyz + (k > 0), n1 = nyz + (k + 2 < d.nz);
@@ -1388,30 +1346,29 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
             const bool more = i + 1 < i_end;
             const double2 xn = in && i + 1 < d.nx ? xo[ps] : zero2, bc = in ? bo[0] : zero2;
             const double2 hn2 = more ? beside(i + 1 - i0) : zero2;
-            // flags and coupling of the row together with the values: one after another they made a plane four
-            // memory latencies long
-            const int on = in ? *f : 0, o0 = in ? *f0 : 1, o1 = in ? *f1 : 1;
+            // marks and coupling of the row together with the values: one after another they made a plane four memory
+            // latencies long
+            const int o0 = in ? *f0 : 1, o1 = in ? *f1 : 1;
             const double cz = in ? *az : 0.;
-            const bool one = scaled & (on != 0) & ((o0 == 0) | (o1 == 0));
-            const long long xp0 = to_fixed(xn.x, emax), xp1 = to_fixed(xn.y, emax);
+            const bool one = (o0 == 0) | (o1 == 0);
+            const F64Fixed xp0 = f64_fixed(xn.x), xp1 = f64_fixed(xn.y);
             if (more) {
-                plane[q ^ 1][ty + 1][2 * tx + 2] = xp0;
-                plane[q ^ 1][ty + 1][2 * tx + 3] = xp1;
+                put1(q ^ 1, ty + 1, 2 * tx + 2, xp0);
+                put1(q ^ 1, ty + 1, 2 * tx + 3, xp1);
                 put(q ^ 1, hn2);
             }
+            const int nx2 = (i > 0) + (i < d.nx - 1);
             double r0 = 0., r1 = 0.;
-            if (one) {
-                const longlong2 ym = *reinterpret_cast<const longlong2 *>(&plane[q][ty][2 * tx + 2]);
-                const longlong2 yp = *reinterpret_cast<const longlong2 *>(&plane[q][ty + 2][2 * tx + 2]);
-                const int nx2 = (i > 0) + (i < d.nx - 1);
-                const long long t0 = xc0 * (n0 + nx2) - (xm0 + xp0 + ym.x + yp.x + plane[q][ty + 1][2 * tx + 1] + xc1);
-                const long long t1 = xc1 * (n1 + nx2) - (xm1 + xp1 + ym.y + yp.y + plane[q][ty + 1][2 * tx + 4] + xc0);
-                r0 = __fma_rn(-cz, from_fixed(t0, emax), bc.x);
-                r1 = __fma_rn(-cz, from_fixed(t1, emax), bc.y);
-            } else if (on) {
+            if (one && fixed_stencil(n0 + nx2, xc0, xm0, xp0, at(q, ty, 2 * tx + 2), at(q, ty + 2, 2 * tx + 2),
+                                     at(q, ty + 1, 2 * tx + 1), xc1, r0))
+                r0 = __fma_rn(-cz, r0, bc.x);
+            else if (in)
                 r0 = residual_cell(d, cf, x, bc.x, i, j, k);
+            if (one && fixed_stencil(n1 + nx2, xc1, xm1, xp1, at(q, ty, 2 * tx + 3), at(q, ty + 2, 2 * tx + 3),
+                                     at(q, ty + 1, 2 * tx + 4), xc0, r1))
+                r1 = __fma_rn(-cz, r1, bc.y);
+            else if (in)
                 r1 = residual_cell(d, cf, x, bc.y, i, j, k + 1);
-            }
             if (r && in) {
                 const int m = m0 + (i - i0) * ps;
                 if (sizeof(TR) == 4) {  // cell k = 2m is of colour (i + j) & 1
@@ -1424,7 +1381,7 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
                     r[2 * (long long)m + 1] = (TR)r1;
                 }
             }
-            if (on) {
+            if (in) {
                 if (!(skip0 && i + j + k == 0)) {
                     v[0] += r0 * r0;
                     if (BB) v[1] += bc.x * bc.x;  // a test of bb_slot here would issue the squares with lanes off
@@ -1438,7 +1395,6 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
             xc1 = xp1;
             xo += ps;
             bo += ps;
-            f += d.ny;
             f0 += d.ny;
             f1 += d.ny;
             az += sx;
@@ -1450,28 +1406,6 @@ __global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> c
         sc[rr_slot] = tot[0];
         if (bb_slot >= 0) sc[bb_slot] = tot[1];
     }
-}
-
-// The upper word of the largest |x| (NaN and infinities included, as the largest), into *m (zero on entry).
-__device__ __forceinline__ unsigned abs_word(double v) {
-    uint32_t h, l;
-    f64_words(v, h, l);
-    return h & 0x7fffffffu;
-}
-__device__ __forceinline__ void block_max(unsigned v, unsigned *m) {
-    v = __reduce_max_sync(0xffffffffu, v);
-    __shared__ unsigned s_max;
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    if (tid == 0) s_max = 0;
-    __syncthreads();
-    if ((tid & 31) == 0 && v) atomicMax(&s_max, v);
-    __syncthreads();
-    if (tid == 0 && s_max) atomicMax(m, s_max);
-}
-__global__ void __launch_bounds__(256) k_abs_max(long long n, const double *__restrict__ x, unsigned *m) {
-    unsigned v = 0;
-    for (long long c = blockIdx.x * 256LL + threadIdx.x; c < n; c += gridDim.x * 256LL) v = max(v, abs_word(x[c]));
-    block_max(v, m);
 }
 
 // r = b for x = 0 (the first refinement step): cast to the inner precision; slots rr = bb = (b, b).
@@ -1593,15 +1527,10 @@ __global__ void k_ir_update(long long n, double *__restrict__ x, const float *__
         x[c] += (double)dlt[c];
 }
 
-__global__ void __launch_bounds__(256) k_shift(long long n, double *__restrict__ x, unsigned *xmax) {
+__global__ void k_shift(long long n, double *__restrict__ x) {
     const double x0 = x[0];  // x[0] itself is not touched here (cleared by a memset afterwards)
-    unsigned v = 0;
-    for (long long c = blockIdx.x * 256LL + threadIdx.x + 1; c < n; c += gridDim.x * 256LL) {
-        const double t = x[c] - x0;
-        x[c] = t;
-        v = max(v, abs_word(t));
-    }
-    block_max(v, xmax);
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x + 1; c < n; c += (long long)gridDim.x * blockDim.x)
+        x[c] -= x0;
 }
 
 template <class T>
@@ -2088,8 +2017,6 @@ cudaError_t MGSolver::configure(const Dims &d, const SolverParams &p) {
     tk_.sc = sc_;
     part_ = (double *)chk(A(8 * 4 * (size_t)(kMaxRedGrid + kMaxRedGrid / kRedGroup + 1)));
     ticket_ = (unsigned *)chk(A(4 * (size_t)(2 + kMaxRedGrid / kRedGroup)));
-    xmax_ = (unsigned *)chk(A(4));
-    xmax_ok_ = false;
     if (p.precision == 0) {
         x64_.assign(L, nullptr);
         b64_.assign(L, nullptr);
@@ -2236,14 +2163,13 @@ void MGSolver::plan_tail() {
     }
 }
 
-const SplitOut *MGSolver::split_targets(bool dense) {
-    dense_ = dense;
+const SplitOut *MGSolver::split_targets(bool marks) {
+    marks_ = marks;
     if (!split0_) return nullptr;
     so_.c32 = c32_;
     so_.c16 = c16s0_;
     so_.rows = rows_[0];
-    so_.other[0] = other_[0];
-    so_.other[1] = other_[1];
+    for (int q = 0; q < 2; q++) so_.other[q] = marks ? other_[q] : nullptr;
     copies_written_ = true;
     return &so_;
 }
@@ -2285,7 +2211,7 @@ cudaError_t MGSolver::build_hierarchy() {
         }
     } else {
         if (split0_) {
-            other_ok_ = copies_written_;
+            other_ok_ = copies_written_ && marks_;
             if (!copies_written_)
                 k_to_split<<<split_rows_grid(lev_dims_[0]), dim3(32, 8), 0, st_>>>(lev_dims_[0], c64_[0], c32_,
                                                                                     c16s0_, rows_[0]);
@@ -2669,7 +2595,6 @@ cudaError_t MGSolver::solve_mixed(bool x_is_zero, SolveResult &res) {
     const dim3 tg = tile_grid(d, xpb, kStencilBlocks);
     cudaError_t e;
     if (x_is_zero) cudaMemsetAsync(x_, 0, 8 * n, st_);
-    xmax_ok_ = false;
     double bb = -1, rr = 0;
     int total_inner = 0, outer = 0;
     const int max_outer = 30;
@@ -2732,10 +2657,8 @@ cudaError_t MGSolver::solve_mixed(bool x_is_zero, SolveResult &res) {
         }
         total_inner += it;
         if (split0_) {
-            cudaMemsetAsync(xmax_, 0, 4, st_);
             k_ir_update_s<<<row_grid((const void *)k_ir_update_s, (long long)d.nx * d.ny * (((d.nz >> 1) + 127) / 128)),
-                            dim3(32, 8), 0, st_>>>(d, x_, d32_, list_[0], count_, xmax_);
-            xmax_ok_ = true;
+                            dim3(32, 8), 0, st_>>>(d, x_, d32_, list_[0], count_);
         } else
             k_ir_update<<<flat_grid(n), 256, 0, st_>>>(n, x_, d32_);
         tk_.launches++;
@@ -2817,27 +2740,19 @@ cudaError_t MGSolver::learned_step(double rr, bool first, bool &stalled, SolveRe
 template <class TR>
 void MGSolver::residual_split(TR *r, bool skip0, int rr_slot, int bb_slot) {
     const Dims &d = lev_dims_[0];
-    int xpb;
-    const dim3 tg = tile_grid(d, xpb, kStencilBlocks);
     if (!other_ok_) {
+        int xpb;
+        const dim3 tg = tile_grid(d, xpb, kStencilBlocks);
         k_residual64<TR><<<tg, dim3(32, 8), 0, st_>>>(d, xpb, c64_[0], x_, b_, r, skip0 ? 1 : 0, rr_slot, bb_slot, sc_,
                                                       part_, ticket_, sizeof(TR) == 4 ? 1 : 0, rows_[0]);
         return;
     }
-    if (!xmax_ok_) {
-        cudaMemsetAsync(xmax_, 0, 4, st_);
-        k_abs_max<<<flat_grid(d.n), 256, 0, st_>>>(d.n, x_, xmax_);
-        xmax_ok_ = true;
-        tk_.launches++;
-    }
-    // planes an item: eight where every row has work (256^3 potential: 189 us against 205 with four); the pressure's
-    // active rows then fall unevenly to the blocks (199 us against 134)
-    const int planes = dense_ ? 8 : 4;
-    const long long items = (long long)((d.nz + 63) / 64) * ((d.ny + 7) / 8) * ((d.nx + planes - 1) / planes);
+    const long long items =
+        (long long)((d.nz + 63) / 64) * ((d.ny + 7) / 8) * ((d.nx + kResidPlanes - 1) / kResidPlanes);
     auto go = [&](auto kernel) {
         const int grid = (int)std::min<long long>(items, std::min(resident_grid((const void *)kernel), kMaxRedGrid));
-        kernel<<<grid, dim3(32, 8), 0, st_>>>(d, c64_[0], rows_[0], other_[0], other_[1], xmax_, x_, b_, r,
-                                              skip0 ? 1 : 0, rr_slot, bb_slot, sc_, part_, ticket_, planes);
+        kernel<<<grid, dim3(32, 8), 0, st_>>>(d, c64_[0], other_[0], other_[1], x_, b_, r, skip0 ? 1 : 0, rr_slot, bb_slot,
+                                              sc_, part_, ticket_);
     };
     if (bb_slot >= 0)
         go(k_residual_rows<TR, true>);
@@ -2866,9 +2781,7 @@ cudaError_t MGSolver::true_relres(bool skip0, double &relres, double &bnorm) {
 
 cudaError_t MGSolver::shift_to_zero_at_origin() {
     const long long n = lev_dims_[0].n;
-    cudaMemsetAsync(xmax_, 0, 4, st_);
-    k_shift<<<flat_grid(n), 256, 0, st_>>>(n, x_, xmax_);
-    xmax_ok_ = true;
+    k_shift<<<flat_grid(n), 256, 0, st_>>>(n, x_);
     tk_.launches++;
     cudaMemsetAsync(x_, 0, 8, st_);
     return cudaGetLastError();

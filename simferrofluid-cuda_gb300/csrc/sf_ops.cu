@@ -106,7 +106,6 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
     }
     double lower[3] = {0, 0, 0};
     double diag = 0, dexv = 0, div = 0;
-    bool one = liquid;  // every in-grid face fully open to a liquid cell
     if (liquid) {
         const int dn[3] = {d.nx, d.ny, d.nz};
 #pragma unroll
@@ -121,12 +120,10 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
             const bool valid = n3[a] >= 0 && n3[a] < dn[a];
             const long long f = fid(d, a, f3[0], f3[1], f3[2]);
             const double w = valid ? 1. - frac.p[a][f] : 0.0;
-            if (valid && __double_as_longlong(w) != kOneBits) one = false;
             if (w > 0) {
                 if (!rhs_only) {
                     const long long nb = cid(d, n3[0], n3[1], n3[2]);
                     const double pn = phi[nb];
-                    if (!le0(pn)) one = false;
                     if (le0(pn)) {
                         diag += w;
                         if (!up) lower[a] = w;
@@ -157,10 +154,7 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
     cf.dex[c] = dexv;
     cf.D[c] = D;
     if (want_invd) cf.invd[c] = liquid ? (D > 0 ? 1. / D : 0.0) : 0.0;
-    if (so.rows) {
-        split_store(so, d, i, j, k, lower[0], lower[1], lower[2], dexv, D > 0);
-        if (!one) so.other[0][(long long)i * d.ny + j] = 1;  // every writer stores 1
-    }
+    if (so.rows) split_store(so, d, i, j, k, lower[0], lower[1], lower[2], dexv, D > 0);
 }
 
 // Pressure::ApplyProjection (core/Pressure.cpp:137-166).  One thread per node (i, j, k) of the cell grid updates
@@ -526,8 +520,6 @@ void launch_build_pressure(cudaStream_t st, const Dims &d, const double *phi, co
     if (so && !rhs_only) {
         o = *so;
         cudaMemsetAsync(o.rows, 0, (size_t)d.nx * d.ny, st);
-        cudaMemsetAsync(o.other[0], 0, (size_t)d.nx * d.ny, st);
-        cudaMemsetAsync(o.other[1], 1, (size_t)d.nx * d.ny, st);  // the projection has no second kind
     }
     k_build_pressure<<<grid3(d.nx, d.ny, d.nz), blk2(), 0, st>>>(d, phi, frac, u, us, jump, vol_error, cf, b,
                                                                   rhs_only ? 1 : 0, want_invd ? 1 : 0, o);

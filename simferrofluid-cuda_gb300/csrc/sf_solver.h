@@ -115,9 +115,9 @@ class MGSolver {
     cudaError_t build_hierarchy();
 
     // Where the assembly kernels may write the split level-0 copies and row flags directly (smoother 3 in the
-    // mixed form), or nullptr; the next build_hierarchy then takes them as written.  dense: every row of the system
-    // has active cells (the potential's).
-    const SplitOut *split_targets(bool dense);
+    // mixed form), or nullptr; the next build_hierarchy then takes them as written.  marks: they write SplitOut::other
+    // too (the potential's).
+    const SplitOut *split_targets(bool marks);
 
     // Solve A x = b.  x holds the initial guess unless x_is_zero.  exclude_cell0_norm: report the residual
     // without row 0 (the potential's pinned row).
@@ -187,9 +187,7 @@ class MGSolver {
     bool copies_written_ = false;        // the assembly wrote the split copies and flags
     uint8_t *other_[2] = {nullptr, nullptr};  // level 0: rows that are not of one exact coupling (SplitOut::other)
     bool other_ok_ = false;              // they belong to the operator in place
-    bool dense_ = false;                 // every row has active cells
-    unsigned *xmax_ = nullptr;           // upper word of the largest |x|
-    bool xmax_ok_ = false;               // it belongs to the x in place
+    bool marks_ = false;                 // the assembly writes them
     // the FP64 residual of the split form, by rows of one coupling where it can (k_residual_rows)
     template <class TR>
     void residual_split(TR *r, bool skip0, int rr_slot, int bb_slot);

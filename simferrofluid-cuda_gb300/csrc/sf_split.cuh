@@ -326,17 +326,12 @@ __global__ void __launch_bounds__(256) k_cast_rhs_s(Dims d, const double *__rest
     }
 }
 
-__device__ __forceinline__ unsigned abs_word(double v);
-__device__ __forceinline__ void block_max(unsigned v, unsigned *m);
-
-// x64 += d32 with d32 in the split layout (zero in inactive rows, which are skipped), and the upper word of the largest
-// |x| over them (*xmax zero on entry).  A lane takes cells 2m and 2m + 1 as one 16-byte vector.
+// x64 += d32 with d32 in the split layout (zero in inactive rows, which are skipped).  A lane takes cells 2m and 2m + 1 as
+// one 16-byte vector.
 __global__ void __launch_bounds__(256) k_ir_update_s(Dims d, double *__restrict__ x, const float *__restrict__ dlt,
-                                                     const int *__restrict__ list, const int *__restrict__ count,
-                                                     unsigned *xmax) {
+                                                     const int *__restrict__ list, const int *__restrict__ count) {
     const int nh = d.nz >> 1;
     const long long hn = d.n >> 1;
-    unsigned most = 0;
     for_list_items(list, count, 1, (nh + 127) / 128, [&](int, int i, int j, int ch, bool) {
         const long long row = (long long)i * d.ny + j;
         const bool p = (i + j) & 1;
@@ -361,10 +356,8 @@ __global__ void __launch_bounds__(256) k_ir_update_s(Dims d, double *__restrict_
             t[q].x += f32_to_f64(p ? d1[q] : d0[q]);
             t[q].y += f32_to_f64(p ? d0[q] : d1[q]);
             xr[m] = t[q];
-            most = max(most, max(abs_word(t[q].x), abs_word(t[q].y)));
         }
     });
-    block_max(most, xmax);
 }
 
 // Krylov vector kernels of the split level: items are the rows of one colour (2 n_rows of them, float4 along a
