@@ -2740,15 +2740,18 @@ cudaError_t MGSolver::learned_step(double rr, bool first, bool &stalled, SolveRe
 template <class TR>
 void MGSolver::residual_split(TR *r, bool skip0, int rr_slot, int bb_slot) {
     const Dims &d = lev_dims_[0];
-    if (!other_ok_) {
+    const long long items =
+        (long long)((d.nz + 63) / 64) * ((d.ny + 7) / 8) * ((d.nx + kResidPlanes - 1) / kResidPlanes);
+    // Marching costs its eight planes' latency whatever the size; below three items an SM the chip is not full and
+    // k_residual64 is the faster (a warm solve that stops at its two residuals: 16^3 198 and 222 us, 96^3 394 and 419, 112^3
+    // 471 and 469, 128^3 516 and 498).
+    if (!other_ok_ || items < 3 * 152) {
         int xpb;
         const dim3 tg = tile_grid(d, xpb, kStencilBlocks);
         k_residual64<TR><<<tg, dim3(32, 8), 0, st_>>>(d, xpb, c64_[0], x_, b_, r, skip0 ? 1 : 0, rr_slot, bb_slot, sc_,
                                                       part_, ticket_, sizeof(TR) == 4 ? 1 : 0, rows_[0]);
         return;
     }
-    const long long items =
-        (long long)((d.nz + 63) / 64) * ((d.ny + 7) / 8) * ((d.nx + kResidPlanes - 1) / kResidPlanes);
     auto go = [&](auto kernel) {
         const int grid = (int)std::min<long long>(items, std::min(resident_grid((const void *)kernel), kMaxRedGrid));
         kernel<<<grid, dim3(32, 8), 0, st_>>>(d, c64_[0], other_[0], other_[1], x_, b_, r, skip0 ? 1 : 0, rr_slot, bb_slot,
