@@ -64,15 +64,15 @@ __device__ __forceinline__ GridPoint grid_point(const double o[3], double h, dou
 // because beside the other form its instructions would be issued with their lanes off.
 __device__ __noinline__ double trilinear_plain(const double *v, int sx, int sy, int sz, AxisPoint x, AxisPoint y,
                                                AxisPoint z) {
+    const int cx[2] = {min(max(x.lo, 0), sx - 1), min(max(x.lo + 1, 0), sx - 1)};
+    const int cy[2] = {min(max(y.lo, 0), sy - 1), min(max(y.lo + 1, 0), sy - 1)};
+    const int cz[2] = {min(max(z.lo, 0), sz - 1), min(max(z.lo + 1, 0), sz - 1)};
+    double f[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) f[q] = v[cz[q >> 2] + sz * (cy[(q >> 1) & 1] + sy * cx[q & 1])];
     double val = 0;
-#pragma unroll 1
-    for (int q = 0; q < 8; q++) {
-        const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
-        const int cx = min(max(x.lo + dx, 0), sx - 1), cy = min(max(y.lo + dy, 0), sy - 1);
-        const int cz = min(max(z.lo + dz, 0), sz - 1);
-        const double wt = (dx ? x.w[1] : x.w[0]) * (dy ? y.w[1] : y.w[0]) * (dz ? z.w[1] : z.w[0]);
-        val += v[cz + sz * (cy + sy * cx)] * wt;
-    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) val += f[q] * (x.w[q & 1] * y.w[(q >> 1) & 1] * z.w[q >> 2]);
     return val;
 }
 
@@ -142,28 +142,45 @@ __device__ __forceinline__ CubicPoint cubic_point(double p, double co, double h,
     return g;
 }
 
-// TriCuInterp::Interpolate of the cell grid: 64 points in (k, j, i) order, clamped At().  In plain FP64, for weights or
-// values outside the integer form's range.
+// TriCuInterp::Interpolate of the cell grid: 64 points in (k, j, i) order, clamped At().  In plain FP64, for weights outside
+// the integer form's range.
 __device__ __noinline__ double tricubic_plain(int nx, int ny, int nz, const double *f, CubicPoint x, CubicPoint y,
                                               CubicPoint z) {
+    int cx[4], cy[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        cx[q] = min(max(x.lo + q, 0), nx - 1) * (ny * nz);
+        cy[q] = min(max(y.lo + q, 0), ny - 1) * nz;
+    }
     double val = 0;
 #pragma unroll 1
-    for (int q = 0; q < 64; q++) {
-        const int i = q & 3, j = (q >> 2) & 3, k = q >> 4;
-        const int cx = min(max(x.lo + i, 0), nx - 1), cy = min(max(y.lo + j, 0), ny - 1);
-        const int cz = min(max(z.lo + k, 0), nz - 1);
-        const double wx = i == 0 ? x.w[0] : (i == 1 ? x.w[1] : (i == 2 ? x.w[2] : x.w[3]));
-        const double wy = j == 0 ? y.w[0] : (j == 1 ? y.w[1] : (j == 2 ? y.w[2] : y.w[3]));
+    for (int k = 0; k < 4; k++) {
+        const double *plane = f + min(max(z.lo + k, 0), nz - 1);
         const double wz = k == 0 ? z.w[0] : (k == 1 ? z.w[1] : (k == 2 ? z.w[2] : z.w[3]));
-        val += f[cz + nz * (cy + ny * cx)] * (wx * wy * wz);
+        double v[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = plane[cx[q & 3] + cy[q >> 2]];
+#pragma unroll
+        for (int q = 0; q < 16; q++) val += v[q] * (x.w[q & 3] * y.w[q >> 2] * wz);
     }
+    return val;
+}
+
+// A sum's next four terms, a row of the stencil: values of any size times products xy[i] wz, in plain FP64.  Its own
+// function for the reason of trilinear_plain.
+__device__ __noinline__ double tricubic_row(double val, double v0, double v1, double v2, double v3, const double *xy,
+                                            double wz) {
+    val += v0 * (xy[0] * wz);
+    val += v1 * (xy[256] * wz);
+    val += v2 * (xy[512] * wz);
+    val += v3 * (xy[768] * wz);
     return val;
 }
 
 // The same.  An axis on which the point sits on a cell (weights exactly 0, 1, 0, 0: no motion along it) keeps its second
 // point alone: the others would add a signed zero to a sum that starts at +0, as long as their values are finite.
-// Otherwise the weights are normal and so is every product, as long as the values are in [2^-100, 2^300); one that is
-// not (a zero among them) leaves the sum to the plain form.
+// Otherwise the weights are normal and so is every product, as long as the values are in [2^-100, 2^300); a row that holds
+// another value (a zero, as on a layer of cells that the surface passes through exactly) is summed in FP64.
 // The sixteen products of the x and y weights wait in shared memory (`xy`, this thread's column of 256), so that the
 // loops over k and j stay loops: unrolled over j they took 2600 us at 192^3, the warps waiting for instructions.
 __device__ __forceinline__ double tricubic(const Dims &d, const double *__restrict__ f, const CubicPoint g[3],
@@ -204,7 +221,7 @@ __device__ __forceinline__ double tricubic(const Dims &d, const double *__restri
                 }
                 if (size < kF64Exp && ((one[2] && k != 1) || (one[1] && j != 1))) continue;  // finite times zero
                 if (far >= (400u << 20)) {
-                    hard = true;
+                    val = tricubic_row(val, v[0], v[1], v[2], v[3], &xy[4 * j][tid], wk);
                     continue;
                 }
 #pragma unroll
