@@ -584,7 +584,8 @@ __global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, dou
     __shared__ uint16_t queue[3 * 256];
     __shared__ int queued;
     const int tid = threadIdx.x, lz = tid & 15, ly = (tid >> 4) & 3, lx = tid >> 6;
-    const int k0 = blockIdx.x * kRz, j0 = blockIdx.y * kRy, i0 = blockIdx.z * kRx;
+    const unsigned zb = (unsigned)(d.nz + kRz - 1) / kRz, yb = blockIdx.x / zb;  // reinit_grid
+    const int k0 = (int)(blockIdx.x - yb * zb) * kRz, j0 = (int)yb * kRy, i0 = blockIdx.y * kRx;
     const int lastx = d.nx - 1, lasty = d.ny - 1, lastz = d.nz - 1;
     if (tid == 0) queued = 0;
     for (int e = tid; e < kRdx; e += 256) {  // [m][y][z], m the lower x plane + 3
@@ -682,8 +683,9 @@ __global__ void __launch_bounds__(256, 4) k_reinit_advance(Dims d, double h, dou
     }
 }
 
+// z and y tiles share x: 65,535 tiles of four rows in a launch's y would refuse a grid that the other kernels take
 inline dim3 reinit_grid(const Dims &d) {
-    return dim3((d.nz + kRz - 1) / kRz, (d.ny + kRy - 1) / kRy, (d.nx + kRx - 1) / kRx);
+    return dim3((unsigned)((d.nz + kRz - 1) / kRz) * ((d.ny + kRy - 1) / kRy), (d.nx + kRx - 1) / kRx);
 }
 
 inline dim3 cell_grid(const Dims &d) { return dim3((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx); }
