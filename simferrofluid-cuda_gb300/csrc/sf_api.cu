@@ -30,12 +30,13 @@ struct Ctx {
     Dims mag_dims{0, 0, 0, 0};
     // staging buffers for the host-pointer entry points
     DevBuf phi, frac[3], vel[3], us[3], jump[3], hext[3], H[3], cells;
-    // velocity pipeline after the projection: extrapolation validity bits, enforce's lists of
-    // faces (their new values in old) and its counters, normals; old also holds advection's copy of the velocity
-    DevBuf mask[6], old[3], enf[4], normal[3];
+    // velocity pipeline after the projection: extrapolation validity bits, the new values of enforce's listed faces
+    // (and advection's copy of the velocity), enforce's counters, normals
+    DevBuf mask[6], old[3], enf, normal[3];
     // interface coupling: mesh vertices, vertex values and edge marks
     DevBuf vpos, vnrm, vval, kappa, edge[3];
-    // level-set operations: two scratch cell fields; advection's table of its first trace points
+    // level-set operations: two scratch cell fields, where enforce lists its faces too; advection's table of its first
+    // trace points
     DevBuf ls1, ls2, own;
     // learned form: attached network (not owned) and its buffers; every network created on this context is
     // registered so that destroying the context first leaves the network handles safe to destroy later
@@ -675,7 +676,6 @@ sf_status enforce_impl(Ctx *c, const sf_grid *g, double *const vel[3], const dou
     long long h2d = 0;
     double *dvel[3];
     Faces ff{}, fn{}, fus{};
-    uint32_t *face[3];
     double *value[3];
     if ((s = stage_vel(c, g, vel, dev, dvel, h2d)) != SF_OK) return s;
     for (int a = 0; a < 3; a++) {
@@ -685,12 +685,15 @@ sf_status enforce_impl(Ctx *c, const sf_grid *g, double *const vel[3], const dou
         if ((s = stage_in(c, c->us[a], us ? us[a] : nullptr, nf, dev, &fus.p[a], h2d)) != SF_OK) return s;
         // Collider::Enforce interpolates the velocity as it was before the call: new values wait in a list
         CK(c->old[a].ensure(8 * (size_t)nf));
-        CK(c->enf[a].ensure(4 * (size_t)nf));
         value[a] = (double *)c->old[a].get();
-        face[a] = (uint32_t *)c->enf[a].get();
     }
-    CK(c->enf[3].ensure(3 * sizeof(unsigned)));
-    launch_enforce(c->st, d, g->origin, g->h, fus, fn, ff, dvel, face, value, (unsigned *)c->enf[3].get());
+    // the lists have room for every face: 12 bytes a cell, in the level-set operations' 16 where those have run
+    const size_t nx = (size_t)face_count(g, 0), ny = (size_t)face_count(g, 1), nz = (size_t)face_count(g, 2);
+    CK(c->ls1.ensure(4 * (nx + ny)));
+    CK(c->ls2.ensure(4 * nz));
+    uint32_t *const face[3] = {(uint32_t *)c->ls1.get(), (uint32_t *)c->ls1.get() + nx, (uint32_t *)c->ls2.get()};
+    CK(c->enf.ensure(3 * sizeof(unsigned)));
+    launch_enforce(c->st, d, g->origin, g->h, fus, fn, ff, dvel, face, value, (unsigned *)c->enf.get());
     CK(cudaGetLastError());
     return unstage_vel(c, g, vel, dev, dvel);
 }
