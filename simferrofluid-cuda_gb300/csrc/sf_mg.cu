@@ -1495,22 +1495,6 @@ __global__ void __launch_bounds__(256) k_learned_update(long long n, float *__re
     }
 }
 
-// (y, b) with y FP32 and b FP64 -> slot
-__global__ void __launch_bounds__(256) k_dot_fd(long long n, const float *__restrict__ y, const double *__restrict__ b,
-                                                int slot, double *sc, double *part, unsigned *ticket) {
-    float acc = 0.f;
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    for (long long c = blockIdx.x * 256LL + tid; c < n; c += (long long)gridDim.x * 256) acc += y[c] * (float)b[c];
-    float v[1] = {acc};
-    double tot[1];
-    if (grid_reduce<1>(v, part, ticket, tot)) sc[slot] = tot[0];
-}
-
-__global__ void k_scale_to64(long long n, double g, const float *__restrict__ y, double *__restrict__ x) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-        x[c] = g * (double)y[c];
-}
-
 // (a, b) of two FP64 vectors -> slot
 __global__ void __launch_bounds__(256) k_dot_dd(long long n, const double *__restrict__ a, const double *__restrict__ b,
                                                 int slot, double *sc, double *part, unsigned *ticket) {
@@ -1531,12 +1515,6 @@ __global__ void k_shift(long long n, double *__restrict__ x) {
     const double x0 = x[0];  // x[0] itself is not touched here (cleared by a memset afterwards)
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x + 1; c < n; c += (long long)gridDim.x * blockDim.x)
         x[c] -= x0;
-}
-
-template <class T>
-__global__ void k_copy_cast(long long n, const double *__restrict__ a, T *__restrict__ o) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-        o[c] = (T)a[c];
 }
 
 static inline int flat_grid(long long n) {
@@ -1988,7 +1966,6 @@ cudaError_t MGSolver::configure(const Dims &d, const SolverParams &p) {
     }
     destroy_graphs();
     free_all();
-    other_ok_ = false;
     lev_dims_ = dims;
     rows64_ = rows64;
     const int L = (int)dims.size();
@@ -2170,7 +2147,6 @@ const SplitOut *MGSolver::split_targets(bool marks) {
     so_.c16 = c16s0_;
     so_.rows = rows_[0];
     for (int q = 0; q < 2; q++) so_.other[q] = marks ? other_[q] : nullptr;
-    copies_written_ = true;
     return &so_;
 }
 
@@ -2211,11 +2187,7 @@ cudaError_t MGSolver::build_hierarchy() {
         }
     } else {
         if (split0_) {
-            other_ok_ = copies_written_ && marks_;
-            if (!copies_written_)
-                k_to_split<<<split_rows_grid(lev_dims_[0]), dim3(32, 8), 0, st_>>>(lev_dims_[0], c64_[0], c32_,
-                                                                                    c16s0_, rows_[0]);
-            copies_written_ = false;
+            // the assembly has written the FP32 and FP16 copies and the row flags (split_targets)
             k_rows_uniform<float><<<split_rows_grid(lev_dims_[0]), dim3(32, 8), 0, st_>>>(lev_dims_[0], c32_, rows_[0],
                                                                                           crow_);
             k_smooth_consts_s<__half><<<split_rows_grid(lev_dims_[0]), dim3(32, 8), 0, st_>>>(
@@ -2292,7 +2264,6 @@ cudaError_t MGSolver::build_hierarchy() {
 
 void MGSolver::enqueue_iter64(bool copy_slots) {
     const Dims &d = lev_dims_[0];
-    const long long n = d.n;
     int xpb;
     const dim3 tg = tile_grid3(d, xpb);
     const long long l0 = tk_.launches;
@@ -2315,7 +2286,6 @@ void MGSolver::enqueue_iter64(bool copy_slots) {
 
 void MGSolver::enqueue_iter32(bool copy_slots) {
     const Dims &d = lev_dims_[0];
-    const long long n = d.n;
     const long long l0 = tk_.launches;
     const std::vector<float *> ts = prm_.smoother == 1 ? t32_ : std::vector<float *>(t32_.size(), nullptr);
     if (split0_) {
@@ -2745,7 +2715,7 @@ void MGSolver::residual_split(TR *r, bool skip0, int rr_slot, int bb_slot) {
     // Marching costs its eight planes' latency whatever the size; below three items an SM the chip is not full and
     // k_residual64 is the faster (a warm solve that stops at its two residuals: 16^3 198 and 222 us, 96^3 394 and 419, 112^3
     // 471 and 469, 128^3 516 and 498).
-    if (!other_ok_ || items < 3 * 152) {
+    if (!marks_ || items < 3 * 152) {
         int xpb;
         const dim3 tg = tile_grid(d, xpb, kStencilBlocks);
         k_residual64<TR><<<tg, dim3(32, 8), 0, st_>>>(d, xpb, c64_[0], x_, b_, r, skip0 ? 1 : 0, rr_slot, bb_slot, sc_,

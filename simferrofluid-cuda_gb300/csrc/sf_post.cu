@@ -52,7 +52,6 @@ __global__ void __launch_bounds__(256) k_extrap_init(Dims d, const double *__res
                                                      BitRows valid, double clear_val, int clear) {
     const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i0 = blockIdx.z * kInitX;
     if (j > d.ny) return;  // whole warps: a warp is one row
-    const long long sx = (long long)d.ny * d.nz;
     const bool col = j < d.ny && k < d.nz;
     double p[kInitX + 1], py[kInitX], pz[kInitX], fr[3][kInitX];
 #pragma unroll

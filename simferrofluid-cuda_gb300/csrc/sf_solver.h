@@ -114,9 +114,8 @@ class MGSolver {
     // Build coarse levels (and the FP32/FP16 copies for the mixed form) from the fine operator.
     cudaError_t build_hierarchy();
 
-    // Where the assembly kernels may write the split level-0 copies and row flags directly (smoother 3 in the
-    // mixed form), or nullptr; the next build_hierarchy then takes them as written.  marks: they write SplitOut::other
-    // too (the potential's).
+    // Where the assembly kernels write the split level-0 copies and row flags (smoother 3 in the mixed form), or nullptr;
+    // build_hierarchy takes them as written.  marks: they write SplitOut::other too (the potential's).
     const SplitOut *split_targets(bool marks);
 
     // Solve A x = b.  x holds the initial guess unless x_is_zero.  exclude_cell0_norm: report the residual
@@ -184,10 +183,8 @@ class MGSolver {
     float *dinv_[2] = {nullptr, nullptr}; // levels 0, 1: the half sweep's 1 / D on general rows
     bool split1_ = false;                // level 1 stored colour by colour too
     SplitOut so_{};                      // split_targets()
-    bool copies_written_ = false;        // the assembly wrote the split copies and flags
     uint8_t *other_[2] = {nullptr, nullptr};  // level 0: rows that are not of one exact coupling (SplitOut::other)
-    bool other_ok_ = false;              // they belong to the operator in place
-    bool marks_ = false;                 // the assembly writes them
+    bool marks_ = false;                 // the assembly in place wrote them
     // the FP64 residual of the split form, by rows of one coupling where it can (k_residual_rows)
     template <class TR>
     void residual_split(TR *r, bool skip0, int rr_slot, int bb_slot);

@@ -191,39 +191,6 @@ static int row_grid(const void *kernel, long long items) {
     return (int)(need < 1 ? 1 : (need < g ? need : g));
 }
 
-// FP64 level 0 -> split FP32 copy (Krylov operator) and FP16 copy (smoother) in one pass, with the roundings
-// of k_to32 / k_to16, and the level's row flags (a row is active when one of its cells has D > 0).  One warp
-// per row: blockDim = (32, 8).
-__global__ void __launch_bounds__(256) k_to_split(Dims d, Coef<double> f, Coef<float> o32, Coef<__half> o16,
-                                                  uint8_t *__restrict__ rows) {
-    const int nh = d.nz >> 1;
-    const long long hn = d.n >> 1, nrows = (long long)d.nx * d.ny;
-    for (long long row = blockIdx.x * (long long)blockDim.y + threadIdx.y; row < nrows;
-         row += (long long)gridDim.x * blockDim.y) {
-        const int i = (int)row / d.ny, j = (int)row - i * d.ny;
-        const int p = (i + j) & 1;
-        const long long nat = row * d.nz, sp = row * nh;
-        bool act = false;
-        for (int m = threadIdx.x; m < nh; m += blockDim.x) {
-            const long long n0 = nat + 2 * m + p, n1 = nat + 2 * m + 1 - p, s0 = sp + m, s1 = hn + sp + m;
-            const double *src[4] = {f.ax, f.ay, f.az, f.dex};
-            float *d32[4] = {o32.ax, o32.ay, o32.az, o32.dex};
-            __half *d16[4] = {o16.ax, o16.ay, o16.az, o16.dex};
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const float v0 = f64_to_f32(src[a][n0]), v1 = f64_to_f32(src[a][n1]);
-                d32[a][s0] = v0;
-                d32[a][s1] = v1;
-                d16[a][s0] = __float2half_rn(v0);
-                d16[a][s1] = __float2half_rn(v1);
-            }
-            act |= (f.D[n0] > 0.0) | (f.D[n1] > 0.0);
-        }
-        act = __any_sync(0xffffffffu, act);
-        if (threadIdx.x == 0) rows[row] = act ? 1 : 0;
-    }
-}
-
 // Row flags of a coarse level from the next finer one: coarse row (I, J) is active when one of the fine rows
 // (2I + di, 2J + dj) is (a coarse cell whose children are all inactive has an all-zero operator row).
 __global__ void k_rows_coarsen(Dims df, const uint8_t *__restrict__ rf, Dims dc, uint8_t *__restrict__ rc) {

@@ -28,9 +28,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&v);
 }
-__device__ __forceinline__ uint32_t pack_raw(bf16 lo, bf16 hi) {
-    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-}
 
 // tap t of a 3x3x3 stencil: offsets (dx, dy, dz) in -1..1, t = 9 (dx+1) + 3 (dy+1) + (dz+1)
 __device__ __forceinline__ void tap_off(int t, int taps, int &dx, int &dy, int &dz) {
