@@ -1264,11 +1264,11 @@ __global__ void __launch_bounds__(256) k_residual64(Dims d, int xpb, Coef<double
 //
 // A block owns a 64 (z) x 8 (y) tile and marches along x, kResidPlanes an item, two cells of a row a thread; each value is
 // taken apart once (f64_fixed) and shared through two planes of shared memory, zero outside the grid; a cell's sum is
-// formed in the unit of its own seven values.  234 us (225 without an output), bound by the latency of a plane between its
-// barriers and the integer pipe; 244 us with five blocks an SM (48 registers, spilled).  One unit for the whole field takes
-// 189 us, but parts of a field far below its largest value lose bits; one for an item, with the cells below an eighth of it
-// left to FP64, 275 us.  The pressure, whose rows mostly lie across the surface or outside the liquid, takes 162 us here and
-// 147 by k_residual64, which it keeps.
+// formed in the unit of its own seven values.  200 us (195 without an output), bound by the latency of a plane between its
+// barriers: the FP64 pipe is 54% busy, the integer pipe 50%; 217 us with four blocks an SM (64 registers, none spilled).
+// One unit for the whole field takes 189 us, but parts of a field far below its largest value lose bits; one for an item,
+// with the cells below an eighth of it left to FP64, 275 us.  The pressure, whose rows mostly lie across the surface or
+// outside the liquid, took 162 us here and 147 by k_residual64, which it keeps.
 constexpr int kResidPlanes = 8;
 // b - A x of one cell in FP64; a call, so that its registers are not the common rows'.
 __device__ __noinline__ double residual_cell(const Dims &d, const Coef<double> &cf, const double *x, double bc, int i,
@@ -1280,7 +1280,7 @@ __device__ __noinline__ double residual_cell(const Dims &d, const Coef<double> &
 }
 
 template <class TR, bool BB>
-__global__ void __launch_bounds__(256, 4) k_residual_rows(Dims d, Coef<double> cf,
+__global__ void __launch_bounds__(256, 5) k_residual_rows(Dims d, Coef<double> cf,
                                                        const uint8_t *__restrict__ other0,
                                                        const uint8_t *__restrict__ other1,
                                                        const double *__restrict__ x, const double *__restrict__ b,
