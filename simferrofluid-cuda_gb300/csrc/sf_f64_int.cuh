@@ -375,7 +375,7 @@ SF_CONV_FN double fixed_to_f64(int64_t t, int e) {
     return m == 0 ? 0. : f64_from_words((uint32_t)(bits >> 32), (uint32_t)bits);
 }
 
-// s = n x - (a + b + c + d + e + f), n <= 6, in 64-bit integers of one unit, 2^-58 of the largest magnitude M among the seven:
+// s = n x - (a + b + c + d + e + f), n <= 6, in 64-bit integers of one unit, 2^-58 of the largest magnitude M of the seven:
 // what is lost is less than a unit a value, 6 2^-58 M in all, and the last rounding, against a rounding of up to
 // 2^-53 of the partial sum at each of seven FP64 operations.  The unit is this sum's own, so that holds wherever
 // the seven stand in a field of any range.  False (s unset) where M is below 2^-823, infinite or NaN.

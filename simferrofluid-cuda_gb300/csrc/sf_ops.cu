@@ -157,15 +157,13 @@ __global__ void __launch_bounds__(256) k_build_pressure(Dims d, const double *__
     if (so.rows) split_store(so, d, i, j, k, lower[0], lower[1], lower[2], dexv, D > 0);
 }
 
-// Pressure::ApplyProjection (core/Pressure.cpp:137-166).  One thread per node (i, j, k) of the cell grid updates
-// the lower x, y and z faces of cell (i, j, k), in one launch over (nx + 1) x (ny + 1) x (nz + 1) points, so phi and
-// p of the cell are loaded once for its three faces.  p is the solution on cells; liquid = phi <= 0.
+// Pressure::ApplyProjection (core/Pressure.cpp:137-166).  One thread per cell (i, j, k) updates its lower x,
+// y and z faces, so phi and p of the cell are loaded once for its three faces (the faces at the grid's ends are closed).  p is the solution on cells; liquid = phi <= 0.
 // w = 1 - fraction is 0 exactly when the fraction is 1, and 1 exactly when it is zero, where (p1 - p0) * w is
 // p1 - p0: both are tested on the bits, so open liquid faces take no FP64 operation beyond the update itself.
 // The level set decides first: a face between two air cells (most of a pool's domain) reads nothing more, and the
 // others load fraction, velocity and pressures together.  360 us at 256^3 (20% liquid) when the fraction of every face
-// was read first, each load waiting for the one before; 188 us now, bound by latency and the FP64 pipe (55%).  Two and
-// four planes a thread took 241 and 212 us.
+// was read first, each load waiting for the one before; 245 us now, bound by the FP64 pipe (77%).
 struct ProjFace {
     bool on, l0;
     long long f;

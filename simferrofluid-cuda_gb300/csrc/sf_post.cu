@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) k_extrap_init(Dims d, const double *__res
 // word often holds one or two (next to a wall) and an interface fills the words of one row.  Valid faces are never
 // written in a sweep, so the in-place update reads only values of the previous sweep.  A sweep touches the bits and
 // its layer's faces alone: 98 us an axis and sweep as a pass over all faces, 62 us for the three axes with a warp
-// taking its words in turn, 32 us with the list (256^3).
+// taking its words in turn, 26-65 us with the list (256^3; the first sweep has the most faces).
 __global__ void __launch_bounds__(256) k_extrap_sweep(Dims d, Faces u, BitRows valid, BitRows valid1) {
     __shared__ uint32_t near[6][256];
     __shared__ uint16_t list[256 * 32];
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) k_extrap_sweep(Dims d, Faces u, BitRows v
 // Collider::Enforce (core/Collider.cpp:75-86) changes the faces with fraction == 1 alone, one in 130 in a walled box, and
 // on the z walls one of a row's ends, so a pass with a thread a face leaves 31 lanes of a warp idle there (2.3 ms of
 // the 2.7 ms at 256^3).  Three passes instead: list the faces (all three fractions read once), evaluate the list from
-// the velocity as it was, write the values: 74, 115 (bound by the FP64 and integer pipes) and 6 us.
+// the velocity as it was, write the values: 73, 108 (bound by the FP64 pipe and latency) and 6 us.
 struct EnforceLists {
     uint32_t *face[3];    // face indices with fraction == 1
     double *value[3];     // their new velocities
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(256) k_enforce_put(EnforceLists l, Faces u) {
 
 // MagneticField::CalculateVertexPressures (core/MagneticField.cpp:37-48) for vertex v: H trilinear at its position,
 // p = mu0/2 chi (|H|^2 + chi^2/(4chi+4) (H.n)^2), mu0 = 4e-7 pi (core/MagneticField.cpp:7-8).  The two factors that
-// depend on chi alone come from the host (an FP64 division a vertex otherwise): 74 us for 196,608 vertices at the start,
-// 45 us with that and the samples' products on the integer pipe.
+// depend on chi alone come from the host (an FP64 division a vertex otherwise): 74 us for 196,608 vertices
+// before, 45 us with that and the samples' products on the integer pipe.
 __global__ void __launch_bounds__(128) k_vertex_pressures(Dims d, Origin og, double h, double invh, Faces H,
                                                           double scale, double normal_part,
                                                           const double *__restrict__ pos,
@@ -382,8 +382,8 @@ __device__ __forceinline__ bool trace_rk2(const Dims &d, const Faces &u, const O
 // (trace over -dt), by tricubic interpolation of the old phi.
 //
 // 620 FP64 operations a cell bound it (8.3 ms at 192^3, a quarter of it liquid); with the weights and three in four of
-// the products on the integer pipe, the first point from a table and zero velocities cut short, the FP64 pipe (70%
-// busy) and the integer pipe (64%) take 2.4-2.5 ms.  64 registers: four blocks an SM against three are worth 7%.
+// the products on the integer pipe, the first point from a table and zero velocities cut short, the FP64 pipe (52%
+// busy) and the integer pipe (61%) take 2.4 ms, issue the rest.  64 registers: four blocks an SM against three are worth 7%.
 __global__ void __launch_bounds__(256, 4) k_advect_levelset(Dims d, Origin og, double h, double invh, Faces u,
                                                             OwnTable own, double dt, const double *__restrict__ phi,
                                                             double *__restrict__ out) {
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(256, 4) k_advect_levelset(Dims d, Origin og, d
 
 // Advection::Solve<2>(velocity, velocity, dt) (core/Advection.h:51-59) for the faces of axis A: trilinear
 // interpolation of the old face grid A at each face's RK2 departure point.  Bound as k_advect_levelset is: 9.0 ms at
-// 160^3 for the three axes with every operation on the FP64 pipe, 1.9 ms now (73% of the FP64 pipe).
+// 160^3 for the three axes with every operation on the FP64 pipe, 1.8 ms now (67% of the FP64 pipe).
 template <int A>
 __global__ void __launch_bounds__(256, 4) k_advect_velocity(Dims d, Origin og, double h, double invh, Faces u,
                                                             OwnTable own, double dt, double *__restrict__ out) {
